@@ -527,7 +527,7 @@ int tsph_pairs_emit(const void* pos, const tsph_grid* grid, int64_t row_limit, v
     return TSPH_OK;
   });
   if (rc) return rc;
-  rc = segmented_sort_u32(cols, w.rowptr, row_limit, sort_scratch, s);
+  rc = segmented_sort_u32(cols, w.rowptr, row_limit, pair_count, sort_scratch, s);
   if (rc) return rc;
   expand_pairs<<<grid_for(row_limit * 32, 256), 256, 0, s>>>(w.rowptr, cols, row_limit, pairs);
   TSPH_LAUNCH_CHECK();

@@ -1,5 +1,6 @@
 // Device-wide scans, the stable LSD radix sort and the segmented row sort.
 #include "common.cuh"
+#include "rowsort.cuh"
 
 namespace tsph {
 
@@ -25,7 +26,10 @@ __global__ void scan_tile_totals(const TIn* __restrict__ in, int64_t n, int64_t*
   if (threadIdx.x == 0) totals[blockIdx.x] = tot;
 }
 
-template <class TIn>
+// kSum: `offsets` holds the tile totals and every block adds up the ones before
+// it itself (at most kScanDirect of them, a few loads per thread), which saves
+// the pass that scans them; otherwise it holds their exclusive scan.
+template <class TIn, bool kSum>
 __global__ void scan_tile_apply(const TIn* __restrict__ in, int64_t* __restrict__ out, int64_t n,
                                 const int64_t* __restrict__ offsets, int64_t* __restrict__ grand,
                                 const int* __restrict__ enable) {
@@ -39,8 +43,16 @@ __global__ void scan_tile_apply(const TIn* __restrict__ in, int64_t* __restrict_
     vals[k] = i < n ? static_cast<int64_t>(in[i]) : 0;
     local += vals[k];
   }
+  int64_t before = 0;
+  if (kSum) {
+    int64_t part = 0;
+    for (int t = threadIdx.x; t < static_cast<int>(blockIdx.x); t += blockDim.x) part += offsets[t];
+    block_exclusive_scan<int64_t>(part, &before);
+  } else if (offsets) {
+    before = offsets[blockIdx.x];
+  }
   int64_t tot;
-  int64_t run = block_exclusive_scan<int64_t>(local, &tot) + (offsets ? offsets[blockIdx.x] : 0);
+  int64_t run = block_exclusive_scan<int64_t>(local, &tot) + before;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     int64_t i = base + threadIdx.x * kScanItems + k;
@@ -49,6 +61,11 @@ __global__ void scan_tile_apply(const TIn* __restrict__ in, int64_t* __restrict_
   }
   if (grand && blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) *grand = run;
 }
+
+// Tiles up to which a block adds up the totals before it (4 per thread):
+// 4.2 M elements.  Two kernels then make a scan instead of three; at 480 k
+// elements 11.5 -> 8.4 us of device time and one launch fewer.
+constexpr int64_t kScanDirect = 2048;
 
 size_t scan_scratch_bytes(int64_t n) {
   size_t bytes = 0;
@@ -69,7 +86,7 @@ static int scan_impl(const TIn* in, int64_t* out, int64_t n, int64_t* total, cha
   }
   const int64_t blocks = (n + kScanTile - 1) / kScanTile;
   if (blocks == 1) {
-    scan_tile_apply<TIn><<<1, kScanBlock, 0, s>>>(in, out, n, nullptr, total, enable);
+    scan_tile_apply<TIn, false><<<1, kScanBlock, 0, s>>>(in, out, n, nullptr, total, enable);
     TSPH_LAUNCH_CHECK();
     return TSPH_OK;
   }
@@ -78,10 +95,16 @@ static int scan_impl(const TIn* in, int64_t* out, int64_t n, int64_t* total, cha
   char* next = scratch + 2 * align_up((blocks + 1) * sizeof(int64_t));
   scan_tile_totals<TIn><<<static_cast<unsigned>(blocks), kScanBlock, 0, s>>>(in, n, totals, enable);
   TSPH_LAUNCH_CHECK();
+  if (blocks <= kScanDirect) {
+    scan_tile_apply<TIn, true><<<static_cast<unsigned>(blocks), kScanBlock, 0, s>>>(in, out, n, totals, total,
+                                                                                    enable);
+    TSPH_LAUNCH_CHECK();
+    return TSPH_OK;
+  }
   int rc = scan_impl<int64_t>(totals, offsets, blocks, nullptr, next, s, enable);
   if (rc) return rc;
-  scan_tile_apply<TIn><<<static_cast<unsigned>(blocks), kScanBlock, 0, s>>>(in, out, n, offsets, total,
-                                                                            enable);
+  scan_tile_apply<TIn, false><<<static_cast<unsigned>(blocks), kScanBlock, 0, s>>>(in, out, n, offsets, total,
+                                                                                   enable);
   TSPH_LAUNCH_CHECK();
   return TSPH_OK;
 }
@@ -214,209 +237,13 @@ int radix_sort_u64_i32(uint64_t* keys, int32_t* vals, uint64_t* keys_tmp, int32_
 
 // ---------------------------------------------------------- segmented sort ---
 
-constexpr int kShortRow = 64;     // one warp, rank sort in shared memory
-constexpr int kMidRow = 1024;     // one 128-thread block, bitonic in shared memory
-constexpr int kMediumRow = 8192;  // one 512-thread block, bitonic in shared memory
-constexpr int kSortWarps = 8;
-
-struct SegsortLists {
-  int64_t* medium;
-  int64_t* long_rows;
-  int64_t* mid;
-  int64_t* counts;  // [0] medium, [1] long, [2] mid
-};
-
-__global__ void segsort_short(uint32_t* __restrict__ vals, const int64_t* __restrict__ rowptr,
-                              int64_t rows, SegsortLists lists) {
-  __shared__ uint32_t buf[kSortWarps][kShortRow];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int64_t r = static_cast<int64_t>(blockIdx.x) * kSortWarps + warp; r < rows;
-       r += static_cast<int64_t>(gridDim.x) * kSortWarps) {
-    const int64_t beg = rowptr[r], len = rowptr[r + 1] - beg;
-    if (len <= 1) continue;
-    if (len > kShortRow) {
-      if (lane == 0) {
-        if (len <= kMidRow)
-          lists.mid[atomicAdd(reinterpret_cast<unsigned long long*>(&lists.counts[2]), 1ull)] = r;
-        else if (len <= kMediumRow)
-          lists.medium[atomicAdd(reinterpret_cast<unsigned long long*>(&lists.counts[0]), 1ull)] = r;
-        else
-          lists.long_rows[atomicAdd(reinterpret_cast<unsigned long long*>(&lists.counts[1]), 1ull)] = r;
-      }
-      continue;
-    }
-    for (int k = lane; k < len; k += 32) buf[warp][k] = vals[beg + k];
-    __syncwarp();
-    for (int k = lane; k < len; k += 32) {
-      const uint32_t e = buf[warp][k];
-      int rank = 0;
-      for (int m = 0; m < len; ++m) {
-        const uint32_t f = buf[warp][m];
-        rank += (f < e) || (f == e && m < k);
-      }
-      vals[beg + rank] = e;
-    }
-    __syncwarp();
-  }
-}
-
-__device__ __forceinline__ void bitonic_smem(uint32_t* a, int p2) {
-  for (int k = 2; k <= p2; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int t = threadIdx.x; t < p2; t += blockDim.x) {
-        int ixj = t ^ j;
-        if (ixj > t) {
-          bool up = (t & k) == 0;
-          uint32_t x = a[t], y = a[ixj];
-          if ((x > y) == up) { a[t] = y; a[ixj] = x; }
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-// Rows of kShortRow + 1 .. kMidRow entries (the symmetric rows of a 3-D
-// pair list at h = 2 dx hold ~330): one warp per row, a bitonic network over
-// the row padded to p2 = 32 E entries held in registers, entry i = r * 32 +
-// lane in register r of its lane.  Stages at distances below 32 exchange
-// across lanes with shuffles, the others compare registers of one lane.
-template <int E>
-__device__ __forceinline__ void warp_bitonic(uint32_t* __restrict__ vals, int64_t beg, int64_t len) {
-  const int lane = threadIdx.x & 31;
-  uint32_t v[E];
-#pragma unroll
-  for (int r = 0; r < E; ++r) {
-    const int64_t i = static_cast<int64_t>(r) * 32 + lane;
-    v[r] = i < len ? vals[beg + i] : 0xffffffffu;
-  }
-#pragma unroll
-  for (int k = 2; k <= 32 * E; k <<= 1) {
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      if (j < 32) {
-        const bool lower = (lane & j) == 0;
-#pragma unroll
-        for (int r = 0; r < E; ++r) {
-          const int i = r * 32 + lane;
-          const bool asc = (i & k) == 0;
-          const uint32_t o = __shfl_xor_sync(0xffffffffu, v[r], j);
-          v[r] = (lower == asc) ? min(v[r], o) : max(v[r], o);
-        }
-      } else {
-        const int jr = j >> 5;
-#pragma unroll
-        for (int r = 0; r < E; ++r) {
-          if (r & jr) continue;
-          const int i = r * 32 + lane;
-          const bool asc = (i & k) == 0;
-          const uint32_t a = v[r], b = v[r | jr];
-          v[r] = asc ? min(a, b) : max(a, b);
-          v[r | jr] = asc ? max(a, b) : min(a, b);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < E; ++r) {
-    const int64_t i = static_cast<int64_t>(r) * 32 + lane;
-    if (i < len) vals[beg + i] = v[r];
-  }
-}
-
-__global__ void __launch_bounds__(256) segsort_mid(uint32_t* __restrict__ vals, const int64_t* __restrict__ rowptr,
-                                                   SegsortLists lists) {
-  const int64_t count = lists.counts[2];
-  const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t q = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); q < count;
-       q += warps) {
-    const int64_t r = lists.mid[q];
-    const int64_t beg = rowptr[r], len = rowptr[r + 1] - beg;
-    if (len <= 128)
-      warp_bitonic<4>(vals, beg, len);
-    else if (len <= 256)
-      warp_bitonic<8>(vals, beg, len);
-    else if (len <= 512)
-      warp_bitonic<16>(vals, beg, len);
-    else
-      warp_bitonic<32>(vals, beg, len);
-  }
-}
-
-__global__ void segsort_medium(uint32_t* __restrict__ vals, const int64_t* __restrict__ rowptr,
-                               SegsortLists lists) {
-  __shared__ uint32_t buf[kMediumRow];
-  const int64_t count = lists.counts[0];
-  for (int64_t q = blockIdx.x; q < count; q += gridDim.x) {
-    const int64_t r = lists.medium[q];
-    const int64_t beg = rowptr[r], len = rowptr[r + 1] - beg;
-    int p2 = 1;
-    while (p2 < len) p2 <<= 1;
-    for (int t = threadIdx.x; t < p2; t += blockDim.x) buf[t] = t < len ? vals[beg + t] : 0xffffffffu;
-    __syncthreads();
-    bitonic_smem(buf, p2);
-    for (int t = threadIdx.x; t < len; t += blockDim.x) vals[beg + t] = buf[t];
-    __syncthreads();
-  }
-}
-
-// Rows longer than kMediumRow: bitonic network directly on global memory,
-// one block per row.  The network is the all-ascending form (the first step
-// of each merge pairs t with t ^ (k - 1)), so the minimum always lands on
-// the lower index and the virtual +inf padding beyond `len` never moves --
-// no padded storage is needed.
-__global__ void segsort_long(uint32_t* __restrict__ vals, const int64_t* __restrict__ rowptr,
-                             SegsortLists lists) {
-  const int64_t count = lists.counts[1];
-  for (int64_t q = blockIdx.x; q < count; q += gridDim.x) {
-    const int64_t r = lists.long_rows[q];
-    const int64_t beg = rowptr[r], len = rowptr[r + 1] - beg;
-    int64_t p2 = 1;
-    while (p2 < len) p2 <<= 1;
-    uint32_t* a = vals + beg;
-    for (int64_t k = 2; k <= p2; k <<= 1) {
-      for (int64_t j = k >> 1; j > 0; j >>= 1) {
-        const int64_t mask = (j == (k >> 1)) ? (k - 1) : j;
-        for (int64_t t = threadIdx.x; t < p2; t += blockDim.x) {
-          const int64_t ixj = t ^ mask;
-          if (ixj > t && t < len && ixj < len) {
-            const uint32_t x = a[t], y = a[ixj];
-            if (x > y) {
-              a[t] = y;
-              a[ixj] = x;
-            }
-          }
-        }
-        __syncthreads();
-      }
-    }
-  }
-}
-
 size_t segsort_scratch_bytes(int64_t rows) {
-  return 3 * align_up(static_cast<size_t>(rows + 1) * sizeof(int64_t)) + 256;
+  return 2 * align_up(static_cast<size_t>(rows + 1) * sizeof(int64_t)) + 256;
 }
 
-int segmented_sort_u32(uint32_t* vals, const int64_t* rowptr, int64_t rows, void* scratch,
+int segmented_sort_u32(uint32_t* vals, const int64_t* rowptr, int64_t rows, int64_t entries, void* scratch,
                        cudaStream_t s) {
-  if (rows <= 0) return TSPH_OK;
-  char* sc = static_cast<char*>(scratch);
-  SegsortLists lists;
-  lists.counts = reinterpret_cast<int64_t*>(sc);
-  lists.medium = reinterpret_cast<int64_t*>(sc + 256);
-  lists.long_rows = reinterpret_cast<int64_t*>(sc + 256 + align_up((rows + 1) * sizeof(int64_t)));
-  lists.mid = reinterpret_cast<int64_t*>(sc + 256 + 2 * align_up((rows + 1) * sizeof(int64_t)));
-  TSPH_CUDA_CHECK(cudaMemsetAsync(lists.counts, 0, 3 * sizeof(int64_t), s));
-  unsigned g = grid_for(rows, kSortWarps, 148 * 16);
-  segsort_short<<<g, kSortWarps * 32, 0, s>>>(vals, rowptr, rows, lists);
-  TSPH_LAUNCH_CHECK();
-  segsort_mid<<<148 * 8, 256, 0, s>>>(vals, rowptr, lists);
-  TSPH_LAUNCH_CHECK();
-  segsort_medium<<<148 * 2, 512, 0, s>>>(vals, rowptr, lists);
-  TSPH_LAUNCH_CHECK();
-  segsort_long<<<148, 1024, 0, s>>>(vals, rowptr, lists);
-  TSPH_LAUNCH_CHECK();
-  return TSPH_OK;
+  return sort_rows(vals, CsrRows{rowptr}, rows, entries, InPlace{vals}, scratch, s);
 }
 
 }  // namespace tsph

@@ -152,9 +152,9 @@ int radix_sort_u64_i32(uint64_t* keys, int32_t* vals, uint64_t* keys_tmp, int32_
                        const int* enable = nullptr);
 
 // Sort every row segment [rowptr[r], rowptr[r+1]) of `vals` ascending (uint32
-// comparison).  Scratch: segsort_scratch_bytes.
+// comparison); `entries` bounds their total length.  Scratch: segsort_scratch_bytes.
 size_t segsort_scratch_bytes(int64_t rows);
-int segmented_sort_u32(uint32_t* vals, const int64_t* rowptr, int64_t rows, void* scratch,
+int segmented_sort_u32(uint32_t* vals, const int64_t* rowptr, int64_t rows, int64_t entries, void* scratch,
                        cudaStream_t s);
 
 }  // namespace tsph

@@ -1,0 +1,60 @@
+"""Symmetric gather rows of a pair list against numpy, at the edges of the
+builder's routes: sorted and unsorted lists, lists off a 16-byte boundary, rows
+of one to more than 65,536 entries, indices out of range."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SECOND = 1 << 31
+
+
+def expected_rows(pairs, n):
+    i = np.concatenate((pairs[:, 0], pairs[:, 1]))
+    e = np.concatenate((pairs[:, 1], pairs[:, 0] | SECOND))
+    ptr = np.zeros(n + 1, dtype=np.int64)
+    np.add.at(ptr, i + 1, 1)
+    return np.cumsum(ptr), e[np.lexsort((e, i))]
+
+
+def check(pairs, n, dev, odd=False):
+    from tensorsph_b200.droplet_impact import symmetric_rows
+    t = torch.from_numpy(np.ascontiguousarray(pairs, dtype=np.int64).reshape(-1, 2)).to(dev)
+    if odd:
+        flat = torch.zeros(t.numel() + 1, dtype=torch.int64, device=dev)
+        flat[1:] = t.reshape(-1)
+        t = flat[1:].view(-1, 2)
+    ptr, entries = symmetric_rows(t, n)
+    want_ptr, want = expected_rows(pairs.reshape(-1, 2), n)
+    assert np.array_equal(ptr.cpu().numpy(), want_ptr)
+    assert np.array_equal(entries.cpu().numpy()[:want.size].view(np.uint32).astype(np.int64), want)
+
+
+@pytest.mark.parametrize("n,count", [(1, 0), (5, 3), (300, 40), (2000, 30000), (50000, 900000), (700, 200000)])
+def test_rows_of_random_lists(gpu, n, count):
+    rng = np.random.default_rng(n)
+    p = rng.integers(0, n, (count, 2))
+    check(p, n, gpu)                                              # any order, both orientations, repeats
+    lex = p[np.lexsort((p[:, 1], p[:, 0]))]
+    check(lex, n, gpu)                                            # sorted, second index on either side
+    q = np.sort(p, axis=1)
+    check(q[np.lexsort((q[:, 1], q[:, 0]))], n, gpu, odd=True)    # sorted i <= j, off a 16-byte boundary
+
+
+@pytest.mark.parametrize("count", [15, 16, 17, 32, 33, 64, 65, 128, 129, 256, 257, 512, 513, 1024, 1025, 8192, 8193,
+                                   65536, 65537])
+def test_rows_at_the_sort_tiers(gpu, count):
+    """One row with ``count`` second-element entries, one with as many first-element
+    ones; the list sorted and reversed."""
+    hub = np.stack((np.arange(count), np.full(count, count)), axis=1)
+    fan = np.stack((np.zeros(count, dtype=np.int64), 1 + np.arange(count)), axis=1)
+    for p in (hub, fan, hub[::-1], fan[::-1]):
+        check(p, count + 1, gpu)
+
+
+@pytest.mark.parametrize("bad", [[[0, 1], [2, 9]], [[0, 9], [1, 2]], [[-1, 2], [0, 1]], [[5, 1], [0, 99]]])
+def test_rows_refuse_bad_indices(gpu, bad):
+    from tensorsph_b200.droplet_impact import symmetric_rows
+    with pytest.raises(ValueError):
+        symmetric_rows(torch.tensor(bad, dtype=torch.int64, device=gpu), 9)
