@@ -61,9 +61,10 @@ typedef struct {
   double box[3];      /* periodic box edges                                   */
   double width[3];    /* periodic cell width = box / ncell (in dtype)         */
   int64_t ncell[3];   /* cells per axis (open: max - min + 1)                 */
-  int64_t origin[3];  /* open grid: per-axis minimum of floor(x / cutoff)     */
+  int64_t origin[3];  /* open: least floor(x / cutoff); periodic: largest |x|
+                       * in cutoffs                                          */
   int64_t total_cells;
-  int64_t dense;      /* 1: dense cell table, 0: binary search over runs      */
+  int64_t dense;      /* 1: dense cell table, 0: bisection over the keys      */
   int64_t key_bits;   /* radix-sort width of the row-major cell key           */
   int64_t workspace_bytes;
 } tsph_grid;
@@ -79,8 +80,8 @@ int64_t tsph_grid_plan_scratch_bytes(void);
 int tsph_grid_plan(const void* pos, int64_t n, int64_t dim, int64_t dtype, double cutoff,
                    const double* box, void* scratch, tsph_grid* grid, tsph_stream stream);
 
-/* Cell keys, stable counting (radix) sort by key and the cell-run table.
- * order_out (nullable, n int64) receives the stable cell order -- the
+/* Particles by cell (counting sort, or a radix sort of the keys of a grid that
+ * is not dense).  order_out (nullable, n int64) receives the stable cell order -- the
  * permutation the reference obtains as argsort(inverse, stable=True). */
 int tsph_grid_build(const void* pos, const tsph_grid* grid, void* ws, int64_t ws_bytes,
                     int64_t* order_out, tsph_stream stream);
@@ -100,6 +101,17 @@ int64_t tsph_pairs_emit_workspace_bytes(int64_t pair_count, int64_t n);
 int tsph_pairs_emit(const void* pos, const tsph_grid* grid, int64_t row_limit, void* ws,
                     int64_t ws_bytes, void* emit_ws, int64_t emit_ws_bytes, int64_t* pairs,
                     int64_t pair_count, tsph_stream stream);
+
+/* The symmetric gather rows (see tsph_csr_from_pairs) of those pairs whose
+ * first index is below row_limit, without the list in between: after
+ * tsph_grid_build, tsph_rows_count writes rowptr (n + 1 int64) and returns the
+ * entry count on the host (synchronises), tsph_rows_emit writes the entries
+ * (entry_count uint32).  Same rows as tsph_csr_from_pairs makes of the list. */
+int tsph_rows_count(const void* pos, const tsph_grid* grid, int64_t row_limit, void* ws,
+                    int64_t ws_bytes, int64_t* rowptr, int64_t* entry_count, tsph_stream stream);
+int tsph_rows_emit(const void* pos, const tsph_grid* grid, int64_t row_limit, void* ws,
+                   int64_t ws_bytes, const int64_t* rowptr, uint32_t* entries, int64_t entry_count,
+                   tsph_stream stream);
 
 /* O(N^2) reference search, same contract (brute_force_pairs). */
 int64_t tsph_brute_workspace_bytes(int64_t n);

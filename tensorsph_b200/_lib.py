@@ -191,6 +191,10 @@ _SIGNATURES = {
     "tsph_pairs_emit_workspace_bytes": (c_int64, [c_int64, c_int64]),
     "tsph_pairs_emit": (c_int, [c_void_p, POINTER(Grid), c_int64, c_void_p, c_int64, c_void_p,
                                 c_int64, c_void_p, c_int64, c_void_p]),
+    "tsph_rows_count": (c_int, [c_void_p, POINTER(Grid), c_int64, c_void_p, c_int64, c_void_p,
+                                POINTER(c_int64), c_void_p]),
+    "tsph_rows_emit": (c_int, [c_void_p, POINTER(Grid), c_int64, c_void_p, c_int64, c_void_p,
+                               c_void_p, c_int64, c_void_p]),
     "tsph_brute_workspace_bytes": (c_int64, [c_int64]),
     "tsph_brute_pairs_count": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_double, c_void_p,
                                        c_int64, POINTER(c_int64), c_void_p]),

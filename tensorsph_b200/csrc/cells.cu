@@ -1,18 +1,35 @@
-// Linked-cell neighbour search: cell keys, stable counting (radix) sort by
-// cell, cell-run table and the exact pair emission of
-// neighbor_search.py:44-120 / threed/neighbors3.py:71-142.
+// Linked-cell neighbour search: cell keys, counting sort by cell and the exact
+// pair emission of neighbor_search.py:44-120 / threed/neighbors3.py:71-142.
 //
 // Bit-exactness with the reference rests on three arithmetic rules, all
 // applied with explicit round-to-nearest intrinsics (no FMA contraction):
 //   cell    = floor(x / cutoff)            IEEE division in the dtype
 //   d^2     = ((dx*dx) + dy*dy) + dz*dz    sequential, in the dtype
 //   accept  = d^2 <= (dtype)(cutoff^2)
-// and on the cell order being a stable sort by row-major key.
+// and, for cell_order, on the order being a stable sort by row-major key.
+//
+// Passes (dense grids):
+//   bounds -> [host: grid]
+//   cell_count   key of every particle, its slot in its cell by an atomic
+//   scan         first sorted position of every cell
+//   cell_scatter a 16-byte record (x, y, z in FP32 from the grid's corner, id)
+//                per particle, cell by cell
+//   scan_rows    per particle (in cell order) the neighbours among the
+//                candidates of its 3^D cells, into a fixed number of slots
+//   scan -> [host: list length]
+//   rows_sort    each row in index order, written out as pairs or gather rows
+// Where a row outgrows its slots, a second scan_rows writes the rows to their
+// places in the list before the sort.
+// A grid with far more cells than particles sorts its keys instead (radix) and
+// finds the cells by bisection.  The order inside a cell is arbitrary (slots
+// come from atomics) and does not show: rows are sorted by index.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
 #include "common.cuh"
 #include "fpmath.cuh"
+#include "rowsort.cuh"
 
 namespace tsph {
 
@@ -30,24 +47,32 @@ struct GridDev {
 };
 
 struct BuildWs {
-  int32_t* cell;       // n * dim, cell coordinates relative to origin
-  uint64_t* keys;      // n
+  uint64_t* keys;      // n (radix), or the key and slot of every particle (dense)
   uint64_t* keys_tmp;  // n
   int32_t* order;      // n (sorted position -> particle)
   int32_t* order_tmp;  // n
-  int32_t* flags;      // n
-  int64_t* run_of;     // n (sorted position -> run index)
-  int32_t* run_start;  // n + 1
-  uint64_t* run_key;   // n
-  int64_t* nruns;      // 1
-  int32_t* table;      // total_cells (dense) or 1
+  float4* rec;         // n, sorted: position from the grid's corner and the particle
+  int32_t* cell;       // n * dim, sorted: cell coordinates relative to origin
+  int32_t* counts;     // total_cells (dense) or 0, then
+  int32_t* longest;    // 1: 0, or the longest row when it has outgrown its slots
+  int64_t* start;      // total_cells + 1 (dense) or 1: first sorted position of a cell
   int64_t* rowptr;     // n + 1 (pair rows)
   int32_t* rowcount;   // n
-  int64_t* total;      // 1
+  uint32_t* slots;     // n * row_slots
   char* radix_scratch;
   char* scan_scratch;
   char* sort_scratch;
 };
+
+// Slots per row: a 3-D row of 2h + 0.25 h holds 104 neighbours, half of them
+// forward in lattice order and up to all in an arbitrary one; 27 in 2-D.
+constexpr int kSlots[4] = {0, 16, 48, 128};
+constexpr int64_t kSlotBytes = int64_t(4) << 30;  // a grid that would take more keeps none
+
+int64_t row_slots(const tsph_grid& g) {
+  const int64_t k = kSlots[g.dim];
+  return g.n * k * static_cast<int64_t>(sizeof(uint32_t)) <= kSlotBytes ? k : 0;
+}
 
 size_t build_layout(const tsph_grid& g, BuildWs* w, void* base) {
   const int64_t n = g.n;
@@ -58,23 +83,22 @@ size_t build_layout(const tsph_grid& g, BuildWs* w, void* base) {
     used += align_up(bytes);
     return p;
   };
+  const int64_t cells = g.dense ? g.total_cells : 1;
   BuildWs t{};
-  t.cell = reinterpret_cast<int32_t*>(take(n * g.dim * sizeof(int32_t)));
   t.keys = reinterpret_cast<uint64_t*>(take(n * sizeof(uint64_t)));
   t.keys_tmp = reinterpret_cast<uint64_t*>(take(n * sizeof(uint64_t)));
   t.order = reinterpret_cast<int32_t*>(take(n * sizeof(int32_t)));
   t.order_tmp = reinterpret_cast<int32_t*>(take(n * sizeof(int32_t)));
-  t.flags = reinterpret_cast<int32_t*>(take(n * sizeof(int32_t)));
-  t.run_of = reinterpret_cast<int64_t*>(take(n * sizeof(int64_t)));
-  t.run_start = reinterpret_cast<int32_t*>(take((n + 1) * sizeof(int32_t)));
-  t.run_key = reinterpret_cast<uint64_t*>(take(n * sizeof(uint64_t)));
-  t.nruns = reinterpret_cast<int64_t*>(take(sizeof(int64_t)));
-  t.table = reinterpret_cast<int32_t*>(take((g.dense ? g.total_cells : 1) * sizeof(int32_t)));
+  t.rec = reinterpret_cast<float4*>(take(n * sizeof(float4)));
+  t.cell = reinterpret_cast<int32_t*>(take(n * g.dim * sizeof(int32_t)));
+  t.counts = reinterpret_cast<int32_t*>(take((cells + 1) * sizeof(int32_t)));
+  t.longest = t.counts ? t.counts + (g.dense ? g.total_cells : 0) : nullptr;
+  t.start = reinterpret_cast<int64_t*>(take((cells + 1) * sizeof(int64_t)));
   t.rowptr = reinterpret_cast<int64_t*>(take((n + 1) * sizeof(int64_t)));
   t.rowcount = reinterpret_cast<int32_t*>(take(n * sizeof(int32_t)));
-  t.total = reinterpret_cast<int64_t*>(take(sizeof(int64_t)));
+  t.slots = reinterpret_cast<uint32_t*>(take(n * row_slots(g) * sizeof(uint32_t)));
   t.radix_scratch = take(radix_scratch_bytes(n));
-  t.scan_scratch = take(scan_scratch_bytes(n + 1));
+  t.scan_scratch = take(scan_scratch_bytes(std::max<int64_t>(n, cells) + 1));
   t.sort_scratch = take(segsort_scratch_bytes(n));
   if (w) *w = t;
   return used;
@@ -102,47 +126,66 @@ GridDev to_dev(const tsph_grid& g) {
 
 // ------------------------------------------------------------------ plan ---
 
+template <class F>
+int dispatch(int64_t dtype, int64_t dim, F&& f) {
+  if (dtype == TSPH_F32) {
+    if (dim == 1) return f(float{}, std::integral_constant<int, 1>{});
+    if (dim == 2) return f(float{}, std::integral_constant<int, 2>{});
+    if (dim == 3) return f(float{}, std::integral_constant<int, 3>{});
+  } else if (dtype == TSPH_F64) {
+    if (dim == 1) return f(double{}, std::integral_constant<int, 1>{});
+    if (dim == 2) return f(double{}, std::integral_constant<int, 2>{});
+    if (dim == 3) return f(double{}, std::integral_constant<int, 3>{});
+  }
+  return TSPH_ERR_ARG;
+}
+
+// out[0..2] smallest cell per axis, out[3..5] largest, out[6] 0 when some
+// coordinate is not finite.  All are unsigned minima, so one memset of ones
+// starts them: a cell is stored with its sign bit flipped, a largest one as
+// the complement of that.  One atomic per value and block: with one per warp
+// the 57 k atomics on six addresses took 43 us of 1 M FP64 particles, now 12.
 template <class T, int D>
-__global__ void bounds_kernel(const T* __restrict__ pos, int64_t n, T cutoff,
-                              long long* __restrict__ out /* min[3], max[3], nonfinite */) {
-  long long lo[D], hi[D];
-  int bad = 0;
+__global__ void __launch_bounds__(kBlock) bounds_kernel(const T* __restrict__ pos, int64_t n, T cutoff,
+                                                        unsigned long long* __restrict__ out) {
+  constexpr unsigned long long kSign = 1ull << 63;
+  constexpr int kWarps = kBlock / 32;
+  __shared__ unsigned long long red[kWarps][2 * D + 1];
+  unsigned long long v[2 * D + 1];
 #pragma unroll
-  for (int k = 0; k < D; ++k) { lo[k] = LLONG_MAX; hi[k] = LLONG_MIN; }
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
+  for (int k = 0; k <= 2 * D; ++k) v[k] = ~0ull;
+  for (int64_t a = blockIdx.x * static_cast<int64_t>(kBlock) + threadIdx.x; a < n;
+       a += static_cast<int64_t>(gridDim.x) * kBlock) {
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-      T x = pos[a * D + k];
-      if (!isfinite(x)) { bad = 1; continue; }
-      long long c = static_cast<long long>(floor(fp<T>::div(x, cutoff)));
-      lo[k] = c < lo[k] ? c : lo[k];
-      hi[k] = c > hi[k] ? c : hi[k];
+      const T x = pos[a * D + k];
+      if (!isfinite(x)) { v[2 * D] = 0; continue; }
+      const unsigned long long c =
+          static_cast<unsigned long long>(static_cast<long long>(floor(fp<T>::div(x, cutoff)))) ^ kSign;
+      v[k] = c < v[k] ? c : v[k];
+      v[D + k] = ~c < v[D + k] ? ~c : v[D + k];
     }
   }
 #pragma unroll
-  for (int k = 0; k < D; ++k) {
+  for (int k = 0; k <= 2 * D; ++k) {
     for (int o = 16; o > 0; o >>= 1) {
-      long long l2 = __shfl_xor_sync(0xffffffffu, lo[k], o);
-      long long h2 = __shfl_xor_sync(0xffffffffu, hi[k], o);
-      lo[k] = l2 < lo[k] ? l2 : lo[k];
-      hi[k] = h2 > hi[k] ? h2 : hi[k];
+      const unsigned long long w = __shfl_xor_sync(0xffffffffu, v[k], o);
+      v[k] = w < v[k] ? w : v[k];
     }
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][k] = v[k];
   }
-  bad = __any_sync(0xffffffffu, bad);
-  if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-      atomicMin(&out[k], lo[k]);
-      atomicMax(&out[3 + k], hi[k]);
-    }
-    if (bad) atomicOr(reinterpret_cast<unsigned long long*>(&out[6]), 1ull);
+  __syncthreads();
+  if (threadIdx.x <= 2 * D) {
+    const int k = threadIdx.x;
+    unsigned long long m = red[0][k];
+    for (int w = 1; w < kWarps; ++w) m = red[w][k] < m ? red[w][k] : m;
+    if (m != ~0ull) atomicMin(&out[k < D ? k : (k < 2 * D ? 3 + k - D : 6)], m);
   }
 }
 
 template <class T, int D>
-int plan_bounds(const void* pos, int64_t n, double cutoff, long long* dev, cudaStream_t s) {
-  long long init[8] = {LLONG_MAX, LLONG_MAX, LLONG_MAX, LLONG_MIN, LLONG_MIN, LLONG_MIN, 0, 0};
-  TSPH_CUDA_CHECK(cudaMemcpyAsync(dev, init, sizeof(init), cudaMemcpyHostToDevice, s));
+int plan_bounds(const void* pos, int64_t n, double cutoff, unsigned long long* dev, cudaStream_t s) {
+  TSPH_CUDA_CHECK(cudaMemsetAsync(dev, 0xff, 8 * sizeof(unsigned long long), s));
   bounds_kernel<T, D><<<grid_for(n, kBlock, 148 * 8), kBlock, 0, s>>>(
       static_cast<const T*>(pos), n, static_cast<T>(cutoff), dev);
   TSPH_LAUNCH_CHECK();
@@ -151,66 +194,89 @@ int plan_bounds(const void* pos, int64_t n, double cutoff, long long* dev, cudaS
 
 // ----------------------------------------------------------------- build ---
 
+// Cell of one coordinate (relative to the grid's origin, or wrapped into the
+// box) and the coordinate from the grid's corner, moved by whole boxes into
+// the same cell when periodic.
+template <class T>
+__device__ __forceinline__ long long cell_of(T x, const GridDev& g, int k, float* local) {
+  if (g.periodic) {
+    const long long raw = static_cast<long long>(floor(fp<T>::div(x, static_cast<T>(g.width[k]))));
+    long long c = raw % g.ncell[k];
+    if (c < 0) c += g.ncell[k];
+    if (local)
+      *local = static_cast<float>(static_cast<double>(x) - static_cast<double>((raw - c) / g.ncell[k]) *
+                                                               static_cast<double>(static_cast<T>(g.box[k])));
+    return c;
+  }
+  if (local) *local = static_cast<float>(static_cast<double>(x) - static_cast<double>(g.origin[k]) * g.cutoff);
+  return static_cast<long long>(floor(fp<T>::div(x, static_cast<T>(g.cutoff)))) - g.origin[k];
+}
+
 template <class T, int D>
-__global__ void key_kernel(const T* __restrict__ pos, int64_t n, GridDev g, int32_t* __restrict__ cell,
-                           uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-    uint64_t key = 0;
+__device__ __forceinline__ uint64_t key_of(const T* __restrict__ pos, int64_t a, const GridDev& g, int* c, float* local) {
+  uint64_t key = 0;
 #pragma unroll
-    for (int k = 0; k < D; ++k) {
-      T x = pos[a * D + k];
-      long long c;
-      if (g.periodic) {
-        c = static_cast<long long>(floor(fp<T>::div(x, static_cast<T>(g.width[k]))));
-        c %= g.ncell[k];
-        if (c < 0) c += g.ncell[k];
-      } else {
-        c = static_cast<long long>(floor(fp<T>::div(x, static_cast<T>(g.cutoff)))) - g.origin[k];
-      }
-      cell[a * D + k] = static_cast<int32_t>(c);
-      key += static_cast<uint64_t>(c) * static_cast<uint64_t>(g.stride[k]);
-    }
-    keys[a] = key;
+  for (int k = 0; k < D; ++k) {
+    const long long ck = cell_of<T>(pos[a * D + k], g, k, local ? local + k : nullptr);
+    if (c) c[k] = static_cast<int>(ck);
+    key += static_cast<uint64_t>(ck) * static_cast<uint64_t>(g.stride[k]);
+  }
+  return key;
+}
+
+template <class T, int D>
+__global__ void key_kernel(const T* __restrict__ pos, int64_t n, GridDev g, uint64_t* __restrict__ keys,
+                           int32_t* __restrict__ vals) {
+  for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n;
+       a += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    keys[a] = key_of<T, D>(pos, a, g, nullptr, nullptr);
     vals[a] = static_cast<int32_t>(a);
   }
 }
 
-__global__ void run_flags(const uint64_t* __restrict__ keys, int64_t n, int32_t* __restrict__ flags) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x)
-    flags[a] = (a == 0 || keys[a] != keys[a - 1]) ? 1 : 0;
+// The slot of every particle in its cell.  2 x 4 bytes a particle instead of
+// the radix sort's 24 per digit, and four launches instead of five per digit.
+template <class T, int D>
+__global__ void cell_count(const T* __restrict__ pos, int64_t n, GridDev g, int32_t* __restrict__ counts,
+                           int32_t* __restrict__ slots) {
+  for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n;
+       a += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    slots[a] = atomicAdd(&counts[key_of<T, D>(pos, a, g, nullptr, nullptr)], 1);
 }
 
-__global__ void run_fill(const uint64_t* __restrict__ keys, const int32_t* __restrict__ flags,
-                         const int64_t* __restrict__ run_incl_excl, int64_t n,
-                         int32_t* __restrict__ run_start, uint64_t* __restrict__ run_key,
-                         int32_t* __restrict__ table, int dense, const int64_t* __restrict__ nruns) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-    if (flags[a]) {
-      int64_t r = run_incl_excl[a];
-      run_start[r] = static_cast<int32_t>(a);
-      run_key[r] = keys[a];
-      if (dense) table[keys[a]] = static_cast<int32_t>(r);
-    }
-    if (a == 0) run_start[*nruns] = static_cast<int32_t>(n);
+// Records in cell order: to start[key] + slot (dense), or from the sorted order.
+template <class T, int D, bool kDense>
+__global__ void cell_scatter(const T* __restrict__ pos, int64_t n, GridDev g, const int64_t* __restrict__ start,
+                             const int32_t* __restrict__ slots, const int32_t* __restrict__ order,
+                             float4* __restrict__ rec, int32_t* __restrict__ cell) {
+  for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < n;
+       t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t a = kDense ? t : order[t];
+    int c[D];
+    float x[3] = {0.f, 0.f, 0.f};
+    const uint64_t key = key_of<T, D>(pos, a, g, c, x);
+    const int64_t at = kDense ? start[key] + slots[a] : t;
+    rec[at] = make_float4(x[0], x[1], x[2], __int_as_float(static_cast<int>(a)));
+#pragma unroll
+    for (int k = 0; k < D; ++k) cell[at * D + k] = c[k];
   }
 }
 
 __global__ void order_to_i64(const int32_t* __restrict__ order, int64_t n, int64_t* __restrict__ out) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x)
+  for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n;
+       a += static_cast<int64_t>(gridDim.x) * blockDim.x)
     out[a] = order[a];
 }
 
 // --------------------------------------------------------------- pairs ---
 
-__device__ __forceinline__ int64_t find_run(uint64_t key, const int32_t* __restrict__ table, int dense,
-                                            const uint64_t* __restrict__ run_key, int64_t nruns) {
-  if (dense) return table[key];
-  int64_t lo = 0, hi = nruns;
+__device__ __forceinline__ int64_t lower_bound(const uint64_t* __restrict__ keys, int64_t n, uint64_t key) {
+  int64_t lo = 0, hi = n;
   while (lo < hi) {
-    int64_t mid = (lo + hi) >> 1;
-    if (run_key[mid] < key) lo = mid + 1; else hi = mid;
+    const int64_t mid = (lo + hi) >> 1;
+    if (keys[mid] < key) lo = mid + 1; else hi = mid;
   }
-  return (lo < nruns && run_key[lo] == key) ? lo : -1;
+  return lo;
 }
 
 template <class T, int D>
@@ -226,66 +292,269 @@ __device__ __forceinline__ T pair_d2(const T* __restrict__ pos, int64_t a, int64
   return acc;
 }
 
-// MODE 0: count rows; MODE 1: emit unsorted rows into out (uint32).
-template <class T, int D, int MODE>
-__global__ void pair_kernel(const T* __restrict__ pos, int64_t n, int64_t row_limit, GridDev g,
-                            const int32_t* __restrict__ cell, const int32_t* __restrict__ order,
-                            const int32_t* __restrict__ run_start, const uint64_t* __restrict__ run_key,
-                            const int64_t* __restrict__ nruns_p, const int32_t* __restrict__ table,
-                            T c2, int32_t* __restrict__ rowcount, const int64_t* __restrict__ rowptr,
-                            uint32_t* __restrict__ out) {
-  const int64_t nruns = *nruns_p;
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-    int32_t count = 0;
-    int64_t slot = MODE == 1 ? rowptr[a] : 0;
-    if (a < row_limit) {
-      int c[3] = {0, 0, 0};
+// Which candidates the FP32 records decide.  A record's coordinate is within
+// 2^-24 of the extent of its true value (and so is an image's shift), so a
+// distance taken from two of them in FP32, and the reference's own distance in
+// its dtype, differ by less than w = 2^-20 extent + 2e-6 cutoff.  Below
+// (cutoff - w)^2 a candidate is in, above (cutoff + w)^2 it is out; between
+// them (about one candidate in 10^4) the reference's arithmetic on the given
+// positions decides.  Where the band would be wide (coordinates many thousand
+// cutoffs from the corner), or a periodic axis has three cells, so that a
+// stencil cell's image need not be the nearest one, every candidate takes the
+// reference's arithmetic.
+struct Band {
+  float in, out;
+};
+
+Band band_of(const tsph_grid& g) {
+  double extent = 0.0;
+  bool exact = false;
+  for (int k = 0; k < g.dim; ++k) {
+    if (g.periodic) {
+      extent = std::max(extent, std::max(g.box[k], 2.0 * static_cast<double>(g.origin[k]) * g.cutoff));
+      if (g.ncell[k] < 4) exact = true;
+    } else {
+      extent = std::max(extent, static_cast<double>(g.ncell[k]) * g.cutoff);
+    }
+  }
+  const double w = extent / 1048576.0 + 2e-6 * g.cutoff;
+  if (exact || !(w < 0.25 * g.cutoff) || g.cutoff * g.cutoff < 1e-30 || extent > 1e15)
+    return Band{-1.f, INFINITY};
+  const double lo = g.cutoff - w, hi = g.cutoff + w;
+  return Band{static_cast<float>(lo * lo * (1.0 - 1e-6)), static_cast<float>(hi * hi * (1.0 + 1e-6))};
+}
+
+struct Cells {
+  const float4* rec;
+  const int32_t* cell;
+  const int64_t* start;   // dense
+  const uint64_t* keys;   // not dense: sorted
+};
+
+// What a row holds: kForward b > a (the list's pairs (a, b)); kBoth every
+// neighbour whose pair's first index is below the limit, as gather-row entries
+// (b, with the top bit when a is the pair's second element).
+enum RowKind { kForward, kBoth };
+enum RowPass { kCount, kSlot, kFill };
+
+// The rows of all particles, thread per row (kLanes = 1) or kLanes lanes per
+// row, in cell order, so that the lanes of a warp walk the same cells.  The
+// cells c - 1 .. c + 1 of the last axis are consecutive keys: a column's
+// candidates are one run (two at a periodic seam), 3^(D-1) runs in all.
+// kCount counts them, kSlot also writes the first `slots` of each row to its
+// slots (in any order) and raises `longest` where that was not all, kFill, run
+// when it was raised, writes the rows from rowptr on.
+//
+// What bounds it: instruction issue (6 FP32 operations, the record load and
+// the tests per candidate; the 3-D list at 2.05 h scans ~500 candidates for
+// ~80 hits) and, with the stores of kSlot, scattered 4-byte writes.  1.0 M FP64
+// particles in 3-D: 0.54 ms (0.39 when it only counts), against 1.55 ms to
+// count and 1.65 to write with a thread per particle in the caller's order,
+// FP64 distances for every candidate and 27 cells by division.
+template <class T, int D, RowKind kKind, RowPass kPass, int kLanes>
+__global__ void __launch_bounds__(128) scan_rows(const T* __restrict__ pos, int64_t n, int64_t row_limit, GridDev g,
+                                                 Cells cs, Band band, T c2, int32_t* __restrict__ rowcount,
+                                                 const int64_t* __restrict__ rowptr, uint32_t* __restrict__ out,
+                                                 int slots, int* longest) {
+  if (kPass == kFill && *longest <= slots) return;
+  constexpr int kColumns = D == 1 ? 1 : (D == 2 ? 3 : 9);
+  constexpr uint32_t kSecond = 0x80000000u;
+  const int lane = threadIdx.x & 31, gl = lane & (kLanes - 1);
+  const unsigned group = kLanes == 1 ? 1u << lane : ((kLanes == 32 ? 0u : 1u << kLanes) - 1u) << (lane - gl);
+  const int64_t t = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / kLanes;
+  if (t >= n) return;
+  const float4 ra = cs.rec[t];
+  const int64_t a = __float_as_int(ra.w);
+  if (kKind == kForward && kPass == kFill && a >= row_limit) return;
+  int c[3] = {0, 0, 0};
 #pragma unroll
-      for (int k = 0; k < D; ++k) c[k] = cell[a * D + k];
-      constexpr int M = D == 1 ? 3 : (D == 2 ? 9 : 27);
-      for (int m = 0; m < M; ++m) {
-        int off[3] = {m % 3 - 1, (m / 3) % 3 - 1, (m / 9) % 3 - 1};
-        uint64_t key = 0;
-        bool inside = true;
+  for (int k = 0; k < D; ++k) c[k] = cs.cell[t * D + k];
+  const float xa[3] = {ra.x, ra.y, ra.z};
+  int count = 0;
+  const int64_t slot = kPass == kFill ? rowptr[a] : a * slots;
+
+  const int me = static_cast<int>(a), limit = static_cast<int>(row_limit);
+  const bool first = me < limit;  // kBoth: a row below the limit takes every neighbour
+  const T* __restrict__ px = pos;
+  auto put = [&](int at, int b) {
+    if (kPass == kSlot && at >= slots) return;
+    out[slot + at] = kKind == kBoth && b < me ? static_cast<uint32_t>(b) | kSecond : static_cast<uint32_t>(b);
+  };
+  // kBatch candidates at once: the tests against the outer bound are predicates,
+  // and one branch per batch looks at those between the bounds
+  auto run = [&](int beg, int end, float x, float y, float z) {
+    constexpr int kBatch = kLanes == 1 ? 4 : 1;
+    for (int p0 = beg; p0 < end; p0 += kBatch * kLanes) {
+      float4 rb[kBatch];
+      bool hit[kBatch];
+      bool unsure = false;
 #pragma unroll
-        for (int k = 0; k < D; ++k) {
-          long long nc = static_cast<long long>(c[k]) + off[k];
-          if (g.periodic) {
-            nc = (nc + g.ncell[k]) % g.ncell[k];
-          } else if (nc < 0 || nc >= g.ncell[k]) {
-            inside = false;
-          }
-          key += static_cast<uint64_t>(nc) * static_cast<uint64_t>(g.stride[k]);
+      for (int j = 0; j < kBatch; ++j) rb[j] = cs.rec[min(p0 + j + gl, end - 1)];
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j) {
+        const int b = __float_as_int(rb[j].w);
+        const float dx = x - rb[j].x, dy = y - rb[j].y, dz = z - rb[j].z;
+        float d2 = dx * dx;
+        if (D > 1) d2 = fmaf(dy, dy, d2);
+        if (D > 2) d2 = fmaf(dz, dz, d2);
+        const bool want = kKind == kForward ? b > me : b != me && (first || b < limit);
+        hit[j] = d2 < band.out && want && p0 + j + gl < end;
+        unsure |= hit[j] && d2 > band.in;
+      }
+      if (unsure) {
+#pragma unroll
+        for (int j = 0; j < kBatch; ++j)
+          if (hit[j]) hit[j] = pair_d2<T, D>(px, a, __float_as_int(rb[j].w), g) <= c2;
+      }
+      if (kLanes == 1) {
+#pragma unroll
+        for (int j = 0; j < kBatch; ++j) {
+          if (kPass != kCount && hit[j]) put(count, __float_as_int(rb[j].w));
+          count += hit[j];
         }
-        if (!inside) continue;
-        int64_t r = find_run(key, table, g.dense, run_key, nruns);
-        if (r < 0) continue;
-        const int32_t beg = run_start[r], end = run_start[r + 1];
-        for (int32_t p = beg; p < end; ++p) {
-          const int32_t b = order[p];
-          if (b <= a) continue;
-          if (pair_d2<T, D>(pos, a, b, g) <= c2) {
-            if (MODE == 1) out[slot + count] = static_cast<uint32_t>(b);
-            ++count;
-          }
-        }
+      } else if (kPass != kCount) {
+        const unsigned m = __ballot_sync(group, hit[0]) & group;
+        if (hit[0]) put(count + __popc(m & ((1u << lane) - 1u)), __float_as_int(rb[0].w));
+        count += __popc(m);
+      } else {
+        count += hit[0];
       }
     }
-    if (MODE == 0) rowcount[a] = count;
+  };
+  // first sorted position of cells [k0, k1] of the key space
+  auto cells = [&](int64_t k0, int64_t k1, float x, float y, float z) {
+    int64_t beg, end;
+    if (g.dense) {
+      beg = cs.start[k0];
+      end = cs.start[k1 + 1];
+    } else {
+      beg = lower_bound(cs.keys, n, static_cast<uint64_t>(k0));
+      end = lower_bound(cs.keys, n, static_cast<uint64_t>(k1) + 1);
+    }
+    run(static_cast<int>(beg), static_cast<int>(end), x, y, z);
+  };
+
+#pragma unroll 1
+  for (int m = 0; m < kColumns; ++m) {
+    const int off[2] = {m % 3 - 1, m / 3 - 1};
+    float x[3] = {xa[0], xa[1], xa[2]};
+    int64_t column = 0;
+    bool inside = true;
+#pragma unroll
+    for (int k = 0; k + 1 < D; ++k) {
+      int64_t nc = c[k] + off[k];
+      if (g.periodic) {
+        if (nc < 0) { nc += g.ncell[k]; x[k] += static_cast<float>(g.box[k]); }
+        else if (nc >= g.ncell[k]) { nc -= g.ncell[k]; x[k] -= static_cast<float>(g.box[k]); }
+      } else if (nc < 0 || nc >= g.ncell[k]) {
+        inside = false;
+      }
+      column += nc * g.stride[k];
+    }
+    if (!inside) continue;
+    const int64_t last = g.ncell[D - 1] - 1;
+    const int64_t z0 = c[D - 1] > 0 ? c[D - 1] - 1 : 0, z1 = c[D - 1] < last ? c[D - 1] + 1 : last;
+    cells(column + z0, column + z1, x[0], x[1], x[2]);
+    if (g.periodic) {
+      const float edge = static_cast<float>(g.box[D - 1]);
+      if (c[D - 1] == 0) {
+        x[D - 1] += edge;
+        cells(column + last, column + last, x[0], x[1], x[2]);
+        x[D - 1] -= edge;
+      }
+      if (c[D - 1] == last) {
+        x[D - 1] -= edge;
+        cells(column, column, x[0], x[1], x[2]);
+      }
+    }
+  }
+  if (kPass != kFill) {
+    if (kPass == kCount && kLanes > 1) {
+#pragma unroll
+      for (int o = kLanes / 2; o > 0; o >>= 1) count += __shfl_xor_sync(group, count, o);
+    }
+    if (gl == 0) {
+      rowcount[a] = count;
+      if (kPass == kSlot && count > slots) atomicMax(longest, count);
+    }
   }
 }
 
-__global__ void expand_pairs(const int64_t* __restrict__ rowptr, const uint32_t* __restrict__ cols,
-                             int64_t n, int64_t* __restrict__ pairs) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t a = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; a < n; a += warps) {
-    const int64_t beg = rowptr[a], end = rowptr[a + 1];
-    for (int64_t p = beg + lane; p < end; p += 32) {
-      pairs[2 * p] = a;
-      pairs[2 * p + 1] = cols[p];
-    }
+// Rows up to which eight lanes share a row: a row per thread leaves most of the
+// chip idle there, eight lanes leave a sixth of theirs idle in every run.  Whole
+// searches (FP32, 3-D, 2.05 h) with eight lanes / one: 8 k particles 132 / 156
+// us, 20 k 137 / 144, 40 k 177 / 154, 100 k 281 / 205; 2-D: the same up to 20 k,
+// 123 / 116 at 40 k.
+constexpr int64_t kLaneRows = 24576;
+
+template <class T, int D, RowKind kKind, RowPass kPass>
+int launch_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, const BuildWs& w, const int64_t* rowptr,
+                uint32_t* out, cudaStream_t s) {
+  const int64_t n = grid.n;
+  const Cells cs{w.rec, w.cell, w.start, w.keys};
+  const T c2 = static_cast<T>(grid.cutoff * grid.cutoff);
+  const T* p = static_cast<const T*>(pos);
+  const int slots = static_cast<int>(row_slots(grid));
+  if (n <= kLaneRows)
+    scan_rows<T, D, kKind, kPass, 8><<<static_cast<unsigned>((n * 8 + 127) / 128), 128, 0, s>>>(
+        p, n, row_limit, to_dev(grid), cs, band_of(grid), c2, w.rowcount, rowptr, out, slots, w.longest);
+  else
+    scan_rows<T, D, kKind, kPass, 1><<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(
+        p, n, row_limit, to_dev(grid), cs, band_of(grid), c2, w.rowcount, rowptr, out, slots, w.longest);
+  TSPH_LAUNCH_CHECK();
+  return TSPH_OK;
+}
+
+// Whether the rows are worth slots: not where the mean row of a full grid
+// already comes near them (most rows would be scanned twice and written twice).
+template <RowKind kKind>
+bool use_slots(const tsph_grid& g) {
+  const double ball[4] = {0.0, 2.0, 3.1416, 4.1888};
+  const double mean = ball[g.dim] * static_cast<double>(g.n) / static_cast<double>(g.total_cells) *
+                      (kKind == kForward ? 0.5 : 1.0);
+  return static_cast<double>(row_slots(g)) > 1.2 * mean;
+}
+
+// Row lengths (and the rows in their slots), scanned into rowptr.
+template <RowKind kKind>
+int count_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, const BuildWs& w, int64_t* rowptr,
+               cudaStream_t s) {
+  const bool slots = use_slots<kKind>(grid);
+  // without slots every row has outgrown them
+  TSPH_CUDA_CHECK(cudaMemsetAsync(w.longest, slots ? 0 : 0x7f, sizeof(int), s));
+  int rc = dispatch(grid.dtype, grid.dim, [&](auto t, auto d) {
+    using T = decltype(t);
+    constexpr int D = decltype(d)::value;
+    return slots ? launch_rows<T, D, kKind, kSlot>(pos, grid, row_limit, w, nullptr, w.slots, s)
+                 : launch_rows<T, D, kKind, kCount>(pos, grid, row_limit, w, nullptr, nullptr, s);
+  });
+  if (rc) return rc;
+  return exclusive_scan_i32_to_i64(w.rowcount, rowptr, grid.n, rowptr + grid.n, w.scan_scratch, s);
+}
+
+// The rows in their slots, or in `full` when some row has outgrown them.
+struct FoundRows {
+  uint32_t *slot, *full;
+  const int64_t* ptr;
+  const int* longest;
+  int slots;
+  __device__ __forceinline__ uint32_t* src(int64_t r) const {
+    return *longest > slots ? full + ptr[r] : slot + r * slots;
   }
+  __device__ __forceinline__ int64_t dst(int64_t r) const { return ptr[r]; }
+  __device__ __forceinline__ int64_t len(int64_t r) const { return ptr[r + 1] - ptr[r]; }
+};
+
+// The first `rows` rows sorted into out; `full`: room for their `count` entries.
+template <RowKind kKind, class Out>
+int emit_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, int64_t rows, const BuildWs& w,
+              const int64_t* rowptr, uint32_t* full, int64_t count, Out out, cudaStream_t s) {
+  int rc = dispatch(grid.dtype, grid.dim, [&](auto t, auto d) {
+    return launch_rows<decltype(t), decltype(d)::value, kKind, kFill>(pos, grid, row_limit, w, rowptr, full, s);
+  });
+  if (rc) return rc;
+  return sort_rows(FoundRows{w.slots, full, rowptr, w.longest, static_cast<int>(row_slots(grid))}, rows, count, out,
+                   w.sort_scratch, s);
 }
 
 // --------------------------------------------------------- brute force ---
@@ -333,20 +602,6 @@ __global__ void displacement_kernel(const T* __restrict__ pos, const T* __restri
   if ((threadIdx.x & 31) == 0) atomicMax(out, static_cast<unsigned long long>(__double_as_longlong(best)));
 }
 
-template <class F>
-int dispatch(int64_t dtype, int64_t dim, F&& f) {
-  if (dtype == TSPH_F32) {
-    if (dim == 1) return f(float{}, std::integral_constant<int, 1>{});
-    if (dim == 2) return f(float{}, std::integral_constant<int, 2>{});
-    if (dim == 3) return f(float{}, std::integral_constant<int, 3>{});
-  } else if (dtype == TSPH_F64) {
-    if (dim == 1) return f(double{}, std::integral_constant<int, 1>{});
-    if (dim == 2) return f(double{}, std::integral_constant<int, 2>{});
-    if (dim == 3) return f(double{}, std::integral_constant<int, 3>{});
-  }
-  return TSPH_ERR_ARG;
-}
-
 template <class T>
 T host_cutoff_sq(double cutoff) {
   return static_cast<T>(cutoff * cutoff);
@@ -375,16 +630,21 @@ int tsph_grid_plan(const void* pos, int64_t n, int64_t dim, int64_t dtype, doubl
   grid->dtype = dtype;
   grid->cutoff = cutoff;
   grid->periodic = box != nullptr;
-  long long host[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  long long host[6] = {0, 0, 0, 0, 0, 0};
   if (n > 0) {
-    long long* dev = static_cast<long long*>(scratch);
+    unsigned long long* dev = static_cast<unsigned long long*>(scratch);
+    unsigned long long raw[8];
     int rc = dispatch(dtype, dim, [&](auto t, auto d) {
       return plan_bounds<decltype(t), decltype(d)::value>(pos, n, cutoff, dev, s);
     });
     if (rc) return rc;
-    TSPH_CUDA_CHECK(cudaMemcpyAsync(host, dev, sizeof(host), cudaMemcpyDeviceToHost, s));
+    TSPH_CUDA_CHECK(cudaMemcpyAsync(raw, dev, sizeof(raw), cudaMemcpyDeviceToHost, s));
     TSPH_CUDA_CHECK(cudaStreamSynchronize(s));
-    if (host[6]) return TSPH_ERR_NONFINITE;
+    if (raw[6] == 0) return TSPH_ERR_NONFINITE;
+    for (int k = 0; k < dim; ++k) {
+      host[k] = static_cast<long long>(raw[k] ^ (1ull << 63));
+      host[3 + k] = static_cast<long long>(~raw[3 + k] ^ (1ull << 63));
+    }
   }
   double cells = 1.0;
   for (int k = 0; k < 3; ++k) {
@@ -407,6 +667,9 @@ int tsph_grid_plan(const void* pos, int64_t n, int64_t dim, int64_t dtype, doubl
         grid->width[k] = box[k] / static_cast<double>(nc);
       }
       grid->ncell[k] = nc;
+      // a wrapped grid has no origin: how far the positions reach, in cutoffs
+      const double reach = std::max(std::fabs(static_cast<double>(host[k])), std::fabs(static_cast<double>(host[3 + k]) + 1.0));
+      grid->origin[k] = static_cast<int64_t>(std::min(reach, 4.0e18));
     } else {
       grid->origin[k] = n > 0 ? host[k] : 0;
       grid->ncell[k] = n > 0 ? host[3 + k] - host[k] + 1 : 1;
@@ -435,31 +698,44 @@ int tsph_grid_build(const void* pos, const tsph_grid* grid, void* ws, int64_t ws
   BuildWs w;
   build_layout(*grid, &w, ws);
   GridDev g = to_dev(*grid);
-  int rc = dispatch(grid->dtype, grid->dim, [&](auto t, auto d) {
+  const bool sorted = !grid->dense || order_out != nullptr;
+  int rc = TSPH_OK;
+  if (sorted) {
+    rc = dispatch(grid->dtype, grid->dim, [&](auto t, auto d) {
+      using T = decltype(t);
+      key_kernel<T, decltype(d)::value><<<grid_for(n, kBlock), kBlock, 0, s>>>(static_cast<const T*>(pos), n, g,
+                                                                               w.keys, w.order);
+      TSPH_LAUNCH_CHECK();
+      return TSPH_OK;
+    });
+    if (rc) return rc;
+    rc = radix_sort_u64_i32(w.keys, w.order, w.keys_tmp, w.order_tmp, n, static_cast<int>(grid->key_bits),
+                            w.radix_scratch, s);
+    if (rc) return rc;
+    if (order_out) {
+      order_to_i64<<<grid_for(n, kBlock), kBlock, 0, s>>>(w.order, n, order_out);
+      TSPH_LAUNCH_CHECK();
+    }
+  }
+  int32_t* slots = w.order_tmp;
+  if (grid->dense) TSPH_CUDA_CHECK(cudaMemsetAsync(w.counts, 0, grid->total_cells * sizeof(int32_t), s));
+  return dispatch(grid->dtype, grid->dim, [&](auto t, auto d) -> int {
     using T = decltype(t);
-    key_kernel<T, decltype(d)::value><<<grid_for(n, kBlock), kBlock, 0, s>>>(
-        static_cast<const T*>(pos), n, g, w.cell, w.keys, w.order);
+    constexpr int D = decltype(d)::value;
+    const T* p = static_cast<const T*>(pos);
+    if (grid->dense) {
+      cell_count<T, D><<<grid_for(n, kBlock), kBlock, 0, s>>>(p, n, g, w.counts, slots);
+      TSPH_LAUNCH_CHECK();
+      int rc2 = exclusive_scan_i32_to_i64(w.counts, w.start, grid->total_cells, w.start + grid->total_cells,
+                                          w.scan_scratch, s);
+      if (rc2) return rc2;
+      cell_scatter<T, D, true><<<grid_for(n, kBlock), kBlock, 0, s>>>(p, n, g, w.start, slots, nullptr, w.rec, w.cell);
+    } else {
+      cell_scatter<T, D, false><<<grid_for(n, kBlock), kBlock, 0, s>>>(p, n, g, nullptr, nullptr, w.order, w.rec, w.cell);
+    }
     TSPH_LAUNCH_CHECK();
     return TSPH_OK;
   });
-  if (rc) return rc;
-  rc = radix_sort_u64_i32(w.keys, w.order, w.keys_tmp, w.order_tmp, n, static_cast<int>(grid->key_bits),
-                          w.radix_scratch, s);
-  if (rc) return rc;
-  run_flags<<<grid_for(n, kBlock), kBlock, 0, s>>>(w.keys, n, w.flags);
-  TSPH_LAUNCH_CHECK();
-  rc = exclusive_scan_i32_to_i64(w.flags, w.run_of, n, w.nruns, w.scan_scratch, s);
-  if (rc) return rc;
-  if (grid->dense)
-    TSPH_CUDA_CHECK(cudaMemsetAsync(w.table, 0xff, grid->total_cells * sizeof(int32_t), s));
-  run_fill<<<grid_for(n, kBlock), kBlock, 0, s>>>(w.keys, w.flags, w.run_of, n, w.run_start, w.run_key,
-                                                  w.table, static_cast<int>(grid->dense), w.nruns);
-  TSPH_LAUNCH_CHECK();
-  if (order_out) {
-    order_to_i64<<<grid_for(n, kBlock), kBlock, 0, s>>>(w.order, n, order_out);
-    TSPH_LAUNCH_CHECK();
-  }
-  return TSPH_OK;
 }
 
 int tsph_pairs_count(const void* pos, const tsph_grid* grid, int64_t row_limit, void* ws,
@@ -476,30 +752,22 @@ int tsph_pairs_count(const void* pos, const tsph_grid* grid, int64_t row_limit, 
   if (row_limit > n) row_limit = n;
   BuildWs w;
   build_layout(*grid, &w, ws);
-  GridDev g = to_dev(*grid);
-  int rc = dispatch(grid->dtype, grid->dim, [&](auto t, auto d) {
-    using T = decltype(t);
-    pair_kernel<T, decltype(d)::value, 0><<<grid_for(n, 128), 128, 0, s>>>(
-        static_cast<const T*>(pos), n, n, g, w.cell, w.order, w.run_start, w.run_key, w.nruns,
-        w.table, host_cutoff_sq<T>(grid->cutoff), w.rowcount, nullptr, nullptr);
-    TSPH_LAUNCH_CHECK();
-    return TSPH_OK;
-  });
+  int rc = count_rows<kForward>(pos, *grid, n, w, w.rowptr, s);
   if (rc) return rc;
-  rc = exclusive_scan_i32_to_i64(w.rowcount, w.rowptr, n, w.total, w.scan_scratch, s);
-  if (rc) return rc;
-  TSPH_CUDA_CHECK(cudaMemcpyAsync(w.rowptr + n, w.total, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
   int64_t host[2] = {0, 0};
-  TSPH_CUDA_CHECK(cudaMemcpyAsync(&host[0], w.rowptr + row_limit, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-  TSPH_CUDA_CHECK(cudaMemcpyAsync(&host[1], w.total, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  TSPH_CUDA_CHECK(cudaMemcpyAsync(&host[1], w.rowptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  if (row_limit < n)
+    TSPH_CUDA_CHECK(cudaMemcpyAsync(&host[0], w.rowptr + row_limit, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   TSPH_CUDA_CHECK(cudaStreamSynchronize(s));
+  if (row_limit == n) host[0] = host[1];
   *pair_count = host[0];
   if (total_count) *total_count = host[1];
   return TSPH_OK;
 }
 
 int64_t tsph_pairs_emit_workspace_bytes(int64_t pair_count, int64_t n) {
-  return static_cast<int64_t>(align_up((pair_count + 1) * sizeof(uint32_t)) + segsort_scratch_bytes(n));
+  (void)n;
+  return static_cast<int64_t>(align_up((pair_count + 1) * sizeof(uint32_t)));
 }
 
 int tsph_pairs_emit(const void* pos, const tsph_grid* grid, int64_t row_limit, void* ws,
@@ -515,23 +783,45 @@ int tsph_pairs_emit(const void* pos, const tsph_grid* grid, int64_t row_limit, v
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   BuildWs w;
   build_layout(*grid, &w, ws);
-  GridDev g = to_dev(*grid);
   uint32_t* cols = static_cast<uint32_t*>(emit_ws);
-  char* sort_scratch = static_cast<char*>(emit_ws) + align_up((pair_count + 1) * sizeof(uint32_t));
-  int rc = dispatch(grid->dtype, grid->dim, [&](auto t, auto d) {
-    using T = decltype(t);
-    pair_kernel<T, decltype(d)::value, 1><<<grid_for(n, 128), 128, 0, s>>>(
-        static_cast<const T*>(pos), n, row_limit, g, w.cell, w.order, w.run_start, w.run_key, w.nruns,
-        w.table, host_cutoff_sq<T>(grid->cutoff), nullptr, w.rowptr, cols);
-    TSPH_LAUNCH_CHECK();
+  if (reinterpret_cast<uintptr_t>(pairs) % 16 == 0)
+    return emit_rows<kForward>(pos, *grid, row_limit, row_limit, w, w.rowptr, cols, pair_count,
+                               AsPairs<true>{pairs}, s);
+  return emit_rows<kForward>(pos, *grid, row_limit, row_limit, w, w.rowptr, cols, pair_count,
+                             AsPairs<false>{pairs}, s);
+}
+
+int tsph_rows_count(const void* pos, const tsph_grid* grid, int64_t row_limit, void* ws, int64_t ws_bytes,
+                    int64_t* rowptr, int64_t* entry_count, tsph_stream stream) {
+  if (!grid || !rowptr || !entry_count) return TSPH_ERR_ARG;
+  if (ws_bytes < grid->workspace_bytes) return TSPH_ERR_WORKSPACE;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const int64_t n = grid->n;
+  *entry_count = 0;
+  if (n < 2) {
+    TSPH_CUDA_CHECK(cudaMemsetAsync(rowptr, 0, (n + 1) * sizeof(int64_t), s));
     return TSPH_OK;
-  });
+  }
+  BuildWs w;
+  build_layout(*grid, &w, ws);
+  int rc = count_rows<kBoth>(pos, *grid, std::min(std::max<int64_t>(row_limit, 0), n), w, rowptr, s);
   if (rc) return rc;
-  rc = segmented_sort_u32(cols, w.rowptr, row_limit, pair_count, sort_scratch, s);
-  if (rc) return rc;
-  expand_pairs<<<grid_for(row_limit * 32, 256), 256, 0, s>>>(w.rowptr, cols, row_limit, pairs);
-  TSPH_LAUNCH_CHECK();
+  TSPH_CUDA_CHECK(cudaMemcpyAsync(entry_count, rowptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  TSPH_CUDA_CHECK(cudaStreamSynchronize(s));
   return TSPH_OK;
+}
+
+int tsph_rows_emit(const void* pos, const tsph_grid* grid, int64_t row_limit, void* ws, int64_t ws_bytes,
+                   const int64_t* rowptr, uint32_t* entries, int64_t entry_count, tsph_stream stream) {
+  if (!grid) return TSPH_ERR_ARG;
+  if (ws_bytes < grid->workspace_bytes) return TSPH_ERR_WORKSPACE;
+  const int64_t n = grid->n;
+  if (entry_count == 0 || n < 2) return TSPH_OK;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  BuildWs w;
+  build_layout(*grid, &w, ws);
+  return emit_rows<kBoth>(pos, *grid, std::min(std::max<int64_t>(row_limit, 0), n), n, w, rowptr, entries,
+                          entry_count, AsEntries{entries}, s);
 }
 
 int64_t tsph_brute_workspace_bytes(int64_t n) {

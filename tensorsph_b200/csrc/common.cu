@@ -243,7 +243,7 @@ size_t segsort_scratch_bytes(int64_t rows) {
 
 int segmented_sort_u32(uint32_t* vals, const int64_t* rowptr, int64_t rows, int64_t entries, void* scratch,
                        cudaStream_t s) {
-  return sort_rows(vals, CsrRows{rowptr}, rows, entries, InPlace{vals}, scratch, s);
+  return sort_rows(CsrRows{vals, rowptr}, rows, entries, AsEntries{vals}, scratch, s);
 }
 
 }  // namespace tsph

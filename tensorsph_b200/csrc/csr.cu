@@ -24,9 +24,9 @@
 //
 // What bounds the first route: the L2 atomics of A (one per pair), the
 // scattered 4-byte stores of B, instruction issue in C.  18.6 M pairs of a
-// periodic column (480 k rows): A 0.13, scan 0.01, B 0.15, C 0.15 ms, against
+// periodic column (480 k rows): A 0.13, scan 0.01, B 0.15, C 0.11 ms, against
 // 0.22 + 0.01 + 0.36 + 0.60 ms by the second route with a rank sort of whole
-// rows; 10.6 M pairs of a 2-D column (1.04 M rows): 0.30 against 0.53 ms.
+// rows; 10.6 M pairs of a 2-D column (1.04 M rows): 0.26 against 0.53 ms.
 #include "common.cuh"
 #include "rowsort.cuh"
 
@@ -101,10 +101,12 @@ __global__ void __launch_bounds__(kBlock) list_fill(const int64_t* __restrict__ 
 
 // The second-element halves of the rows.
 struct SecondHalves {
+  uint32_t* entries;
   const int64_t* rowptr;
   const int2* run;
-  __device__ __forceinline__ int64_t beg(int64_t r) const { return rowptr[r] + (run[r].y - run[r].x); }
-  __device__ __forceinline__ int64_t len(int64_t r) const { return rowptr[r + 1] - beg(r); }
+  __device__ __forceinline__ int64_t dst(int64_t r) const { return rowptr[r] + (run[r].y - run[r].x); }
+  __device__ __forceinline__ uint32_t* src(int64_t r) const { return entries + dst(r); }
+  __device__ __forceinline__ int64_t len(int64_t r) const { return rowptr[r + 1] - dst(r); }
 };
 
 __global__ void csr_degree(const int64_t* __restrict__ pairs, int64_t npairs, int64_t nrows,
@@ -193,7 +195,7 @@ int rows_of_sorted(const int64_t* pairs, int64_t npairs, int64_t nrows, int64_t*
   if (rc) return rc;
   list_fill<kWide><<<g, kBlock, 0, s>>>(pairs, npairs, run, rowptr, w.slot, entries);
   TSPH_LAUNCH_CHECK();
-  return sort_rows(entries, SecondHalves{rowptr, run}, nrows, npairs, InPlace{entries}, w.sort, s);
+  return sort_rows(SecondHalves{entries, rowptr, run}, nrows, npairs, AsEntries{entries}, w.sort, s);
 }
 
 }  // namespace

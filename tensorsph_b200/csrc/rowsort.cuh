@@ -1,30 +1,35 @@
-// Ascending sort of short uint32 rows, one row per warp (or two rows of up to
-// 16 entries per warp), held in registers as a bitonic network: entry i of a
-// row sits in register i / W of lane i % W of its W-lane group, so exchanges
-// at distances below W are shuffles and the others stay inside a lane.
+// Ascending sort of short uint32 rows in registers: W lanes share a row, each
+// holding E entries; a warp takes 32 / W neighbouring rows at once.
 //
-// What bounds it: instruction issue and the latency of the row bounds, not
-// bytes.  A row of 39 entries (the one-sided 3-D list at 2.6 dx) takes a
-// 64-entry network, 21 exchanges of two registers, against 39 x 2 compare
-// steps per lane of a rank sort over shared memory: 480 k rows of 39 entries
-// sort in 0.15 ms against 0.32.
+// A bitonic network with the sorted position i = lane * E + register, so that
+// exchanges at distances below E stay inside a lane (two min/max instructions)
+// and only log2(W) (log2(W) + 1) / 2 of its steps are shuffles: three with the
+// four lanes that rows of up to 64 entries get, six with eight lanes (up to
+// 128), ten with 16.  Sixteen registers of entries are the most (with 32 the
+// kernel takes 168 registers and loses more to idle warps than the shuffles
+// cost).  Entries are loaded strided (any arrangement will do as input) and
+// leave through shared memory, so that a row's stores are contiguous.
 //
-// Rows is a view: beg(r) and len(r).  Out takes (r, position, value).  Rows
-// longer than kWarpRow are appended to `lists` for rows_sort_rest.
+// What bounds it: instruction issue and, for pairs, the 16 bytes written per
+// entry.  With a row per warp (entry = register * 32 + lane) the shuffles
+// bound it, 40 for a 64-entry row against 6 here.  1.0 M rows of 38 entries,
+// sorted and written out as pairs (0.77 GB moved), take 0.23 ms against 0.31,
+// and 0.74 + 0.18 ms for a rank sort over shared memory and a pass that writes
+// the pairs; 1.04 M 2-D rows of 10 entries in place 0.09 against 0.14 and 0.31.
 #pragma once
 
 #include "common.cuh"
 
 namespace tsph {
 
-constexpr int kWarpRow = 256;       // longest row a warp sorts in eight registers a lane
-constexpr int kMidRow = 1024;       // longest row a warp sorts in 32
+constexpr int kGroupRow = 256;      // longest row rows_sort takes
+constexpr int kMidRow = 1024;       // longest row a warp of rows_sort_rest takes
 constexpr int kMediumRow = 8192;    // longest row a block sorts in shared memory
-constexpr int kSortBlock = 256;
+constexpr int kSortBlock = 128;
 constexpr int kRestBlock = 512;
 
 struct LongRows {
-  int64_t* mid;      // rows of kWarpRow + 1 .. kMidRow entries
+  int64_t* mid;      // rows of kGroupRow + 1 .. kMidRow entries
   int64_t* big;      // longer ones
   unsigned long long* counts;  // [0] mid, [1] big
 };
@@ -38,130 +43,179 @@ inline LongRows long_rows(void* scratch, int64_t rows) {
   return l;
 }
 
-// Rows of a CSR table.
+// A view of rows: where row r's entries are, the output position of its first
+// one, how many there are.
 struct CsrRows {
+  uint32_t* vals;
   const int64_t* ptr;
-  __device__ __forceinline__ int64_t beg(int64_t r) const { return ptr[r]; }
+  __device__ __forceinline__ uint32_t* src(int64_t r) const { return vals + ptr[r]; }
+  __device__ __forceinline__ int64_t dst(int64_t r) const { return ptr[r]; }
   __device__ __forceinline__ int64_t len(int64_t r) const { return ptr[r + 1] - ptr[r]; }
 };
 
-// Back into the array the rows came from.
-struct InPlace {
+// Outputs take (row, position, value).
+struct AsEntries {
   uint32_t* vals;
-  static constexpr bool kAll = false;  // rows of one entry are already in place
   __device__ __forceinline__ void operator()(int64_t, int64_t pos, uint32_t v) const { vals[pos] = v; }
 };
 
-// E registers x W lanes, ascending over each group of W lanes.
+// (row, value) pairs; kWide: pairs is 16-byte aligned, one store each.
+template <bool kWide>
+struct AsPairs {
+  int64_t* pairs;
+  __device__ __forceinline__ void operator()(int64_t r, int64_t pos, uint32_t v) const {
+    if (kWide) {
+      *reinterpret_cast<longlong2*>(pairs + 2 * pos) = make_longlong2(r, static_cast<long long>(v));
+    } else {
+      pairs[2 * pos] = r;
+      pairs[2 * pos + 1] = static_cast<int64_t>(v);
+    }
+  }
+};
+
+// Ascending over the W * E entries of a group of W lanes, at i = gl * E + r.
 template <int E, int W>
 __device__ __forceinline__ void bitonic_regs(uint32_t (&v)[E], int gl) {
 #pragma unroll
   for (int k = 2; k <= W * E; k <<= 1) {
 #pragma unroll
     for (int j = k >> 1; j > 0; j >>= 1) {
-      if (j < W) {
-        const bool lower = (gl & j) == 0;
+      if (j < E) {
 #pragma unroll
         for (int r = 0; r < E; ++r) {
-          const bool asc = ((r * W + gl) & k) == 0;
-          const uint32_t o = __shfl_xor_sync(0xffffffffu, v[r], j);
-          v[r] = (lower == asc) ? min(v[r], o) : max(v[r], o);
+          if (r & j) continue;
+          const bool asc = ((gl * E + r) & k) == 0;  // known at compile time for k < E
+          const uint32_t a = v[r], b = v[r | j];
+          v[r] = asc ? min(a, b) : max(a, b);
+          v[r | j] = asc ? max(a, b) : min(a, b);
         }
       } else {
-        const int jr = j / W;
+        const bool keep_low = ((gl & (j / E)) == 0) == (((gl * E) & k) == 0);
 #pragma unroll
         for (int r = 0; r < E; ++r) {
-          if (r & jr) continue;
-          const bool asc = ((r * W + gl) & k) == 0;
-          const uint32_t a = v[r], b = v[r | jr];
-          v[r] = asc ? min(a, b) : max(a, b);
-          v[r | jr] = asc ? max(a, b) : min(a, b);
+          const uint32_t o = __shfl_xor_sync(0xffffffffu, v[r], j / E);
+          v[r] = keep_low ? min(v[r], o) : max(v[r], o);
         }
       }
     }
   }
 }
 
-template <int E, int W, class Out>
-__device__ __forceinline__ void sort_row(const uint32_t* __restrict__ vals, int64_t r, int64_t beg, int len,
-                                         int gl, const Out& out) {
+// 32 / W rows from r0 on, every one of at most W * E entries; all lanes of the
+// warp take part.  buf: 32 * (E + 1) words of the warp's own.
+template <int E, int W, class Rows, class Out>
+__device__ __forceinline__ void sort_group(const Rows& rows, int64_t r0, int64_t n, const Out& out,
+                                           uint32_t* buf) {
+  const int lane = threadIdx.x & 31, gl = lane & (W - 1), g = lane / W;
+  const int64_t r = r0 + g;
+  const int len = r < n ? static_cast<int>(rows.len(r)) : 0;
+  const uint32_t* src = r < n ? rows.src(r) : nullptr;
+  const int64_t dst = r < n ? rows.dst(r) : 0;
   uint32_t v[E];
 #pragma unroll
-  for (int i = 0; i < E; ++i) v[i] = i * W + gl < len ? vals[beg + i * W + gl] : 0xffffffffu;
+  for (int i = 0; i < E; ++i) v[i] = i * W + gl < len ? src[i * W + gl] : 0xffffffffu;
   bitonic_regs<E, W>(v, gl);
+  // sorted position p of group g at ((g * W + p / E) * (E + 1) + p % E): one
+  // spare word per lane keeps the stores off each other's banks
+  __syncwarp();
 #pragma unroll
-  for (int i = 0; i < E; ++i)
-    if (i * W + gl < len) out(r, beg + i * W + gl, v[i]);
+  for (int i = 0; i < E; ++i) buf[lane * (E + 1) + i] = v[i];
+  __syncwarp();
+#pragma unroll 1
+  for (int q = 0; q < 32 / W; ++q) {
+    const int lq = __shfl_sync(0xffffffffu, len, q * W);
+    const int64_t dq = __shfl_sync(0xffffffffu, dst, q * W);
+    for (int p = lane; p < lq; p += 32) out(r0 + q, dq + p, buf[(q * W + p / E) * (E + 1) + p % E]);
+  }
 }
 
-// `vals` is not __restrict__: with InPlace it is also the output, and every
-// row is read into registers before any of it is written.
+// Rows with those beyond kGroupRow left out.
+template <class Rows>
+struct Bounded {
+  const Rows& rows;
+  __device__ __forceinline__ uint32_t* src(int64_t r) const { return rows.src(r); }
+  __device__ __forceinline__ int64_t dst(int64_t r) const { return rows.dst(r); }
+  __device__ __forceinline__ int64_t len(int64_t r) const {
+    const int64_t l = rows.len(r);
+    return l <= kGroupRow ? l : 0;
+  }
+};
+
+// The rows may lie where the output goes: a row is read whole before any of it
+// is written, and rows do not overlap.
 template <class Rows, class Out>
-__global__ void __launch_bounds__(kSortBlock) rows_sort(const uint32_t* vals, Rows rows, int64_t n, Out out,
-                                                        LongRows lists) {
+__global__ void __launch_bounds__(kSortBlock, 8) rows_sort(Rows rows, int64_t n, Out out, LongRows lists) {
+  __shared__ uint32_t buf[kSortBlock / 32][32 * 17];
   const int lane = threadIdx.x & 31;
+  uint32_t* mine = buf[threadIdx.x >> 5];
   const int64_t warps = (static_cast<int64_t>(gridDim.x) * kSortBlock) >> 5;
-  for (int64_t w = (static_cast<int64_t>(blockIdx.x) * kSortBlock + threadIdx.x) >> 5; 2 * w < n; w += warps) {
-    const int64_t r0 = 2 * w;
-    const bool two = r0 + 1 < n;
-    // half a warp per row of the pair: lengths of both rows in every lane
-    const int64_t b0 = rows.beg(r0), l0 = rows.len(r0);
-    const int64_t b1 = two ? rows.beg(r0 + 1) : 0, l1 = two ? rows.len(r0 + 1) : 0;
-    if (l0 <= 16 && l1 <= 16) {
-      const bool second = lane >= 16;
-      const int len = static_cast<int>(second ? l1 : l0);
-      if ((l0 > l1 ? l0 : l1) > (Out::kAll ? 0 : 1))
-        sort_row<1, 16>(vals, second ? r0 + 1 : r0, second ? b1 : b0, len, lane & 15, out);
-      continue;
-    }
-#pragma unroll 1
-    for (int k = 0; k < 2; ++k) {
-      const int64_t r = r0 + k, beg = k ? b1 : b0, len = k ? l1 : l0;
-      const int n32 = static_cast<int>(len);
-      if (len <= (Out::kAll ? 0 : 1)) continue;
-      if (len <= 32)
-        sort_row<1, 32>(vals, r, beg, n32, lane, out);
-      else if (len <= 64)
-        sort_row<2, 32>(vals, r, beg, n32, lane, out);
-      else if (len <= 128)
-        sort_row<4, 32>(vals, r, beg, n32, lane, out);
-      else if (len <= kWarpRow)
-        sort_row<8, 32>(vals, r, beg, n32, lane, out);
-      else if (lane == 0) {
+  for (int64_t w = (static_cast<int64_t>(blockIdx.x) * kSortBlock + threadIdx.x) >> 5; 8 * w < n; w += warps) {
+    const int64_t r0 = 8 * w, r = r0 + (lane & 7);
+    const int64_t len = r < n ? rows.len(r) : 0;
+    int64_t longest = len;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+    if (longest == 0) continue;
+    if (longest <= 8)
+      sort_group<2, 4>(rows, r0, n, out, mine);
+    else if (longest <= 16)
+      sort_group<4, 4>(rows, r0, n, out, mine);
+    else if (longest <= 32)
+      sort_group<8, 4>(rows, r0, n, out, mine);
+    else if (longest <= 64)
+      sort_group<16, 4>(rows, r0, n, out, mine);
+    else {
+      // a row beyond kGroupRow is listed and left empty here
+      if (lane < 8 && len > kGroupRow) {
         if (len <= kMidRow)
           lists.mid[atomicAdd(&lists.counts[0], 1ull)] = r;
         else
           lists.big[atomicAdd(&lists.counts[1], 1ull)] = r;
       }
+      const Bounded<Rows> bounded{rows};
+      if (longest <= 128) {
+#pragma unroll 1
+        for (int h = 0; h < 8; h += 4) sort_group<16, 8>(bounded, r0 + h, n, out, mine);
+      } else {
+#pragma unroll 1
+        for (int h = 0; h < 8; h += 2) sort_group<16, 16>(bounded, r0 + h, n, out, mine);
+      }
     }
   }
 }
 
-// The rows beyond kWarpRow: mid rows by one warp each, longer ones by one
-// block each, in shared memory up to kMediumRow and beyond it directly in
-// global memory.  The global network is the all-ascending form (the first
-// step of each merge pairs t with t ^ (k - 1)), so the minimum always lands
-// on the lower index and the virtual +inf padding beyond `len` never moves.
+// The rows beyond kGroupRow: mid rows by one warp each (entry = register * 32 +
+// lane of the sorted order, as above with 32 lanes), longer ones by one block
+// each, in shared memory up to kMediumRow and beyond it directly where they
+// lie.  The global network is the
+// all-ascending form (the first step of each merge pairs t with t ^ (k - 1)),
+// so the minimum always lands on the lower index and the virtual +inf padding
+// beyond `len` never moves.
 template <class Rows, class Out>
-__global__ void __launch_bounds__(kRestBlock) rows_sort_rest(uint32_t* vals, Rows rows, Out out, LongRows lists) {
+__global__ void __launch_bounds__(kRestBlock, 1) rows_sort_rest(Rows rows, Out out, LongRows lists) {
   __shared__ uint32_t buf[kMediumRow];
-  const int lane = threadIdx.x & 31;
   const int64_t mids = static_cast<int64_t>(lists.counts[0]), bigs = static_cast<int64_t>(lists.counts[1]);
+  const int lane = threadIdx.x & 31;
   const int64_t warps = (static_cast<int64_t>(gridDim.x) * kRestBlock) >> 5;
   for (int64_t q = (static_cast<int64_t>(blockIdx.x) * kRestBlock + threadIdx.x) >> 5; q < mids; q += warps) {
-    const int64_t r = lists.mid[q], beg = rows.beg(r);
+    const int64_t r = lists.mid[q], dst = rows.dst(r);
+    const uint32_t* src = rows.src(r);
     const int len = static_cast<int>(rows.len(r));
-    if (len <= 512)
-      sort_row<16, 32>(vals, r, beg, len, lane, out);
-    else
-      sort_row<32, 32>(vals, r, beg, len, lane, out);
+    uint32_t v[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = i * 32 + lane < len ? src[i * 32 + lane] : 0xffffffffu;
+    bitonic_regs<32, 32>(v, lane);
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (lane * 32 + i < len) out(r, dst + lane * 32 + i, v[i]);
   }
   for (int64_t q = blockIdx.x; q < bigs; q += gridDim.x) {
-    const int64_t r = lists.big[q], beg = rows.beg(r), len = rows.len(r);
+    const int64_t r = lists.big[q], dst = rows.dst(r), len = rows.len(r);
+    uint32_t* a = rows.src(r);
     int64_t p2 = 1;
     while (p2 < len) p2 <<= 1;
     if (len <= kMediumRow) {
-      for (int t = threadIdx.x; t < p2; t += blockDim.x) buf[t] = t < len ? vals[beg + t] : 0xffffffffu;
+      for (int t = threadIdx.x; t < p2; t += blockDim.x) buf[t] = t < len ? a[t] : 0xffffffffu;
       __syncthreads();
       for (int k = 2; k <= p2; k <<= 1) {
         for (int j = k >> 1; j > 0; j >>= 1) {
@@ -176,9 +230,8 @@ __global__ void __launch_bounds__(kRestBlock) rows_sort_rest(uint32_t* vals, Row
           __syncthreads();
         }
       }
-      for (int t = threadIdx.x; t < len; t += blockDim.x) out(r, beg + t, buf[t]);
+      for (int t = threadIdx.x; t < len; t += blockDim.x) out(r, dst + t, buf[t]);
     } else {
-      uint32_t* a = vals + beg;
       for (int64_t k = 2; k <= p2; k <<= 1) {
         for (int64_t j = k >> 1; j > 0; j >>= 1) {
           const int64_t mask = (j == (k >> 1)) ? (k - 1) : j;
@@ -192,27 +245,25 @@ __global__ void __launch_bounds__(kRestBlock) rows_sort_rest(uint32_t* vals, Row
           __syncthreads();
         }
       }
-      if (Out::kAll)
-        for (int64_t t = threadIdx.x; t < len; t += blockDim.x) out(r, beg + t, a[t]);
+      for (int64_t t = threadIdx.x; t < len; t += blockDim.x) out(r, dst + t, a[t]);
     }
     __syncthreads();
   }
 }
 
-// Sort the n rows of `rows` in vals and hand them to out.  `entries` bounds
-// the entries of all rows together: below kWarpRow + 1 no row can be long, and
-// the second kernel is not launched.  Scratch: segsort_scratch_bytes(n).
+// Sort the n rows of `rows` and hand them to out.  `longest` bounds
+// the length of a row (or the entries of all rows together): up to kGroupRow the
+// second kernel is not launched.  Scratch: segsort_scratch_bytes(n).
 template <class Rows, class Out>
-int sort_rows(uint32_t* vals, Rows rows, int64_t n, int64_t entries, Out out, void* scratch, cudaStream_t s) {
+int sort_rows(Rows rows, int64_t n, int64_t longest, Out out, void* scratch, cudaStream_t s) {
   if (n <= 0) return TSPH_OK;
   const LongRows lists = long_rows(scratch, n);
-  const bool rest = entries > kWarpRow;
+  const bool rest = longest > kGroupRow;
   if (rest) TSPH_CUDA_CHECK(cudaMemsetAsync(lists.counts, 0, 2 * sizeof(unsigned long long), s));
-  rows_sort<Rows, Out><<<grid_for((n + 1) / 2, kSortBlock / 32, 148 * 16), kSortBlock, 0, s>>>(vals, rows, n, out,
-                                                                                              lists);
+  rows_sort<Rows, Out><<<grid_for((n + 7) / 8, kSortBlock / 32, 148 * 64), kSortBlock, 0, s>>>(rows, n, out, lists);
   TSPH_LAUNCH_CHECK();
   if (rest) {
-    rows_sort_rest<Rows, Out><<<148 * 2, kRestBlock, 0, s>>>(vals, rows, out, lists);
+    rows_sort_rest<Rows, Out><<<148, kRestBlock, 0, s>>>(rows, out, lists);
     TSPH_LAUNCH_CHECK();
   }
   return TSPH_OK;

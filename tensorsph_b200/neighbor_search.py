@@ -21,7 +21,7 @@ import torch
 from . import _lib
 
 __all__ = ["brute_force_pairs", "cell_linked_pairs", "cell_order", "PairListCache",
-           "grid_pairs"]
+           "grid_pairs", "grid_rows"]
 
 
 def _validate(positions, cutoff):
@@ -89,6 +89,30 @@ def grid_pairs(pos: torch.Tensor, cutoff: float, box=None, row_limit: int | None
                                      ws.numel(), ews.data_ptr(), ews.numel(), pairs.data_ptr(),
                                      kept.value, s), "tsph_pairs_emit")
     return pairs, int(total.value), order
+
+
+def grid_rows(pos: torch.Tensor, cutoff: float, row_limit: int | None = None):
+    """Symmetric gather rows ``(rowptr, entries, entry_count)`` of a CUDA-resident cloud (two
+    particles at least): the rows that ``symmetric_rows`` makes of the pairs whose first
+    index is below ``row_limit``, built from the cells without the pair list."""
+    L = _lib.lib()
+    dev = pos.device
+    n = pos.shape[0]
+    grid, ws = _plan(pos, cutoff)
+    s = _lib.stream(dev)
+    _lib.check(L.tsph_grid_build(pos.data_ptr(), ctypes.byref(grid), ws.data_ptr(), ws.numel(),
+                                 None, s), "tsph_grid_build")
+    limit = n if row_limit is None else max(0, min(int(row_limit), n))
+    rowptr = torch.empty(n + 1, dtype=torch.long, device=dev)
+    count = ctypes.c_int64(0)
+    _lib.check(L.tsph_rows_count(pos.data_ptr(), ctypes.byref(grid), limit, ws.data_ptr(),
+                                 ws.numel(), rowptr.data_ptr(), ctypes.byref(count), s),
+               "tsph_rows_count")
+    entries = torch.empty(max(count.value, 1), dtype=torch.int32, device=dev)
+    _lib.check(L.tsph_rows_emit(pos.data_ptr(), ctypes.byref(grid), limit, ws.data_ptr(),
+                                ws.numel(), rowptr.data_ptr(), entries.data_ptr(), count.value, s),
+               "tsph_rows_emit")
+    return rowptr, entries, count.value
 
 
 def cell_linked_pairs(positions: torch.Tensor, cutoff: float) -> torch.Tensor:

@@ -1,0 +1,119 @@
+"""The cell search against the oracle where its routes change: the number of
+rows that switches lanes per row, three and four cells on a periodic axis,
+particles outside the box, distances at the cutoff, a far-off origin, and the
+list ends of a pruned search."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import neighbors as on
+
+pytestmark = pytest.mark.gpu
+
+
+def lattice(counts, dx, dtype, jitter, seed=0):
+    g = np.stack(np.meshgrid(*[np.arange(c) for c in counts], indexing="ij"), -1).reshape(-1, len(counts))
+    rng = np.random.default_rng(seed)
+    return ((g + 0.5 + jitter * rng.uniform(-1, 1, g.shape)) * dx).astype(dtype)
+
+
+def search(pos, cutoff, dev, box=None):
+    from tensorsph_b200.neighbor_search import cell_linked_pairs
+    from tensorsph_b200.threed import periodic_pairs
+    t = torch.from_numpy(pos).to(dev)
+    return (cell_linked_pairs(t, cutoff) if box is None else periodic_pairs(t, box, cutoff)).cpu().numpy()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("cutoff", [1.0, 2.0, 2.6])
+def test_lattice_shells_at_the_cutoff(gpu, dtype, cutoff):
+    """Unjittered lattices: whole shells lie exactly at the cutoff, where the last bit decides."""
+    for counts, scale in (((40, 31), 0.1), ((13, 11, 12), 0.013), ((900,), 0.37)):
+        pos = lattice(counts, scale, dtype, 0.0)
+        pos = pos[np.random.default_rng(1).permutation(pos.shape[0])]
+        assert np.array_equal(search(pos, cutoff * scale, gpu), on.cell_linked_pairs(pos, cutoff * scale))
+
+
+@pytest.mark.parametrize("n", [24575, 24576, 24577])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_lanes_per_row_switch(gpu, n, dtype):
+    pos = lattice((160, 160), 0.01, dtype, 0.2)[:n]
+    pos = pos[np.random.default_rng(2).permutation(n)]
+    assert np.array_equal(search(pos, 0.027, gpu), on.cell_linked_pairs(pos, 0.027))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("cells", [1.5, 3.0, 3.9, 4.0, 4.5, 7.0])
+def test_periodic_axes_of_few_cells(gpu, dtype, cells):
+    rng = np.random.default_rng(5)
+    for dim in (1, 2, 3):
+        pos = rng.random((700, dim)).astype(dtype)
+        pos[:50] += rng.integers(-3, 4, (50, dim))            # whole boxes away
+        pos[50:60] = 0.0
+        pos[60:70] = 1.0
+        cutoff = 1.0 / cells
+        assert np.array_equal(search(pos, cutoff, gpu, [1.0] * dim),
+                              on.periodic_pairs(pos, [1.0] * dim, cutoff))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("offset", [0.0, -3.7, 900.0, 2.0e5])
+def test_far_origin(gpu, dtype, offset):
+    """FP32 records measured from the grid's corner; coordinates far from zero."""
+    pos = (lattice((25, 24, 5), 0.1, np.float64, 0.2) + offset).astype(dtype)
+    assert np.array_equal(search(pos, 0.27, gpu), on.cell_linked_pairs(pos, 0.27))
+
+
+def test_long_thin_cloud(gpu):
+    """A grid many thousand cutoffs long: the FP32 records no longer decide, the exact distances do."""
+    rng = np.random.default_rng(8)
+    pos = np.concatenate((rng.random((600, 2)) * [0.5, 0.2], rng.random((600, 2)) * [0.5, 0.2] + [8.0e5, 0.0]))
+    assert np.array_equal(search(pos, 0.03, gpu), on.cell_linked_pairs(pos, 0.03))
+
+
+def test_pruned_list_and_order(gpu):
+    from tensorsph_b200.neighbor_search import cell_order, grid_pairs
+    pos = lattice((60, 50), 0.01, np.float64, 0.2)
+    t = torch.from_numpy(pos).to(gpu)
+    full = on.cell_linked_pairs(pos, 0.027)
+    for limit in (0, 1, 1234, 2999, 3000):
+        pairs, total, order = grid_pairs(t, 0.027, row_limit=limit, with_order=True)
+        assert total == full.shape[0]
+        assert np.array_equal(pairs.cpu().numpy(), full[full[:, 0] < limit])
+        assert torch.equal(order, cell_order(t, 0.027))
+
+
+def rows_and_pairs(pos, cutoff, limit, dev):
+    from tensorsph_b200.droplet_impact import symmetric_rows
+    from tensorsph_b200.neighbor_search import grid_pairs, grid_rows
+    t = torch.from_numpy(pos).to(dev)
+    pairs, _, _ = grid_pairs(t, cutoff, row_limit=limit)
+    return grid_rows(t, cutoff, row_limit=limit), symmetric_rows(pairs, pos.shape[0]), pairs
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("counts,cutoff", [((41, 30), 0.026), ((300, 301), 0.0293), ((17, 16, 15), 0.026),
+                                           ((45, 44, 43), 0.0293), ((12, 13, 11), 0.055), ((400,), 0.03)])
+def test_rows_without_the_list(gpu, dtype, counts, cutoff):
+    """Gather rows straight from the cells equal those made of the pair list; the
+    0.055 rows (about 700 neighbours) outgrow their slots."""
+    pos = lattice(counts, 0.01, dtype, 0.2)
+    n = pos.shape[0]
+    for limit in (n, n // 2, 1, 0):
+        (ptr, entries, count), (ptr2, entries2), pairs = rows_and_pairs(pos, cutoff, limit, gpu)
+        assert count == 2 * pairs.shape[0]
+        assert torch.equal(ptr, ptr2)
+        assert torch.equal(entries[:count], entries2[:count])
+
+
+@pytest.mark.parametrize("count", [15, 16, 17, 47, 48, 49, 50, 127, 128, 129, 130, 300])
+@pytest.mark.parametrize("dim", [1, 2, 3])
+def test_rows_at_their_slots(gpu, count, dim):
+    """A cluster of ``count`` neighbours among spread-out particles, around the number of
+    slots a row has in each dimension."""
+    rng = np.random.default_rng(count)
+    pos = np.concatenate((0.01 * rng.random((count, dim)), 1.0 + np.arange(2000)[:, None] * 0.1 + np.zeros(dim)))
+    pos = pos[rng.permutation(pos.shape[0])]
+    (ptr, entries, total), (ptr2, entries2), pairs = rows_and_pairs(pos, 0.02, pos.shape[0], gpu)
+    assert np.array_equal(pairs.cpu().numpy(), on.cell_linked_pairs(pos, 0.02))
+    assert torch.equal(ptr, ptr2) and torch.equal(entries[:total], entries2[:total])
