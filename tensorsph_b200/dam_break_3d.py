@@ -18,7 +18,7 @@ import torch
 
 from . import _lib
 from .droplet_impact import Config, cell_centres, hydrostatic_density, symmetric_rows
-from .neighbor_search import grid_pairs
+from .neighbor_search import grid_pairs, grid_rows
 from .integrate import clamp_box
 
 __all__ = ["DamBreak3DConfig", "make_column_3d", "wall_lattice_3d", "rhs_3d",
@@ -164,10 +164,12 @@ def rhs_3d(pos, vel, mass, cfg: DamBreak3DConfig, pairs=None, wall=None, dt=None
     Wp = _lib.to_dev(wall.detach(), dev, dtype) if nw else None
     if pairs is None:
         all_pos = torch.cat((P, Wp), dim=0) if nw else P
-        pairs_dev, _, _ = grid_pairs(all_pos, 2.0 * h, row_limit=n)
+        if n + nw < 2:
+            rowptr, entries = symmetric_rows(grid_pairs(all_pos, 2.0 * h, row_limit=n)[0], n + nw)
+        else:
+            rowptr, entries, _ = grid_rows(all_pos, 2.0 * h, row_limit=n)
     else:
-        pairs_dev = _lib.to_dev(pairs, dev)
-    rowptr, entries = symmetric_rows(pairs_dev, n + nw)
+        rowptr, entries = symmetric_rows(_lib.to_dev(pairs, dev), n + nw)
     prm = _lib.WcsphParams()
     prm.dim, prm.dtype, prm.n_fluid, prm.n_wall = 3, code, n, nw
     prm.flags = _lib.RHS_WALL_SELF | (_lib.RHS_SPLIT if return_wall_force else 0)

@@ -19,7 +19,7 @@ import torch
 
 from . import _lib
 from .droplet_impact import symmetric_rows
-from .neighbor_search import grid_pairs
+from .neighbor_search import grid_rows
 
 __all__ = ["DeltaPlusStep", "delta_plus_step", "delta_plus_step3"]
 
@@ -135,9 +135,10 @@ def _delta_plus(dim, pos, velocity, density, mass, *, dx, sound_speed, reference
     W, WV, WN = (_lib.to_dev(t.detach(), dev, dtype).contiguous() for t in (wall, wall_velocity, wall_normal))
     if pairs is None:
         cloud = torch.cat((P, W)) if nw else P
-        pairs_dev, _, _ = grid_pairs(cloud, 2 * h) if n + nw >= 2 else (
-            torch.zeros((0, 2), dtype=torch.long, device=dev), 0, None)
-        rowptr, entries = symmetric_rows(pairs_dev, n + nw)
+        if n + nw >= 2:
+            rowptr, entries, _ = grid_rows(cloud, 2 * h)
+        else:
+            rowptr, entries = symmetric_rows(torch.zeros((0, 2), dtype=torch.long, device=dev), n + nw)
     else:
         if pairs.ndim != 2 or pairs.shape[1] != 2 or pairs.dtype != torch.long:
             raise ValueError("expected a (P, 2) long pair list")

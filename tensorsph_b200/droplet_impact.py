@@ -21,7 +21,7 @@ import math
 import torch
 
 from . import _lib
-from .neighbor_search import PairListCache, cell_linked_pairs, grid_pairs
+from .neighbor_search import PairListCache, cell_linked_pairs, grid_pairs, grid_rows
 
 __all__ = [
     "Config", "SimulationUnstableError", "VISCOUS_LAPLACIAN_FACTOR",
@@ -484,16 +484,22 @@ def rhs(pos, vel, mass, cfg: Config, pairs=None, wall=None, dt=None, wall_vel=No
     M = _lib.to_dev(mass.detach(), dev, dtype)
     Wp = _lib.to_dev(wall.detach(), dev) if nw else None
 
+    rowptr = entries = pairs_dev = None
     if pairs is None:
         all_pos = torch.cat((P, Wp), dim=0) if nw else P
-        pairs_dev, _, _ = grid_pairs(all_pos, 2.0 * h, row_limit=n)
+        if cfg.surface_tension_coefficient > 0.0 or n + nw < 2:
+            pairs_dev, _, _ = grid_pairs(all_pos, 2.0 * h, row_limit=n)   # the CSF reads the list
+            empty = pairs_dev.shape[0] == 0
+        else:
+            rowptr, entries, count = grid_rows(all_pos, 2.0 * h, row_limit=n)
+            empty = count == 0
     else:
         if pairs.ndim != 2 or pairs.shape[1] != 2 or pairs.dtype != torch.long:
             raise ValueError("pairs must be a long tensor with shape (pair_count, 2)")
         if pairs.device != pos.device:
             raise ValueError("pairs and pos must be on the same device")
         pairs_dev = _lib.to_dev(pairs, dev)
-    empty = pairs_dev.shape[0] == 0
+        empty = pairs_dev.shape[0] == 0
     if density_offset is not None and not empty:
         if density_offset.shape != (n,) or density_offset.device != pos.device:
             raise ValueError("density_offset must match the fluid particles")
@@ -526,7 +532,8 @@ def rhs(pos, vel, mass, cfg: Config, pairs=None, wall=None, dt=None, wall_vel=No
             regularizer = CompressionRegularization(rule=cfg.compression_regularization_rule,
                                                     normalization=cfg.compression_normalization)
 
-    rowptr, entries = symmetric_rows(pairs_dev, n + nw)
+    if rowptr is None:
+        rowptr, entries = symmetric_rows(pairs_dev, n + nw)
     prm = _lib.WcsphParams()
     prm.dim, prm.dtype, prm.n_fluid, prm.n_wall = 2, code, n, nw
     flags = 0

@@ -18,7 +18,7 @@ import torch
 
 from . import _lib
 from .droplet_impact import symmetric_rows
-from .neighbor_search import grid_pairs
+from .neighbor_search import grid_rows
 
 __all__ = ["ShiftingState", "shift_positions", "concentration", "estimate_reference_concentration"]
 
@@ -47,12 +47,12 @@ def _run(pos, volume, h, magnitude, cap, free_surface, pairs, c_reference):
     dtype = pos.dtype
     P = _lib.to_dev(pos.detach(), dev)
     Vol = _lib.to_dev(volume.detach(), dev, dtype)
-    if pairs is None:
-        pairs_dev, _, _ = grid_pairs(P, 2.0 * h) if n >= 2 else (
-            torch.zeros((0, 2), dtype=torch.long, device=dev), 0, None)
+    if pairs is None and n >= 2:
+        rowptr, entries, _ = grid_rows(P, 2.0 * h)
     else:
-        pairs_dev = _lib.to_dev(pairs, dev)
-    rowptr, entries = symmetric_rows(pairs_dev, n)
+        pairs_dev = (torch.zeros((0, 2), dtype=torch.long, device=dev) if pairs is None
+                     else _lib.to_dev(pairs, dev))
+        rowptr, entries = symmetric_rows(pairs_dev, n)
     prm = _lib.ShiftParams()
     prm.dim, prm.dtype, prm.n = dim, _lib.dtype_code(dtype), n
     prm.h, prm.sigma = float(h), 10.0 / (7.0 * math.pi * h * h)
