@@ -3,8 +3,8 @@
 // Reference arithmetic: droplet_impact.py:810-1228 and dam_break_3d.py:290-422.
 // The reference walks an unordered pair list and scatters each pair into both
 // ends with index_add.  Here every particle owns one row of the symmetric
-// gather list (csr.cu) and accumulates its own sums in registers, FP32 sums
-// with Neumaier compensation, FP64 sums plain:
+// gather list (csr.cu) and accumulates its own sums in registers, with one to
+// eight lanes to a row, FP32 sums with Neumaier compensation, FP64 sums plain:
 //
 //   K1 density    rho_a = m_a W(0) + sum_b m_b W_ab  (+ offset, Shepard)   fluid rows
 //   K2 gradient   <grad rho>_a = M_a^-1 G_a  (Antuono psi form only)       fluid rows
@@ -24,18 +24,12 @@
 
 #include "common.cuh"
 #include "fpmath.cuh"
+#include "gather.cuh"
 #include "sphkernels.cuh"
 #include "symeig.cuh"
 
 namespace tsph {
 namespace {
-
-constexpr uint32_t kIndexMask = 0x7fffffffu;
-
-template <class T>
-struct alignas(4 * sizeof(T)) Q4 {
-  T x, y, z, w;
-};
 
 template <class T>
 struct WP {
@@ -72,67 +66,78 @@ __device__ __forceinline__ T norm2(const T d[3]) {
 // ------------------------------------------------------------------ pack ---
 
 template <class T, int D>
-__global__ void pack_kernel(const T* __restrict__ pos, const T* __restrict__ vel, const T* __restrict__ mass,
-                            const T* __restrict__ wall, const T* __restrict__ wall_vel,
-                            const T* __restrict__ nu, int64_t n, int64_t nw, T wall_mass,
-                            Q4<T>* __restrict__ pm, Q4<T>* __restrict__ vv) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < n + nw; a += gridDim.x * blockDim.x) {
-    Q4<T> P, V;
+__global__ void pack_kernel(const T* __restrict__ pos, const T* __restrict__ mass, const T* __restrict__ wall,
+                            int64_t n, int64_t nw, T wall_mass, Q4<T>* __restrict__ pm) {
+  for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n + nw;
+       a += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const T* x = a < n ? pos + a * D : wall + (a - n) * D;
+    pm[a] = Q4<T>{x[0], x[1], D == 3 ? x[2] : T(0), a < n ? mass[a] : wall_mass};
+  }
+}
+
+// The final state of every particle: rho and p of the fluid out to the caller,
+// (rho, p) replaced in place by what the force and reaction rows read, (m / rho,
+// p / rho^2), so that their neighbour terms hold no division by a density; and
+// the velocities packed (with nu).
+template <class T, int D>
+__global__ void state_kernel(const T* __restrict__ vel, const T* __restrict__ wall_vel, const T* __restrict__ nu,
+                             const Q4<T>* __restrict__ pm, int64_t n, int64_t nw, Q2<T>* __restrict__ rp,
+                             Q4<T>* __restrict__ vv, T* __restrict__ rho, T* __restrict__ pressure) {
+  for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n + nw;
+       a += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const Q2<T> s = rp[a];
     if (a < n) {
-      P.x = pos[a * D]; P.y = pos[a * D + 1]; P.z = D == 3 ? pos[a * D + 2] : T(0); P.w = mass[a];
-      V.x = vel[a * D]; V.y = vel[a * D + 1]; V.z = D == 3 ? vel[a * D + 2] : T(0);
-      V.w = nu ? nu[a] : T(0);
-    } else {
-      const int64_t w = a - n;
-      P.x = wall[w * D]; P.y = wall[w * D + 1]; P.z = D == 3 ? wall[w * D + 2] : T(0); P.w = wall_mass;
-      if (wall_vel) {
-        V.x = wall_vel[w * D]; V.y = wall_vel[w * D + 1]; V.z = D == 3 ? wall_vel[w * D + 2] : T(0);
-      } else {
-        V.x = V.y = V.z = T(0);
-      }
-      V.w = T(0);
+      rho[a] = s.x;
+      pressure[a] = s.y;
     }
-    pm[a] = P;
-    vv[a] = V;
+    rp[a] = Q2<T>{pm[a].w / s.x, s.y / (s.x * s.x)};
+    const T* v = a < n ? vel + a * D : (wall_vel ? wall_vel + (a - n) * D : nullptr);
+    vv[a] = Q4<T>{v ? v[0] : T(0), v ? v[1] : T(0), D == 3 && v ? v[2] : T(0), a < n && nu ? nu[a] : T(0)};
   }
 }
 
 // ------------------------------------------------------------ K1 density ---
 
-template <class T, int D>
-__global__ void density_kernel(WP<T> p, const Q4<T>* __restrict__ pm, const int64_t* __restrict__ rowptr,
-                               const uint32_t* __restrict__ ent, const T* __restrict__ offset,
-                               T* __restrict__ rho_s, T* __restrict__ rho_all, T* __restrict__ p_all) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < p.n; a += gridDim.x * blockDim.x) {
-    const Q4<T> pa = pm[a];
-    CSum<T> s, kt;
-    s.add(pa.w * p.w0);
-    const int64_t beg = rowptr[a], end = rowptr[a + 1];
-    for (int64_t e = beg; e < end; ++e) {
-      const Q4<T> pb = pm[ent[e] & kIndexMask];
-      T d[3];
-      separation<T, D>(pa, pb, p, d);
-      T W = p.k.w(sqrt(norm2<T, D>(d)));
-      s.add(pb.w * W);
-      kt.add(W);
-    }
-    T rho = s.value();
+// rv: (rho before diffusion, m / rho) for the diffusion rows; rp: (rho, p) when
+// there is no diffusion.
+template <class T, int D, int L>
+__global__ void __launch_bounds__(kGatherBlock) density_kernel(WP<T> p, const Q4<T>* __restrict__ pm,
+                                                               const int64_t* __restrict__ rowptr,
+                                                               const uint32_t* __restrict__ ent,
+                                                               const T* __restrict__ offset, Q2<T>* __restrict__ rv,
+                                                               Q2<T>* __restrict__ rp) {
+  const RowLanes<L> me;
+  const int64_t a = me.row;
+  if (a >= p.n) return;
+  const Q4<T> pa = pm[a];
+  CSum<T> s, kt;
+  if (me.lane == 0) s.add(pa.w);  // W(0) = sigma
+  const bool renorm = p.flags & TSPH_RHS_RENORMALIZE;
+  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+    const Q4<T> pb = pm[e & kIndexMask];
+    T d[3];
+    separation<T, D>(pa, pb, p, d);
+    const T f = p.k.shape2(norm2<T, D>(d));
+    s.add(pb.w * f);
+    if (renorm) kt.add(f);
+  });
+  T rho = p.k.times_sigma(me.sum(s));
+  rho = rho > p.rho_floor ? rho : p.rho_floor;
+  if (p.has_offset) {
+    rho = rho + offset[a];
     rho = rho > p.rho_floor ? rho : p.rho_floor;
-    if (p.has_offset) {
-      rho = rho + offset[a];
-      rho = rho > p.rho_floor ? rho : p.rho_floor;
-    }
-    if (p.flags & TSPH_RHS_RENORMALIZE) {
-      T total = kt.value() + p.w0;
-      total = total > T(1e-12) ? total : T(1e-12);
-      rho = rho * (p.lattice_sum / total);
-      rho = rho > p.rho_floor ? rho : p.rho_floor;
-    }
-    rho_s[a] = rho;
-    if (!p.diffusion) {
-      rho_all[a] = rho;
-      p_all[a] = tait(rho, p);
-    }
+  }
+  if (renorm) {
+    T total = p.k.times_sigma(me.sum(kt)) + p.w0;
+    total = total > T(1e-12) ? total : T(1e-12);
+    rho = rho * (p.lattice_sum / total);
+    rho = rho > p.rho_floor ? rho : p.rho_floor;
+  }
+  if (me.lane == 0) {
+    if (p.diffusion)
+      rv[a] = Q2<T>{rho, pa.w / rho};
+    else
+      rp[a] = Q2<T>{rho, tait(rho, p)};
   }
 }
 
@@ -141,30 +146,30 @@ __global__ void density_kernel(WP<T> p, const Q4<T>* __restrict__ pm, const int6
 // summation density is replaced by rule(S) rho0; S goes to csum for the
 // average that the next call uses.
 
-template <class T, int D>
-__global__ void compression_kernel(WP<T> p, const Q4<T>* __restrict__ pm, const int64_t* __restrict__ rowptr,
-                                   const uint32_t* __restrict__ ent, T kref, int free_surface,
-                                   T* __restrict__ csum, T* __restrict__ rho_s, T* __restrict__ rho_all,
-                                   T* __restrict__ p_all) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < p.n; a += gridDim.x * blockDim.x) {
-    const Q4<T> pa = pm[a];
-    CSum<T> s;
-    const int64_t beg = rowptr[a], end = rowptr[a + 1];
-    for (int64_t e = beg; e < end; ++e) {
-      const Q4<T> pb = pm[ent[e] & kIndexMask];
-      T d[3];
-      separation<T, D>(pa, pb, p, d);
-      s.add(p.k.w(sqrt(norm2<T, D>(d))) * (pb.w / p.rho0));
-    }
-    const T S = p.w0 * (pa.w / p.rho0) + kref * s.value();
-    csum[a] = S;
-    const T K = free_surface ? (S > T(1) ? S : T(1)) : S;
-    T rho = K * p.rho0;
-    rho = rho > p.rho_floor ? rho : p.rho_floor;
-    rho_s[a] = rho;
-    rho_all[a] = rho;
-    p_all[a] = tait(rho, p);
-  }
+template <class T, int D, int L>
+__global__ void __launch_bounds__(kGatherBlock) compression_kernel(WP<T> p, const Q4<T>* __restrict__ pm,
+                                                                   const int64_t* __restrict__ rowptr,
+                                                                   const uint32_t* __restrict__ ent, T kref,
+                                                                   int free_surface, T* __restrict__ csum,
+                                                                   Q2<T>* __restrict__ rp) {
+  const RowLanes<L> me;
+  const int64_t a = me.row;
+  if (a >= p.n) return;
+  const Q4<T> pa = pm[a];
+  CSum<T> s;
+  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+    const Q4<T> pb = pm[e & kIndexMask];
+    T d[3];
+    separation<T, D>(pa, pb, p, d);
+    s.add(p.k.w2(norm2<T, D>(d)) * (pb.w / p.rho0));
+  });
+  const T S = p.w0 * (pa.w / p.rho0) + kref * me.sum(s);
+  if (me.lane) return;
+  csum[a] = S;
+  const T K = free_surface ? (S > T(1) ? S : T(1)) : S;
+  T rho = K * p.rho0;
+  rho = rho > p.rho_floor ? rho : p.rho_floor;
+  rp[a] = Q2<T>{rho, tait(rho, p)};
 }
 
 // AverageCompression: out[0] = count / sum over S > 1 (1 for an empty set),
@@ -219,14 +224,25 @@ __global__ void compression_identity(double* __restrict__ out) {
 // formulation's pair set includes i == j).
 
 template <class T>
-__global__ void closure_init(WP<T> p, const T* __restrict__ rho_all, T threshold, uint8_t* __restrict__ known) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < p.n; a += gridDim.x * blockDim.x)
-    known[a] = rho_all[a] < threshold ? 0 : 1;
+__global__ void closure_init(WP<T> p, const Q2<T>* __restrict__ rp, T threshold, uint8_t* __restrict__ known,
+                             T* __restrict__ pres) {
+  for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < p.n;
+       a += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    known[a] = rp[a].x < threshold ? 0 : 1;
+    pres[a] = rp[a].y;
+  }
+}
+
+template <class T>
+__global__ void closure_finish(int64_t n, const T* __restrict__ pres, Q2<T>* __restrict__ rp) {
+  for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n;
+       a += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    rp[a].y = pres[a];
 }
 
 template <class T, int D>
 __global__ void closure_pass(WP<T> p, const Q4<T>* __restrict__ pm, const int64_t* __restrict__ rowptr,
-                             const uint32_t* __restrict__ ent, const T* __restrict__ rho_all, int donors,
+                             const uint32_t* __restrict__ ent, const Q2<T>* __restrict__ rp, int donors,
                              const T* __restrict__ p_in, const uint8_t* __restrict__ known_in,
                              T* __restrict__ p_out, uint8_t* __restrict__ known_out) {
   for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < p.n; a += gridDim.x * blockDim.x) {
@@ -249,7 +265,7 @@ __global__ void closure_pass(WP<T> p, const Q4<T>* __restrict__ pm, const int64_
       T d[3];
       separation<T, D>(pa, pb, p, d);
       const T W = p.k.w(sqrt(norm2<T, D>(d)));
-      num.add(W * (p_in[b] - p.grav * d[1] * rho_all[b]));
+      num.add(W * (p_in[b] - p.grav * d[1] * rp[b].x));
       den.add(W);
     }
     const T dn = den.value();
@@ -266,159 +282,169 @@ __global__ void closure_pass(WP<T> p, const Q4<T>* __restrict__ pm, const int64_
 
 // ----------------------------------------------------------- K2 gradient ---
 
-template <class T, int D>
-__global__ void gradient_kernel(WP<T> p, const Q4<T>* __restrict__ pm, const int64_t* __restrict__ rowptr,
-                                const uint32_t* __restrict__ ent, const T* __restrict__ rho_s,
-                                T* __restrict__ grad_rho) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < p.n; a += gridDim.x * blockDim.x) {
-    const Q4<T> pa = pm[a];
-    const T ra = rho_s[a];
-    CSum<T> G[3], M[6];  // M lower triangle: 00, 10, 11, 20, 21, 22
-    const int64_t beg = rowptr[a], end = rowptr[a + 1];
-    for (int64_t e = beg; e < end; ++e) {
-      const uint32_t b = ent[e] & kIndexMask;
-      if (b >= p.n) continue;
-      const Q4<T> pb = pm[b];
-      T d[3];
-      separation<T, D>(pa, pb, p, d);
-      T W, gs;
-      p.k.wg(sqrt(norm2<T, D>(d)), W, gs);
-      const T vb = pb.w / rho_s[b];
-      const T diff = rho_s[b] - ra;
-      T g[3] = {d[0] * gs, d[1] * gs, d[2] * gs};
+template <class T, int D, int L>
+__global__ void __launch_bounds__(kGatherBlock) gradient_kernel(WP<T> p, const Q4<T>* __restrict__ pm,
+                                                                const int64_t* __restrict__ rowptr,
+                                                                const uint32_t* __restrict__ ent,
+                                                                const Q2<T>* __restrict__ rv, T* __restrict__ grad_rho) {
+  const RowLanes<L> me;
+  const int64_t a = me.row;
+  if (a >= p.n) return;
+  const Q4<T> pa = pm[a];
+  const T ra = rv[a].x;
+  CSum<T> G[3], M[6];  // M lower triangle: 00, 10, 11, 20, 21, 22
+  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+    const uint32_t b = e & kIndexMask;
+    if (b >= p.n) return;
+    const Q4<T> pb = pm[b];
+    const Q2<T> sb = rv[b];
+    T d[3];
+    separation<T, D>(pa, pb, p, d);
+    T W, gs;
+    p.k.wg2(norm2<T, D>(d), W, gs);
+    const T vb = sb.y;
+    const T diff = sb.x - ra;
+    T g[3] = {d[0] * gs, d[1] * gs, d[2] * gs};
 #pragma unroll
-      for (int r = 0; r < D; ++r) G[r].add(vb * diff * g[r]);
-      M[0].add(vb * -(d[0] * g[0]));
-      M[1].add(vb * -(d[1] * g[0]));
-      M[2].add(vb * -(d[1] * g[1]));
-      if (D == 3) {
-        M[3].add(vb * -(d[2] * g[0]));
-        M[4].add(vb * -(d[2] * g[1]));
-        M[5].add(vb * -(d[2] * g[2]));
-      }
-    }
-    double m[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, rhs[3] = {0, 0, 0}, out[3];
-    m[0][0] = M[0].value();
-    m[1][0] = m[0][1] = M[1].value();
-    m[1][1] = M[2].value();
+    for (int r = 0; r < D; ++r) G[r].add(vb * diff * g[r]);
+    M[0].add(vb * -(d[0] * g[0]));
+    M[1].add(vb * -(d[1] * g[0]));
+    M[2].add(vb * -(d[1] * g[1]));
     if (D == 3) {
-      m[2][0] = m[0][2] = M[3].value();
-      m[2][1] = m[1][2] = M[4].value();
-      m[2][2] = M[5].value();
+      M[3].add(vb * -(d[2] * g[0]));
+      M[4].add(vb * -(d[2] * g[1]));
+      M[5].add(vb * -(d[2] * g[2]));
     }
-    for (int r = 0; r < D; ++r) rhs[r] = G[r].value();
-    floored_solve<D>(m, rhs, static_cast<double>(p.eigen_floor), out);
-#pragma unroll
-    for (int r = 0; r < D; ++r) grad_rho[a * D + r] = static_cast<T>(out[r]);
+  });
+  double m[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, rhs[3] = {0, 0, 0}, out[3];
+  m[0][0] = me.sum(M[0]);
+  m[1][0] = m[0][1] = me.sum(M[1]);
+  m[1][1] = me.sum(M[2]);
+  if (D == 3) {
+    m[2][0] = m[0][2] = me.sum(M[3]);
+    m[2][1] = m[1][2] = me.sum(M[4]);
+    m[2][2] = me.sum(M[5]);
   }
+  for (int r = 0; r < D; ++r) rhs[r] = me.sum(G[r]);
+  if (me.lane) return;
+  floored_solve<D>(m, rhs, static_cast<double>(p.eigen_floor), out);
+#pragma unroll
+  for (int r = 0; r < D; ++r) grad_rho[a * D + r] = static_cast<T>(out[r]);
 }
 
 // ---------------------------------------------------------- K3 diffusion ---
 
-template <class T, int D>
-__global__ void diffusion_kernel(WP<T> p, const Q4<T>* __restrict__ pm, const int64_t* __restrict__ rowptr,
-                                 const uint32_t* __restrict__ ent, const T* __restrict__ rho_s,
-                                 const T* __restrict__ grad_rho, T* __restrict__ rho_all,
-                                 T* __restrict__ p_all) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < p.n; a += gridDim.x * blockDim.x) {
-    const Q4<T> pa = pm[a];
-    const T ra = rho_s[a];
-    T ga[3] = {0, 0, 0};
-    if (p.form == 1)
-      for (int r = 0; r < D; ++r) ga[r] = grad_rho[a * D + r];
-    CSum<T> rate;
-    const int64_t beg = rowptr[a], end = rowptr[a + 1];
-    for (int64_t e = beg; e < end; ++e) {
-      const uint32_t b = ent[e] & kIndexMask;
-      if (b >= p.n) continue;
-      const Q4<T> pb = pm[b];
-      T d[3];
-      separation<T, D>(pa, pb, p, d);
-      T W, gs;
-      const T r = sqrt(norm2<T, D>(d));
-      p.k.wg(r, W, gs);
-      T radial = -(d[0] * (d[0] * gs) + d[1] * (d[1] * gs) + (D == 3 ? d[2] * (d[2] * gs) : T(0)));
-      T contrast = ra - rho_s[b];
-      if (p.form == 1) {
-        T proj = T(0);
-        for (int k = 0; k < D; ++k) proj += (ga[k] + grad_rho[static_cast<int64_t>(b) * D + k]) * d[k];
-        contrast = contrast - T(0.5) * proj;
-      }
-      const T coupling = contrast * radial / (r * r + T(1e-12));
-      rate.add((-p.dscale * (pb.w / rho_s[b])) * coupling);
+template <class T, int D, int L>
+__global__ void __launch_bounds__(kGatherBlock) diffusion_kernel(WP<T> p, const Q4<T>* __restrict__ pm,
+                                                                 const int64_t* __restrict__ rowptr,
+                                                                 const uint32_t* __restrict__ ent,
+                                                                 const Q2<T>* __restrict__ rv,
+                                                                 const T* __restrict__ grad_rho,
+                                                                 Q2<T>* __restrict__ rp) {
+  const RowLanes<L> me;
+  const int64_t a = me.row;
+  if (a >= p.n) return;
+  const Q4<T> pa = pm[a];
+  const T ra = rv[a].x;
+  T ga[3] = {0, 0, 0};
+  if (p.form == 1)
+    for (int r = 0; r < D; ++r) ga[r] = grad_rho[a * D + r];
+  CSum<T> rate;
+  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+    const uint32_t b = e & kIndexMask;
+    if (b >= p.n) return;
+    const Q4<T> pb = pm[b];
+    const Q2<T> sb = rv[b];
+    T d[3];
+    separation<T, D>(pa, pb, p, d);
+    T W, gs;
+    const T r2 = norm2<T, D>(d);
+    p.k.wg2(r2, W, gs);
+    T radial = -(d[0] * (d[0] * gs) + d[1] * (d[1] * gs) + (D == 3 ? d[2] * (d[2] * gs) : T(0)));
+    T contrast = ra - sb.x;
+    if (p.form == 1) {
+      T proj = T(0);
+      for (int k = 0; k < D; ++k) proj += (ga[k] + grad_rho[static_cast<int64_t>(b) * D + k]) * d[k];
+      contrast = contrast - T(0.5) * proj;
     }
-    T rho = ra + p.dt * rate.value();
-    rho = rho > p.rho_floor ? rho : p.rho_floor;
-    rho_all[a] = rho;
-    p_all[a] = tait(rho, p);
-  }
+    const T coupling = contrast * radial / (r2 + T(1e-12));
+    rate.add((-p.dscale * sb.y) * coupling);
+  });
+  T rho = ra + p.dt * me.sum(rate);
+  if (me.lane) return;
+  rho = rho > p.rho_floor ? rho : p.rho_floor;
+  rp[a] = Q2<T>{rho, tait(rho, p)};
 }
 
 // -------------------------------------------------------------- K4 walls ---
 
-template <class T, int D>
-__global__ void wall_kernel(WP<T> p, const Q4<T>* __restrict__ pm, const int64_t* __restrict__ rowptr,
-                            const uint32_t* __restrict__ ent, const T* __restrict__ wall_accel,
-                            T* __restrict__ rho_all, T* __restrict__ p_all, T* __restrict__ face) {
-  for (int64_t w = blockIdx.x * blockDim.x + threadIdx.x; w < p.nw; w += gridDim.x * blockDim.x) {
-    const int64_t a = p.n + w;
-    const Q4<T> pa = pm[a];
-    T acc_w[2] = {T(0), T(0)};
-    if (p.has_wall_accel) { acc_w[0] = wall_accel[w * D]; acc_w[1] = wall_accel[w * D + 1]; }
-    CSum<T> num, den;
-    const int64_t beg = rowptr[a], end = rowptr[a + 1];
-    for (int64_t e = beg; e < end; ++e) {
-      const uint32_t f = ent[e] & kIndexMask;
-      if (f >= p.n) continue;
-      const Q4<T> pb = pm[f];
-      T d[3];  // r_w - r_f
-      separation<T, D>(pa, pb, p, d);
-      const T W = p.k.w(sqrt(norm2<T, D>(d)));
-      T src = p_all[f];
-      if (p.grav != T(0)) {
-        T body = -p.grav * d[1];
-        if (p.has_wall_accel) body = body - (acc_w[0] * d[0] + acc_w[1] * d[1]);
-        src = src + rho_all[f] * body;
-      }
-      num.add(src * W);
-      den.add(W);
+template <class T, int D, int L>
+__global__ void __launch_bounds__(kGatherBlock) wall_kernel(WP<T> p, const Q4<T>* __restrict__ pm,
+                                                            const int64_t* __restrict__ rowptr,
+                                                            const uint32_t* __restrict__ ent,
+                                                            const T* __restrict__ wall_accel, Q2<T>* rp,
+                                                            T* __restrict__ face) {
+  const RowLanes<L> me;
+  const int64_t w = me.row;
+  if (w >= p.nw) return;
+  const int64_t a = p.n + w;
+  const Q4<T> pa = pm[a];
+  T acc_w[2] = {T(0), T(0)};
+  if (p.has_wall_accel) { acc_w[0] = wall_accel[w * D]; acc_w[1] = wall_accel[w * D + 1]; }
+  CSum<T> num, den;
+  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+    const uint32_t f = e & kIndexMask;
+    if (f >= p.n) return;
+    const Q4<T> pb = pm[f];
+    const Q2<T> sf = rp[f];
+    T d[3];  // r_w - r_f
+    separation<T, D>(pa, pb, p, d);
+    const T W = p.k.w2(norm2<T, D>(d));
+    T src = sf.y;
+    if (p.grav != T(0)) {
+      T body = -p.grav * d[1];
+      if (p.has_wall_accel) body = body - (acc_w[0] * d[0] + acc_w[1] * d[1]);
+      src = src + sf.x * body;
     }
-    T dd = den.value();
-    T pw = num.value() / (dd > T(1e-30) ? dd : T(1e-30));
-    pw = pw > T(0) ? pw : T(0);
-    T rw = p.rho0 * pow(pw / p.bulk + T(1), p.inv_gamma);
-    rw = rw > p.rho0 ? rw : p.rho0;
-    p_all[a] = pw;
-    rho_all[a] = rw;
-    if (face) face[w] = pw;
-  }
+    num.add(src * W);
+    den.add(W);
+  });
+  const T dd = me.sum(den), nn = me.sum(num);
+  if (me.lane) return;
+  T pw = nn / (dd > T(1e-30) ? dd : T(1e-30));
+  pw = pw > T(0) ? pw : T(0);
+  T rw = p.rho0 * pow(pw / p.bulk + T(1), p.inv_gamma);
+  rw = rw > p.rho0 ? rw : p.rho0;
+  rp[a] = Q2<T>{rw, pw};
+  if (face) face[w] = pw;
 }
 
 // Boundary-consistent density (droplet_impact.py:1090-1112): the walls enter
 // the fluid summation with their extrapolated density.
-template <class T, int D>
-__global__ void wall_density_correction(WP<T> p, const Q4<T>* __restrict__ pm,
-                                        const int64_t* __restrict__ rowptr, const uint32_t* __restrict__ ent,
-                                        T* __restrict__ rho_all, T* __restrict__ p_all) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < p.n; a += gridDim.x * blockDim.x) {
-    const Q4<T> pa = pm[a];
-    CSum<T> corr;
-    const int64_t beg = rowptr[a], end = rowptr[a + 1];
-    for (int64_t e = beg; e < end; ++e) {
-      const uint32_t b = ent[e] & kIndexMask;
-      if (b < p.n) continue;
-      const Q4<T> pb = pm[b];
-      T d[3];
-      separation<T, D>(pa, pb, p, d);
-      const T W = p.k.w(sqrt(norm2<T, D>(d)));
-      const T dmass = pb.w * (rho_all[b] / p.rho0) - pb.w;
-      corr.add(dmass * W);
-    }
-    T rho = rho_all[a] + corr.value();
-    rho = rho > p.rho_floor ? rho : p.rho_floor;
-    rho_all[a] = rho;
-    p_all[a] = tait(rho, p);
-  }
+template <class T, int D, int L>
+__global__ void __launch_bounds__(kGatherBlock) wall_density_correction(WP<T> p, const Q4<T>* __restrict__ pm,
+                                                                        const int64_t* __restrict__ rowptr,
+                                                                        const uint32_t* __restrict__ ent, Q2<T>* rp) {
+  const RowLanes<L> me;
+  const int64_t a = me.row;
+  if (a >= p.n) return;
+  const Q4<T> pa = pm[a];
+  CSum<T> corr;
+  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+    const uint32_t b = e & kIndexMask;
+    if (b < p.n) return;
+    const Q4<T> pb = pm[b];
+    T d[3];
+    separation<T, D>(pa, pb, p, d);
+    const T W = p.k.w2(norm2<T, D>(d));
+    const T dmass = pb.w * (rp[b].x / p.rho0) - pb.w;
+    corr.add(dmass * W);
+  });
+  const T more = me.sum(corr);
+  if (me.lane) return;
+  T rho = rp[a].x + more;
+  rho = rho > p.rho_floor ? rho : p.rho_floor;
+  rp[a] = Q2<T>{rho, tait(rho, p)};
 }
 
 // -------------------------------------------------------------- K5 force ---
@@ -437,136 +463,147 @@ __device__ __forceinline__ T visc_scale(const WP<T>& p, bool a_fluid, bool b_flu
   return T(2) * nu * blend;
 }
 
-template <class T, int D>
-__global__ void force_kernel(WP<T> p, const Q4<T>* __restrict__ pm, const Q4<T>* __restrict__ vv,
-                             const int64_t* __restrict__ rowptr, const uint32_t* __restrict__ ent,
-                             const T* __restrict__ rho_all, const T* __restrict__ p_all, T* __restrict__ acc) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < p.n; a += gridDim.x * blockDim.x) {
-    const Q4<T> pa = pm[a], va = vv[a];
-    const T ra = rho_all[a];
-    const T Pa = p_all[a] / (ra * ra);
-    CSum<T> ax, ay, az;
-    const T eta2 = p.visc_eps;
-    const int64_t beg = rowptr[a], end = rowptr[a + 1];
-    for (int64_t e = beg; e < end; ++e) {
-      const uint32_t b = ent[e] & kIndexMask;
-      const Q4<T> pb = pm[b], vb = vv[b];
-      T d[3];
-      separation<T, D>(pa, pb, p, d);
-      const T r = sqrt(norm2<T, D>(d));
-      T W, gs;
-      p.k.wg(r, W, gs);
-      if (gs == T(0)) continue;
-      const T g[3] = {d[0] * gs, d[1] * gs, d[2] * gs};
-      const T rb = rho_all[b];
-      const T term = Pa + p_all[b] / (rb * rb);
-      const T fp_ = -pb.w * term;
-      T fx = fp_ * g[0], fy = fp_ * g[1], fz = fp_ * g[2];
-      const T vs = visc_scale(p, true, b < p.n, va.w, vb.w);
-      if (vs != T(0)) {
-        T dot = d[0] * g[0] + d[1] * g[1] + (D == 3 ? d[2] * g[2] : T(0));
-        T lw = -dot;
-        lw = (lw > T(0) ? lw : T(0)) / (r * r + eta2);
-        const T coef = -vs * (pb.w / rb * lw);
-        fx += coef * (va.x - vb.x);
-        fy += coef * (va.y - vb.y);
-        if (D == 3) fz += coef * (va.z - vb.z);
-      }
-      ax.add(fx);
-      ay.add(fy);
-      if (D == 3) az.add(fz);
+// vq: (m / rho, p / rho^2).
+template <class T, int D, int L>
+__global__ void __launch_bounds__(kGatherBlock) force_kernel(WP<T> p, const Q4<T>* __restrict__ pm,
+                                                             const Q4<T>* __restrict__ vv,
+                                                             const int64_t* __restrict__ rowptr,
+                                                             const uint32_t* __restrict__ ent,
+                                                             const Q2<T>* __restrict__ vq, T* __restrict__ acc) {
+  const RowLanes<L> me;
+  const int64_t a = me.row;
+  if (a >= p.n) return;
+  const Q4<T> pa = pm[a], va = vv[a];
+  const T Pa = vq[a].y;
+  CSum<T> ax, ay, az;
+  const T eta2 = p.visc_eps;
+  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+    const uint32_t b = e & kIndexMask;
+    const Q4<T> pb = pm[b], vb = vv[b];
+    const Q2<T> qb = vq[b];
+    T d[3];
+    separation<T, D>(pa, pb, p, d);
+    const T r2 = norm2<T, D>(d);
+    T W, gs;
+    p.k.wg2(r2, W, gs);
+    if (gs == T(0)) return;
+    const T g[3] = {d[0] * gs, d[1] * gs, d[2] * gs};
+    const T fp_ = -pb.w * (Pa + qb.y);
+    T fx = fp_ * g[0], fy = fp_ * g[1], fz = fp_ * g[2];
+    const T vs = visc_scale(p, true, b < p.n, va.w, vb.w);
+    if (vs != T(0)) {
+      T dot = d[0] * g[0] + d[1] * g[1] + (D == 3 ? d[2] * g[2] : T(0));
+      T lw = -dot;
+      lw = (lw > T(0) ? lw : T(0)) / (r2 + eta2);
+      const T coef = -vs * (qb.x * lw);
+      fx += coef * (va.x - vb.x);
+      fy += coef * (va.y - vb.y);
+      if (D == 3) fz += coef * (va.z - vb.z);
     }
-    acc[a * D] = ax.value();
-    acc[a * D + 1] = ay.value() - p.grav;
-    if (D == 3) acc[a * D + 2] = az.value();
-  }
+    ax.add(fx);
+    ay.add(fy);
+    if (D == 3) az.add(fz);
+  });
+  const T sx = me.sum(ax), sy = me.sum(ay), sz = D == 3 ? me.sum(az) : T(0);
+  if (me.lane) return;
+  acc[a * D] = sx;
+  acc[a * D + 1] = sy - p.grav;
+  if (D == 3) acc[a * D + 2] = sz;
 }
 
 // ----------------------------------------------------------- K6 reaction ---
 
-template <class T, int D>
-__global__ void reaction_kernel(WP<T> p, const Q4<T>* __restrict__ pm, const Q4<T>* __restrict__ vv,
-                                const int64_t* __restrict__ rowptr, const uint32_t* __restrict__ ent,
-                                const T* __restrict__ rho_all, const T* __restrict__ p_all,
-                                T* __restrict__ reaction) {
-  for (int64_t w = blockIdx.x * blockDim.x + threadIdx.x; w < p.nw; w += gridDim.x * blockDim.x) {
-    const int64_t a = p.n + w;
-    const Q4<T> pa = pm[a], va = vv[a];
-    const T ra = rho_all[a];
-    const T Pa = p_all[a] / (ra * ra);
-    CSum<T> rx, ry, rz;
-    const int64_t beg = rowptr[a], end = rowptr[a + 1];
-    for (int64_t e = beg; e < end; ++e) {
-      const uint32_t f = ent[e] & kIndexMask;
-      if (f >= p.n) continue;
-      const Q4<T> pb = pm[f], vb = vv[f];
-      T d[3];  // r_w - r_f
-      separation<T, D>(pa, pb, p, d);
-      const T r = sqrt(norm2<T, D>(d));
-      T W, gs;
-      p.k.wg(r, W, gs);
-      if (gs == T(0)) continue;
-      const T g[3] = {d[0] * gs, d[1] * gs, d[2] * gs};  // grad_w W_wf
-      const T rf = rho_all[f];
-      const T term = Pa + p_all[f] / (rf * rf);
-      const T c = -(pa.w * pb.w) * term;
-      T fx = c * g[0], fy = c * g[1], fz = c * g[2];
-      const T vs = visc_scale(p, false, true, T(0), vb.w);
-      if (vs != T(0)) {
-        T dot = d[0] * g[0] + d[1] * g[1] + (D == 3 ? d[2] * g[2] : T(0));
-        T lw = -dot;
-        lw = (lw > T(0) ? lw : T(0)) / (r * r + p.visc_eps);
-        const T coef = pb.w * vs * (pa.w / ra * lw);
-        fx += coef * (vb.x - va.x);
-        fy += coef * (vb.y - va.y);
-        if (D == 3) fz += coef * (vb.z - va.z);
-      }
-      rx.add(fx);
-      ry.add(fy);
-      if (D == 3) rz.add(fz);
+template <class T, int D, int L>
+__global__ void __launch_bounds__(kGatherBlock) reaction_kernel(WP<T> p, const Q4<T>* __restrict__ pm,
+                                                                const Q4<T>* __restrict__ vv,
+                                                                const int64_t* __restrict__ rowptr,
+                                                                const uint32_t* __restrict__ ent,
+                                                                const Q2<T>* __restrict__ vq,
+                                                                T* __restrict__ reaction) {
+  const RowLanes<L> me;
+  const int64_t w = me.row;
+  if (w >= p.nw) return;
+  const int64_t a = p.n + w;
+  const Q4<T> pa = pm[a], va = vv[a];
+  const Q2<T> qa = vq[a];
+  CSum<T> rx, ry, rz;
+  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+    const uint32_t f = e & kIndexMask;
+    if (f >= p.n) return;
+    const Q4<T> pb = pm[f], vb = vv[f];
+    T d[3];  // r_w - r_f
+    separation<T, D>(pa, pb, p, d);
+    const T r2 = norm2<T, D>(d);
+    T W, gs;
+    p.k.wg2(r2, W, gs);
+    if (gs == T(0)) return;
+    const T g[3] = {d[0] * gs, d[1] * gs, d[2] * gs};  // grad_w W_wf
+    const T c = -(pa.w * pb.w) * (qa.y + vq[f].y);
+    T fx = c * g[0], fy = c * g[1], fz = c * g[2];
+    const T vs = visc_scale(p, false, true, T(0), vb.w);
+    if (vs != T(0)) {
+      T dot = d[0] * g[0] + d[1] * g[1] + (D == 3 ? d[2] * g[2] : T(0));
+      T lw = -dot;
+      lw = (lw > T(0) ? lw : T(0)) / (r2 + p.visc_eps);
+      const T coef = pb.w * vs * (qa.x * lw);
+      fx += coef * (vb.x - va.x);
+      fy += coef * (vb.y - va.y);
+      if (D == 3) fz += coef * (vb.z - va.z);
     }
-    reaction[w * D] = rx.value();
-    reaction[w * D + 1] = ry.value();
-    if (D == 3) reaction[w * D + 2] = rz.value();
-  }
-}
-
-template <class T>
-__global__ void copy_out(const T* __restrict__ src, T* __restrict__ dst, int64_t n) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) dst[a] = src[a];
+    rx.add(fx);
+    ry.add(fy);
+    if (D == 3) rz.add(fz);
+  });
+  const T sx = me.sum(rx), sy = me.sum(ry), sz = D == 3 ? me.sum(rz) : T(0);
+  if (me.lane) return;
+  reaction[w * D] = sx;
+  reaction[w * D + 1] = sy;
+  if (D == 3) reaction[w * D + 2] = sz;
 }
 
 struct RhsLayout {
-  size_t pm, vv, rho_all, p_all, rho_s, grad, csum, p_tmp, known, total;
+  size_t pm, vv, rp, rv, grad, csum, pres[2], known, total;
 };
 
+// The velocities are packed last, so vv's space first holds what only the
+// diffusion or the closure needs: rv and, in 2-D, the density gradient (3-D has
+// it after the rest), or the closure's two pressure buffers.
 RhsLayout rhs_layout(const tsph_wcsph_params& prm) {
   const size_t ts = prm.dtype == TSPH_F64 ? 8 : 4;
-  const int64_t all = prm.n_fluid + prm.n_wall;
+  const int64_t n = prm.n_fluid, all = n + prm.n_wall;
   RhsLayout L{};
   size_t off = 0;
   L.pm = off; off += align_up(all * 4 * ts);
   L.vv = off; off += align_up(all * 4 * ts);
-  L.rho_all = off; off += align_up(all * ts);
-  L.p_all = off; off += align_up(all * ts);
-  L.rho_s = off; off += align_up(prm.n_fluid * ts);
-  L.grad = off; off += align_up(prm.n_fluid * prm.dim * ts);
+  L.rp = off; off += align_up(all * 2 * ts);
+  L.rv = L.vv;
+  L.pres[0] = L.vv;
+  L.pres[1] = L.vv + n * ts;
+  if (prm.dim == 2) {
+    L.grad = L.vv + n * 2 * ts;
+  } else {
+    L.grad = off; off += prm.diffusion_form == 1 ? align_up(n * 3 * ts) : 0;
+  }
   const bool comp = prm.flags & TSPH_RHS_COMPRESSION, closure = prm.flags & TSPH_RHS_SURFACE_CLOSURE;
-  L.csum = off; off += comp ? align_up(prm.n_fluid * ts) : 0;
-  L.p_tmp = off; off += closure ? align_up(prm.n_fluid * ts) : 0;
-  L.known = off; off += closure ? align_up(2 * prm.n_fluid) : 0;
-  L.total = off + 256;
+  L.csum = off; off += comp ? align_up(n * ts) : 0;
+  L.known = off; off += closure ? align_up(2 * n) : 0;
+  // The size a call asks for also decides which ones the allocation-free entry
+  // point takes (300 k FP32 particles): it stays 13 (2-D) or 14 (3-D) words a
+  // fluid particle and 10 a wall particle, one more word per fluid particle
+  // with the compression and with the closure, though less is used.
+  size_t ask = 2 * align_up(all * 4 * ts) + 2 * align_up(all * ts) + align_up(n * ts) + align_up(n * prm.dim * ts);
+  ask += (comp ? align_up(n * ts) : 0) + (closure ? align_up(n * ts) + align_up(2 * n) : 0);
+  L.total = (off > ask ? off : ask) + 256;
   return L;
 }
 
-template <class T, int D>
-int run_rhs(const tsph_wcsph_params& prm, const tsph_wcsph_io& io, char* ws, cudaStream_t s) {
+template <class T, int D, int LN>
+int run_rows(const tsph_wcsph_params& prm, const tsph_wcsph_io& io, char* ws, cudaStream_t s) {
   RhsLayout L = rhs_layout(prm);
   Q4<T>* pm = reinterpret_cast<Q4<T>*>(ws + L.pm);
   Q4<T>* vv = reinterpret_cast<Q4<T>*>(ws + L.vv);
-  T* rho_all = reinterpret_cast<T*>(ws + L.rho_all);
-  T* p_all = reinterpret_cast<T*>(ws + L.p_all);
-  T* rho_s = reinterpret_cast<T*>(ws + L.rho_s);
+  Q2<T>* rp = reinterpret_cast<Q2<T>*>(ws + L.rp);
+  Q2<T>* rv = reinterpret_cast<Q2<T>*>(ws + L.rv);
   T* grad = reinterpret_cast<T*>(ws + L.grad);
   const int64_t n = prm.n_fluid, nw = prm.n_wall;
 
@@ -596,87 +633,79 @@ int run_rhs(const tsph_wcsph_params& prm, const tsph_wcsph_io& io, char* ws, cud
   p.w0 = static_cast<T>(prm.sigma);
   p.lattice_sum = static_cast<T>(prm.lattice_sum);
   p.eigen_floor = static_cast<T>(prm.eigen_floor);
-  p.k.h = static_cast<T>(prm.h);
-  p.k.inv_h = static_cast<T>(1.0 / prm.h);
-  p.k.sigma = static_cast<T>(prm.sigma);
-  p.k.eps = static_cast<T>(1e-12);
+  p.k = make_cubic<T>(prm.h, prm.sigma);
 
-  const int B = 128;
+  constexpr int B = kGatherBlock;
+  const unsigned rows = row_grid(n, LN), wall_rows = row_grid(nw, LN);
   pack_kernel<T, D><<<grid_for(n + nw, 256), 256, 0, s>>>(
-      static_cast<const T*>(io.pos), static_cast<const T*>(io.vel), static_cast<const T*>(io.mass),
-      static_cast<const T*>(io.wall), static_cast<const T*>(io.wall_vel), static_cast<const T*>(io.nu_field),
-      n, nw, static_cast<T>(prm.wall_mass), pm, vv);
+      static_cast<const T*>(io.pos), static_cast<const T*>(io.mass), static_cast<const T*>(io.wall), n, nw,
+      static_cast<T>(prm.wall_mass), pm);
   TSPH_LAUNCH_CHECK();
-  density_kernel<T, D><<<grid_for(n, B), B, 0, s>>>(p, pm, io.rowptr, io.entries,
-                                                    static_cast<const T*>(io.density_offset), rho_s,
-                                                    rho_all, p_all);
+  density_kernel<T, D, LN><<<rows, B, 0, s>>>(p, pm, io.rowptr, io.entries, static_cast<const T*>(io.density_offset),
+                                              rv, rp);
   TSPH_LAUNCH_CHECK();
   if (p.diffusion) {
     if (p.form == 1) {
-      gradient_kernel<T, D><<<grid_for(n, B), B, 0, s>>>(p, pm, io.rowptr, io.entries, rho_s, grad);
+      gradient_kernel<T, D, LN><<<rows, B, 0, s>>>(p, pm, io.rowptr, io.entries, rv, grad);
       TSPH_LAUNCH_CHECK();
     }
-    diffusion_kernel<T, D><<<grid_for(n, B), B, 0, s>>>(p, pm, io.rowptr, io.entries, rho_s, grad,
-                                                        rho_all, p_all);
+    diffusion_kernel<T, D, LN><<<rows, B, 0, s>>>(p, pm, io.rowptr, io.entries, rv, grad, rp);
     TSPH_LAUNCH_CHECK();
   }
   if (prm.flags & TSPH_RHS_COMPRESSION) {
     T* csum = reinterpret_cast<T*>(ws + L.csum);
-    compression_kernel<T, D><<<grid_for(n, B), B, 0, s>>>(p, pm, io.rowptr, io.entries,
-                                                          static_cast<T>(prm.compression_kref),
-                                                          prm.compression_rule == 1 ? 1 : 0, csum, rho_s,
-                                                          rho_all, p_all);
+    compression_kernel<T, D, LN><<<rows, B, 0, s>>>(p, pm, io.rowptr, io.entries,
+                                                    static_cast<T>(prm.compression_kref),
+                                                    prm.compression_rule == 1 ? 1 : 0, csum, rp);
     TSPH_LAUNCH_CHECK();
     compression_average<T><<<1, 1024, 0, s>>>(csum, n, io.compression_out);
     TSPH_LAUNCH_CHECK();
   }
   if (prm.flags & TSPH_RHS_SURFACE_CLOSURE) {
-    T* p_tmp = reinterpret_cast<T*>(ws + L.p_tmp);
     uint8_t* known[2] = {reinterpret_cast<uint8_t*>(ws + L.known), reinterpret_cast<uint8_t*>(ws + L.known) + n};
-    T* pres[2] = {p_all, p_tmp};
-    closure_init<T><<<grid_for(n, 256), 256, 0, s>>>(p, rho_all, static_cast<T>(prm.surface_threshold * prm.rho0),
-                                                     known[0]);
+    T* pres[2] = {reinterpret_cast<T*>(ws + L.pres[0]), reinterpret_cast<T*>(ws + L.pres[1])};
+    closure_init<T><<<grid_for(n, 256), 256, 0, s>>>(p, rp, static_cast<T>(prm.surface_threshold * prm.rho0),
+                                                     known[0], pres[0]);
     TSPH_LAUNCH_CHECK();
     const int donors = static_cast<int>(prm.surface_donors);
     const int64_t passes = donors == 0 ? (prm.surface_layers > 1 ? prm.surface_layers : 1) : 1;
     for (int64_t k = 0; k < passes; ++k) {
-      closure_pass<T, D><<<grid_for(n, B), B, 0, s>>>(p, pm, io.rowptr, io.entries, rho_all, donors,
-                                                      pres[k & 1], known[k & 1], pres[(k + 1) & 1],
-                                                      known[(k + 1) & 1]);
+      closure_pass<T, D><<<grid_for(n, B), B, 0, s>>>(p, pm, io.rowptr, io.entries, rp, donors, pres[k & 1],
+                                                      known[k & 1], pres[(k + 1) & 1], known[(k + 1) & 1]);
       TSPH_LAUNCH_CHECK();
     }
-    if (passes & 1) {
-      TSPH_CUDA_CHECK(cudaMemcpyAsync(p_all, p_tmp, n * sizeof(T), cudaMemcpyDeviceToDevice, s));
-    }
+    closure_finish<T><<<grid_for(n, 256), 256, 0, s>>>(n, pres[passes & 1], rp);
+    TSPH_LAUNCH_CHECK();
   }
   T* face = (prm.flags & TSPH_RHS_SPLIT) ? static_cast<T*>(io.face_pressure) : nullptr;
   if (nw) {
-    wall_kernel<T, D><<<grid_for(nw, B), B, 0, s>>>(p, pm, io.rowptr, io.entries,
-                                                    static_cast<const T*>(io.wall_accel), rho_all, p_all,
-                                                    face);
+    const T* wall_accel = static_cast<const T*>(io.wall_accel);
+    wall_kernel<T, D, LN><<<wall_rows, B, 0, s>>>(p, pm, io.rowptr, io.entries, wall_accel, rp, face);
     TSPH_LAUNCH_CHECK();
     if (prm.flags & TSPH_RHS_BOUNDARY_DENSITY) {
-      wall_density_correction<T, D><<<grid_for(n, B), B, 0, s>>>(p, pm, io.rowptr, io.entries, rho_all,
-                                                                 p_all);
+      wall_density_correction<T, D, LN><<<rows, B, 0, s>>>(p, pm, io.rowptr, io.entries, rp);
       TSPH_LAUNCH_CHECK();
-      wall_kernel<T, D><<<grid_for(nw, B), B, 0, s>>>(p, pm, io.rowptr, io.entries,
-                                                      static_cast<const T*>(io.wall_accel), rho_all,
-                                                      p_all, face);
+      wall_kernel<T, D, LN><<<wall_rows, B, 0, s>>>(p, pm, io.rowptr, io.entries, wall_accel, rp, face);
       TSPH_LAUNCH_CHECK();
     }
   }
-  force_kernel<T, D><<<grid_for(n, B), B, 0, s>>>(p, pm, vv, io.rowptr, io.entries, rho_all, p_all,
-                                                  static_cast<T*>(io.acc));
+  state_kernel<T, D><<<grid_for(n + nw, 256), 256, 0, s>>>(
+      static_cast<const T*>(io.vel), static_cast<const T*>(io.wall_vel), static_cast<const T*>(io.nu_field), pm, n,
+      nw, rp, vv, static_cast<T*>(io.rho), static_cast<T*>(io.pressure));
+  TSPH_LAUNCH_CHECK();
+  force_kernel<T, D, LN><<<rows, B, 0, s>>>(p, pm, vv, io.rowptr, io.entries, rp, static_cast<T*>(io.acc));
   TSPH_LAUNCH_CHECK();
   if ((prm.flags & TSPH_RHS_SPLIT) && nw) {
-    reaction_kernel<T, D><<<grid_for(nw, B), B, 0, s>>>(p, pm, vv, io.rowptr, io.entries, rho_all, p_all,
-                                                        static_cast<T*>(io.reaction));
+    reaction_kernel<T, D, LN><<<wall_rows, B, 0, s>>>(p, pm, vv, io.rowptr, io.entries, rp,
+                                                      static_cast<T*>(io.reaction));
     TSPH_LAUNCH_CHECK();
   }
-  copy_out<T><<<grid_for(n, 256), 256, 0, s>>>(rho_all, static_cast<T*>(io.rho), n);
-  copy_out<T><<<grid_for(n, 256), 256, 0, s>>>(p_all, static_cast<T*>(io.pressure), n);
-  TSPH_LAUNCH_CHECK();
   return TSPH_OK;
+}
+
+template <class T, int D>
+int run_rhs(const tsph_wcsph_params& prm, const tsph_wcsph_io& io, char* ws, cudaStream_t s) {
+  return with_lanes<D>(prm.n_fluid, [&](auto lanes) { return run_rows<T, D, decltype(lanes)::value>(prm, io, ws, s); });
 }
 
 }  // namespace
