@@ -635,7 +635,7 @@ L2 layout2(int64_t n, int64_t m, int64_t dtype) {
   L.minv = take(3 * n * t);
   L.det = take(n * t);
   L.keys = take(n * 8);
-  L.hist = take(256 * 4);
+  L.hist = take(kSelectHist);
   L.sel = take(2 * 8);
   L.mag = take(n * t);
   L.n0 = take(2 * n * t);
@@ -758,9 +758,8 @@ int run_csf2(const tsph_csf2_params& prm, const tsph_csf2_io& io, char* ws, cuda
                                                vol);
   k2_colour<T><<<g, 128, 0, s>>>(p, xy, vol, io.rowptr, io.entries, color, mm, det, keys);
   TSPH_LAUNCH_CHECK();
-  TSPH_CUDA_CHECK(cudaMemsetAsync(hist, 0, 256 * sizeof(unsigned int), s));
   TSPH_CUDA_CHECK(cudaMemsetAsync(maxima, 0, 4 * sizeof(unsigned long long), s));
-  radix_select_u64(keys, n, sizeof(T) == 8 ? 64 : 32, (n - 1) / 2, sel, hist, s, grid_for(n, 256, 148 * 4));
+  if (int rc = radix_select_u64(keys, n, sizeof(T) == 8 ? 64 : 32, (n - 1) / 2, sel, hist, s)) return rc;
   const int passes = static_cast<int>(prm.normal_smoothing);
   Walls<T> walls;
   const bool rotate = prm.n_wall > 0 && prm.contact_model == 1;
@@ -832,8 +831,7 @@ int run_accel2(const tsph_csf2_params& prm, const tsph_csf2_io& io, const void* 
       uint64_t* keys = reinterpret_cast<uint64_t*>(ws + L.wkeys);
       unsigned int* hist = reinterpret_cast<unsigned int*>(ws + L.hist);
       k2_wall_nn<T><<<static_cast<unsigned>((m + kTile - 1) / kTile), kTile, 0, s>>>(m, wall, keys);
-      TSPH_CUDA_CHECK(cudaMemsetAsync(hist, 0, 256 * sizeof(unsigned int), s));
-      radix_select_u64(keys, m, sizeof(T) == 8 ? 64 : 32, (m - 1) / 2, sel, hist, s, grid_for(m, 256, 148 * 4));
+      if (int rc = radix_select_u64(keys, m, sizeof(T) == 8 ? 64 : 32, (m - 1) / 2, sel, hist, s)) return rc;
     }
     weight = reinterpret_cast<T*>(ws + L.wweight);
     k2_wall_weight<T><<<static_cast<unsigned>((prm.n + kTile - 1) / kTile), kTile, 0, s>>>(p, m, pos, wall, sel,

@@ -18,13 +18,14 @@
 //                           0 where the fit does not hold (csf3.py:168-220)
 //   A  acceleration         a = -sigma kappa delta_s [delta_s > cutoff max delta_s] n / rho
 // Separations use the minimum image in a periodic box (operators3.py:51-67).
-// Every row is summed by its own thread in a fixed order: no floating-point
-// atomics, deterministic results.  The 3x3 inverse is the adjugate over the
+// Every row is summed by its own two to eight lanes in a fixed order
+// (gather.cuh): no floating-point atomics, deterministic results.  The 3x3 inverse is the adjugate over the
 // determinant (the reference solves with LU; both round at the last bits).
 #include <cmath>
 
 #include "common.cuh"
 #include "fpmath.cuh"
+#include "gather.cuh"
 #include "sphkernels.cuh"
 #include "quadfit.cuh"
 #include "radix_select.cuh"
@@ -32,18 +33,11 @@
 namespace tsph {
 namespace {
 
-constexpr uint32_t kIndexMask = 0x7fffffffu;
-
-template <class T>
-struct alignas(4 * sizeof(T)) Q4 {
-  T x, y, z, w;
-};
-
 template <class T>
 struct CP {
   int64_t n;
   int periodic, has_volume;
-  T box[3];
+  T box[3], half[3];
   T rho0, w0, sigma, cutoff;
   Cubic<T> k;
 };
@@ -53,19 +47,16 @@ __device__ __forceinline__ void sep(const Q4<T>& a, const Q4<T>& b, const CP<T>&
   d[0] = a.x - b.x;
   d[1] = a.y - b.y;
   d[2] = a.z - b.z;
-  if (p.periodic) {
+  // most neighbours need no image on any axis
+  if (p.periodic && !(fabs(d[0]) <= p.half[0] && fabs(d[1]) <= p.half[1] && fabs(d[2]) <= p.half[2])) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) d[k] = fp<T>::min_image(d[k], p.box[k]);
   }
 }
 
-// grad_a W_ab = d * g for the separation d = x_a - x_b
 template <class T>
-__device__ __forceinline__ T grad_scale(const CP<T>& p, const T d[3], T* W) {
-  T w, g;
-  p.k.wg(sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]), w, g);
-  if (W) *W = w;
-  return g;
+__device__ __forceinline__ T norm2(const T d[3]) {
+  return d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
 }
 
 // Symmetric 3x3 stored as (xx, xy, xz, yy, yz, zz).
@@ -96,131 +87,143 @@ __global__ void c_pack(CP<T> p, const T* __restrict__ pos, const T* __restrict__
 }
 
 // C1: colour, M (symmetric, 6 values) and |det M| (as its IEEE bits for the select)
-template <class T>
-__global__ void c_colour(CP<T> p, const Q4<T>* __restrict__ pv, const int64_t* __restrict__ rowptr,
-                         const uint32_t* __restrict__ ent, T* __restrict__ color, T* __restrict__ mm,
-                         T* __restrict__ det, uint64_t* __restrict__ keys) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < p.n; a += gridDim.x * blockDim.x) {
-    const Q4<T> pa = pv[a];
-    CSum<T> c;
-    CSum<T> m[6];
-    for (int64_t e = rowptr[a]; e < rowptr[a + 1]; ++e) {
-      const Q4<T> pb = pv[ent[e] & kIndexMask];
-      T d[3], w;
-      sep(pa, pb, p, d);
-      const T g = grad_scale(p, d, &w);
-      c.add(pb.w * w);
-      // V_b (x_b - x_a) (x) grad_a W = -V_b g d (x) d
-      const T s = -pb.w * g;
-      m[0].add(s * d[0] * d[0]);
-      m[1].add(s * d[0] * d[1]);
-      m[2].add(s * d[0] * d[2]);
-      m[3].add(s * d[1] * d[1]);
-      m[4].add(s * d[1] * d[2]);
-      m[5].add(s * d[2] * d[2]);
-    }
-    c.add(pa.w * p.w0);
-    color[a] = c.value();
-    T mv[6];
+template <class T, int L>
+__global__ void __launch_bounds__(kGatherBlock) c_colour(CP<T> p, const Q4<T>* __restrict__ pv,
+                                                         const int64_t* __restrict__ rowptr,
+                                                         const uint32_t* __restrict__ ent, T* __restrict__ color,
+                                                         T* __restrict__ mm, T* __restrict__ det,
+                                                         uint64_t* __restrict__ keys) {
+  const RowLanes<L> me;
+  const int64_t a = me.row;
+  if (a >= p.n) return;
+  const Q4<T> pa = pv[a];
+  CSum<T> c;
+  CSum<T> m[6];
+  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+    const Q4<T> pb = pv[e & kIndexMask];
+    T d[3], w, g;
+    sep(pa, pb, p, d);
+    p.k.wg2(norm2(d), w, g);
+    c.add(pb.w * w);
+    // V_b (x_b - x_a) (x) grad_a W = -V_b g d (x) d
+    const T s = -pb.w * g;
+    m[0].add(s * d[0] * d[0]);
+    m[1].add(s * d[0] * d[1]);
+    m[2].add(s * d[0] * d[2]);
+    m[3].add(s * d[1] * d[1]);
+    m[4].add(s * d[1] * d[2]);
+    m[5].add(s * d[2] * d[2]);
+  });
+  if (me.lane == 0) c.add(pa.w * p.w0);
+  const T cv = me.sum(c);
+  T mv[6];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      mv[k] = m[k].value();
-      mm[6 * a + k] = mv[k];
-    }
-    const T dv = det_sym(mv);
-    det[a] = dv;
-    const T ad = dv < T(0) ? -dv : dv;
-    keys[a] = sizeof(T) == 8 ? static_cast<uint64_t>(__double_as_longlong(static_cast<double>(ad)))
-                             : static_cast<uint64_t>(__float_as_uint(static_cast<float>(ad)));
-  }
+  for (int k = 0; k < 6; ++k) mv[k] = me.sum(m[k]);
+  if (me.lane) return;
+  color[a] = cv;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) mm[6 * a + k] = mv[k];
+  const T dv = det_sym(mv);
+  det[a] = dv;
+  const T ad = dv < T(0) ? -dv : dv;
+  keys[a] = sizeof(T) == 8 ? static_cast<uint64_t>(__double_as_longlong(static_cast<double>(ad)))
+                           : static_cast<uint64_t>(__float_as_uint(static_cast<float>(ad)));
 }
 
 // C3: validity, inverse, colour gradient, delta_s and the normal
-template <class T>
-__global__ void c_gradient(CP<T> p, const Q4<T>* __restrict__ pv, const int64_t* __restrict__ rowptr,
-                           const uint32_t* __restrict__ ent, const T* __restrict__ color,
-                           const T* __restrict__ mm, const T* __restrict__ det,
-                           const unsigned long long* __restrict__ sel, T* __restrict__ minv,
-                           T* __restrict__ grad_c, T* __restrict__ normal, Q4<T>* __restrict__ nq,
-                           T* __restrict__ delta_s, uint8_t* __restrict__ valid) {
+template <class T, int L>
+__global__ void __launch_bounds__(kGatherBlock) c_gradient(CP<T> p, const Q4<T>* __restrict__ pv,
+                                                           const int64_t* __restrict__ rowptr,
+                                                           const uint32_t* __restrict__ ent,
+                                                           const T* __restrict__ color, const T* __restrict__ mm,
+                                                           const T* __restrict__ det,
+                                                           const unsigned long long* __restrict__ sel,
+                                                           T* __restrict__ minv, T* __restrict__ grad_c,
+                                                           T* __restrict__ normal, Q4<T>* __restrict__ nq,
+                                                           T* __restrict__ delta_s, uint8_t* __restrict__ valid) {
+  const RowLanes<L> me;
+  const int64_t a = me.row;
+  if (a >= p.n) return;
   const uint64_t mk = sel[0];
   const T med = sizeof(T) == 8 ? static_cast<T>(__longlong_as_double(static_cast<long long>(mk)))
                                : static_cast<T>(__uint_as_float(static_cast<uint32_t>(mk)));
   const T scale = med > T(1e-30) ? med : T(1e-30);
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < p.n; a += gridDim.x * blockDim.x) {
-    const Q4<T> pa = pv[a];
-    const T ca = color[a];
-    CSum<T> nx, ny, nz;
-    for (int64_t e = rowptr[a]; e < rowptr[a + 1]; ++e) {
-      const uint32_t b = ent[e] & kIndexMask;
-      const Q4<T> pb = pv[b];
-      T d[3];
-      sep(pa, pb, p, d);
-      const T s = pb.w * (color[b] - ca) * grad_scale<T>(p, d, nullptr);
-      nx.add(s * d[0]);
-      ny.add(s * d[1]);
-      nz.add(s * d[2]);
-    }
-    const T dv = det[a];
-    const bool ok = (dv < T(0) ? -dv : dv) > T(1e-6) * scale;
-    T iv[6];
-    if (ok) {
-      T m[6];
+  const Q4<T> pa = pv[a];
+  const T ca = color[a];
+  CSum<T> nx, ny, nz;
+  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+    const uint32_t b = e & kIndexMask;
+    const Q4<T> pb = pv[b];
+    T d[3];
+    sep(pa, pb, p, d);
+    const T s = pb.w * (color[b] - ca) * p.k.g2(p.k.radial(norm2(d)));
+    nx.add(s * d[0]);
+    ny.add(s * d[1]);
+    nz.add(s * d[2]);
+  });
+  const T u[3] = {me.sum(nx), me.sum(ny), me.sum(nz)};
+  if (me.lane) return;
+  const T dv = det[a];
+  const bool ok = (dv < T(0) ? -dv : dv) > T(1e-6) * scale;
+  T iv[6];
+  if (ok) {
+    T m[6];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) m[k] = mm[6 * a + k];
-      inv_sym(m, dv, iv);
-    } else {
-      iv[0] = iv[3] = iv[5] = T(1);
-      iv[1] = iv[2] = iv[4] = T(0);
-    }
-#pragma unroll
-    for (int k = 0; k < 6; ++k) minv[6 * a + k] = iv[k];
-    const T u[3] = {nx.value(), ny.value(), nz.value()};
-    const T g[3] = {iv[0] * u[0] + iv[1] * u[1] + iv[2] * u[2], iv[1] * u[0] + iv[3] * u[1] + iv[4] * u[2],
-                    iv[2] * u[0] + iv[4] * u[1] + iv[5] * u[2]};
-    const T mag = sqrt(g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
-    const T den = mag > T(1e-30) ? mag : T(1e-30);
-    const T n3[3] = {-g[0] / den, -g[1] / den, -g[2] / den};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      grad_c[3 * a + k] = g[k];
-      normal[3 * a + k] = n3[k];
-    }
-    nq[a] = Q4<T>{n3[0], n3[1], n3[2], T(0)};
-    delta_s[a] = mag;
-    valid[a] = ok ? 1 : 0;
+    for (int k = 0; k < 6; ++k) m[k] = mm[6 * a + k];
+    inv_sym(m, dv, iv);
+  } else {
+    iv[0] = iv[3] = iv[5] = T(1);
+    iv[1] = iv[2] = iv[4] = T(0);
   }
+#pragma unroll
+  for (int k = 0; k < 6; ++k) minv[6 * a + k] = iv[k];
+  const T g[3] = {iv[0] * u[0] + iv[1] * u[1] + iv[2] * u[2], iv[1] * u[0] + iv[3] * u[1] + iv[4] * u[2],
+                  iv[2] * u[0] + iv[4] * u[1] + iv[5] * u[2]};
+  const T mag = sqrt(g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
+  const T den = mag > T(1e-30) ? mag : T(1e-30);
+  const T n3[3] = {-g[0] / den, -g[1] / den, -g[2] / den};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    grad_c[3 * a + k] = g[k];
+    normal[3 * a + k] = n3[k];
+  }
+  nq[a] = Q4<T>{n3[0], n3[1], n3[2], T(0)};
+  delta_s[a] = mag;
+  valid[a] = ok ? 1 : 0;
 }
 
-// C4: kappa = trace(S M^-1), S_pq = sum_b V_b (n_b - n_a)_p grad_q W
-template <class T>
-__global__ void c_kappa(CP<T> p, const Q4<T>* __restrict__ pv, const int64_t* __restrict__ rowptr,
-                        const uint32_t* __restrict__ ent, const Q4<T>* __restrict__ nq,
-                        const T* __restrict__ minv, const uint8_t* __restrict__ valid, T* __restrict__ kappa) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < p.n; a += gridDim.x * blockDim.x) {
-    const Q4<T> pa = pv[a];
-    const Q4<T> na = nq[a];
-    CSum<T> s[9];
-    for (int64_t e = rowptr[a]; e < rowptr[a + 1]; ++e) {
-      const uint32_t b = ent[e] & kIndexMask;
-      const Q4<T> pb = pv[b];
-      const Q4<T> nb = nq[b];
-      T d[3];
-      sep(pa, pb, p, d);
-      const T g = pb.w * grad_scale<T>(p, d, nullptr);
-      const T dn[3] = {nb.x - na.x, nb.y - na.y, nb.z - na.z};
+// C4: kappa = trace(S M^-1), S_pq = sum_b V_b (n_b - n_a)_p grad_q W: the trace
+// of each neighbour's term, V_b g (n_b - n_a) . (M^-1 d), so one sum a row
+// instead of nine.
+template <class T, int L>
+__global__ void __launch_bounds__(kGatherBlock) c_kappa(CP<T> p, const Q4<T>* __restrict__ pv,
+                                                        const int64_t* __restrict__ rowptr,
+                                                        const uint32_t* __restrict__ ent,
+                                                        const Q4<T>* __restrict__ nq, const T* __restrict__ minv,
+                                                        const uint8_t* __restrict__ valid, T* __restrict__ kappa) {
+  const RowLanes<L> me;
+  const int64_t a = me.row;
+  if (a >= p.n) return;
+  const Q4<T> pa = pv[a];
+  const Q4<T> na = nq[a];
+  T iv[6];
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) s[3 * i + j].add(dn[i] * (g * d[j]));
-    }
-    const T* iv = minv + 6 * a;
-    const T full[9] = {iv[0], iv[1], iv[2], iv[1], iv[3], iv[4], iv[2], iv[4], iv[5]};
-    T k = T(0);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) k += s[i].value() * full[i];
-    kappa[a] = valid[a] ? k : T(0);
-  }
+  for (int k = 0; k < 6; ++k) iv[k] = minv[6 * a + k];
+  CSum<T> sum;
+  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+    const uint32_t b = e & kIndexMask;
+    const Q4<T> pb = pv[b];
+    const Q4<T> nb = nq[b];
+    T d[3];
+    sep(pa, pb, p, d);
+    const T g = pb.w * p.k.g2(p.k.radial(norm2(d)));
+    const T ux = iv[0] * d[0] + iv[1] * d[1] + iv[2] * d[2];
+    const T uy = iv[1] * d[0] + iv[3] * d[1] + iv[4] * d[2];
+    const T uz = iv[2] * d[0] + iv[4] * d[1] + iv[5] * d[2];
+    sum.add(g * ((nb.x - na.x) * ux + (nb.y - na.y) * uy + (nb.z - na.z) * uz));
+  });
+  const T k = me.sum(sum);
+  if (me.lane == 0) kappa[a] = valid[a] ? k : T(0);
 }
 
 // A: max delta_s (non-negative: its IEEE bits order as unsigned integers)
@@ -321,7 +324,7 @@ CLayout c_layout(int64_t n, int64_t dtype, int64_t curvature) {
   L.minv = take(n * 6 * t);
   L.det = take(n * t);
   L.keys = take(n * 8);
-  L.hist = take(256 * 4);
+  L.hist = take(kSelectHist);
   L.sel = take(2 * 8);
   L.maxbits = take(8);
   const bool axi = curvature == 1;
@@ -341,21 +344,21 @@ CP<T> make_cp(const tsph_csf3_params& prm) {
   CP<T> p{};
   p.n = prm.n;
   p.periodic = static_cast<int>(prm.periodic);
-  for (int k = 0; k < 3; ++k) p.box[k] = static_cast<T>(prm.box[k]);
+  for (int k = 0; k < 3; ++k) {
+    p.box[k] = static_cast<T>(prm.box[k]);
+    p.half[k] = T(0.5) * p.box[k];
+  }
   p.rho0 = static_cast<T>(prm.rho0);
   const double sigma3 = 1.0 / (M_PI * prm.h * prm.h * prm.h);
   p.w0 = static_cast<T>(sigma3);
   p.sigma = static_cast<T>(prm.sigma);
   p.cutoff = static_cast<T>(prm.cutoff);
-  p.k.h = static_cast<T>(prm.h);
-  p.k.inv_h = static_cast<T>(1.0 / prm.h);
-  p.k.sigma = static_cast<T>(sigma3);
-  p.k.eps = static_cast<T>(1e-12);
+  p.k = make_cubic<T>(prm.h, sigma3);
   return p;
 }
 
-template <class T>
-int run_fields(const tsph_csf3_params& prm, const tsph_csf3_io& io, char* ws, cudaStream_t s) {
+template <class T, int LN>
+int run_rows(const tsph_csf3_params& prm, const tsph_csf3_io& io, char* ws, cudaStream_t s) {
   const CLayout L = c_layout(prm.n, prm.dtype, prm.curvature);
   CP<T> p = make_cp<T>(prm);
   p.has_volume = io.volume != nullptr;
@@ -372,19 +375,17 @@ int run_fields(const tsph_csf3_params& prm, const tsph_csf3_io& io, char* ws, cu
   const unsigned g = grid_for(n, 128);
   c_pack<T><<<grid_for(n, 256), 256, 0, s>>>(p, static_cast<const T*>(io.pos), static_cast<const T*>(io.mass),
                                               static_cast<const T*>(io.volume), pv);
-  c_colour<T><<<g, 128, 0, s>>>(p, pv, io.rowptr, io.entries, color, mm, det, keys);
+  const unsigned gr = row_grid(n, LN);
+  c_colour<T, LN><<<gr, kGatherBlock, 0, s>>>(p, pv, io.rowptr, io.entries, color, mm, det, keys);
   TSPH_LAUNCH_CHECK();
   // lower median of |det M| (torch.median of an even count: the lower middle)
-  TSPH_CUDA_CHECK(cudaMemsetAsync(hist, 0, 256 * sizeof(unsigned int), s));
-  const int top = sizeof(T) == 8 ? 64 : 32;
-  const long long rank = (n - 1) / 2;
-  const unsigned gh = grid_for(n, 256, 148 * 4);
-  radix_select_u64(keys, n, top, rank, sel, hist, s, gh);
-  TSPH_LAUNCH_CHECK();
-  c_gradient<T><<<g, 128, 0, s>>>(p, pv, io.rowptr, io.entries, color, mm, det, sel, minv,
-                                  static_cast<T*>(io.grad_c), static_cast<T*>(io.normal), nq,
-                                  static_cast<T*>(io.delta_s), io.valid);
-  c_kappa<T><<<g, 128, 0, s>>>(p, pv, io.rowptr, io.entries, nq, minv, io.valid, static_cast<T*>(io.kappa));
+  int rc = radix_select_u64(keys, n, sizeof(T) == 8 ? 64 : 32, (n - 1) / 2, sel, hist, s);
+  if (rc) return rc;
+  c_gradient<T, LN><<<gr, kGatherBlock, 0, s>>>(p, pv, io.rowptr, io.entries, color, mm, det, sel, minv,
+                                                static_cast<T*>(io.grad_c), static_cast<T*>(io.normal), nq,
+                                                static_cast<T*>(io.delta_s), io.valid);
+  c_kappa<T, LN><<<gr, kGatherBlock, 0, s>>>(p, pv, io.rowptr, io.entries, nq, minv, io.valid,
+                                             static_cast<T*>(io.kappa));
   TSPH_LAUNCH_CHECK();
   if (prm.curvature == 1) {
     T* mer = reinterpret_cast<T*>(ws + L.mer);
@@ -406,6 +407,11 @@ int run_fields(const tsph_csf3_params& prm, const tsph_csf3_io& io, char* ws, cu
     TSPH_LAUNCH_CHECK();
   }
   return TSPH_OK;
+}
+
+template <class T>
+int run_fields(const tsph_csf3_params& prm, const tsph_csf3_io& io, char* ws, cudaStream_t s) {
+  return with_lanes<3>(prm.n, [&](auto lanes) { return run_rows<T, decltype(lanes)::value>(prm, io, ws, s); });
 }
 
 template <class T>

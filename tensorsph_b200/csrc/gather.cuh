@@ -40,9 +40,13 @@ struct RowLanes {
       : row((blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / L),
         lane(threadIdx.x & (L - 1)),
         group((L == 32 ? 0xffffffffu : (1u << L) - 1u) << (threadIdx.x & 31 & ~(L - 1))) {}
-  // The sum over the row's lanes, in every lane.
+  // The sum over the row's lanes, in every lane; total() with its compensation.
   template <class T>
-  __device__ __forceinline__ T sum(CSum<T> s) const;
+  __device__ __forceinline__ CSum<T> total(CSum<T> s) const;
+  template <class T>
+  __device__ __forceinline__ T sum(CSum<T> s) const {
+    return total(s).value();
+  }
   // Calls use(entry) for this lane's part of the row's entries [beg, end).
   template <class Use>
   __device__ __forceinline__ void walk(const uint32_t* __restrict__ ent, int64_t beg, int64_t end, Use&& use) const {
@@ -66,10 +70,10 @@ __device__ __forceinline__ void join<float>(CSum<float>& s, unsigned group, int 
 
 template <int L>
 template <class T>
-__device__ __forceinline__ T RowLanes<L>::sum(CSum<T> s) const {
+__device__ __forceinline__ CSum<T> RowLanes<L>::total(CSum<T> s) const {
 #pragma unroll
   for (int o = L / 2; o > 0; o >>= 1) join(s, group, o);
-  return s.value();
+  return s;
 }
 
 // Blocks for n rows of L lanes.

@@ -14,6 +14,8 @@
 
 #include <cuda_runtime.h>
 
+#include "common.cuh"
+
 namespace tsph {
 
 template <class T>
@@ -21,6 +23,7 @@ struct Cubic {
   T inv_h, h, sigma, eps;
   T inv_lo;    // 1 / h = inv_h + inv_lo (FP32; 0 in FP64)
   T sigma_h;   // sigma / h
+  T sigma_hh;  // sigma / h^2
   T sigma_lo;  // sigma to twice the precision: sigma + sigma_lo (FP32; 0 in FP64)
   // Both branches and a select: the neighbours of a warp lie on both sides.
   __device__ __forceinline__ T shape(T q) const {
@@ -50,25 +53,43 @@ struct Cubic {
   // every q of a call alike, and that common error, not the terms' own, is most
   // of a density's (measured: 4e-8 to 1.8e-7 of rho0 as 1 / h happens to round).
   // 1 / r is a reciprocal square root (2 ulp in FP32, 1 in FP64, where it gives
-  // r as well).  Below eps, where g is a division by eps, w() and wg().
+  // r as well).
   __device__ __forceinline__ T scaled(T r) const {
     return sizeof(T) == 8 ? r * inv_h : fma(r, inv_h, r * inv_lo);
   }
-  __device__ __forceinline__ T shape2(T r2) const { return shape(scaled(sqrt(r2))); }
+  __device__ __forceinline__ T shape2(T r2) const { return shape(sizeof(T) == 8 ? radial(r2).q : scaled(sqrt(r2))); }
   __device__ __forceinline__ T w2(T r2) const {
     const T s = shape2(r2);
     return sigma * (s > T(0) ? s : T(0));
   }
-  // sigma times a sum of shapes
-  __device__ __forceinline__ T times_sigma(T s) const { return sizeof(T) == 8 ? sigma * s : fma(s, sigma, s * sigma_lo); }
+  // sigma times a sum of shapes, rounded once
+  __device__ __forceinline__ T times_sigma(const CSum<double>& s) const { return sigma * s.s; }
+  __device__ __forceinline__ T times_sigma(const CSum<float>& s) const {
+    return fma(s.s, sigma, fma(s.s, sigma_lo, s.c * sigma));
+  }
+  // q = r / h and 1 / max(r, eps).  For r < eps in FP64 q is r^2 / (eps h), as
+  // good as r / h there: f is 1 to the last bit and f' too small to matter.
+  struct Radial {
+    T q, ir;
+  };
+  __device__ __forceinline__ Radial radial(T r2) const {
+    const T ir = r2 > eps * eps ? rsqrt(r2) : T(1) / eps;
+    return Radial{scaled(sizeof(T) == 8 ? r2 * ir : sqrt(r2)), ir};
+  }
+  // The gradient scale g (grad_i W = delta * g) and, with it, W.
+  __device__ __forceinline__ T g2(const Radial& R) const { return sigma_h * dshape(R.q) * R.ir; }
   __device__ __forceinline__ void wg2(T r2, T& W, T& g) const {
-    if (r2 > eps * eps) {
-      const T ir = rsqrt(r2), q = scaled(sizeof(T) == 8 ? r2 * ir : sqrt(r2)), s = shape(q);
-      W = sigma * (s > T(0) ? s : T(0));
-      g = sigma_h * dshape(q) * ir;
-    } else {
-      wg(sqrt(r2), W, g);
-    }
+    const Radial R = radial(r2);
+    const T s = shape(R.q);
+    W = sigma * (s > T(0) ? s : T(0));
+    g = g2(R);
+  }
+  // lap3 from q and 1 / r: f'' + 2 f' / q with the quotient written out (-6 + 4.5 q
+  // below q = 1, its limit at 0 included).
+  __device__ __forceinline__ T lap2(const Radial& R) const {
+    const T t = T(2) - R.q;
+    const T near = T(-9) + T(9) * R.q, far = t * (T(1.5) - T(1.5) * t * (h * R.ir));
+    return sigma_hh * (R.q < T(1) ? near : (R.q < T(2) ? far : T(0)));
   }
   // 3-D Laplacian of W (threed/kernel3.py:108-124).
   __device__ __forceinline__ T lap3(T r) const {
@@ -88,6 +109,7 @@ __host__ inline Cubic<T> make_cubic(double h, double sigma) {
   k.inv_lo = static_cast<T>(1.0 / h - static_cast<double>(k.inv_h));
   k.sigma = static_cast<T>(sigma);
   k.sigma_h = static_cast<T>(sigma / h);
+  k.sigma_hh = static_cast<T>(sigma / (h * h));
   k.sigma_lo = static_cast<T>(sigma - static_cast<double>(k.sigma));
   k.eps = static_cast<T>(1e-12);
   return k;

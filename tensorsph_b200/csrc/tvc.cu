@@ -10,16 +10,15 @@
 //   S  per fluid row:    limiter f_a = 1, min(slope h_ref^2 |g|^2, 1) or given;
 //      shift = alpha h_ref^2 f g [/ h_ratio^2] [* active] [* (|g| h_ref <= tol)],
 //      then scaled to max_shift where longer (the count of those comes back).
-// One thread per row, sums in a fixed order: deterministic, no atomics on
-// particle data.
+// One to eight lanes per row (gather.cuh), sums in a fixed order: deterministic,
+// no atomics on particle data.
 #include <cmath>
 
 #include "common.cuh"
+#include "gather.cuh"
 
 namespace tsph {
 namespace {
-
-constexpr uint32_t kIndexMask = 0x7fffffffu;
 
 template <class T>
 struct VP {
@@ -36,46 +35,61 @@ __device__ __forceinline__ T sigma_d(T h) {
   return T(1) / (T(M_PI) * h * h * h);
 }
 
-template <int D, class T>
-__global__ void v_gradient(VP<T> p, const T* __restrict__ pos, const T* __restrict__ vol,
-                           const T* __restrict__ ratio, const T* __restrict__ corr,
-                           const int64_t* __restrict__ rowptr, const uint32_t* __restrict__ ent,
-                           T* __restrict__ grad, T* __restrict__ squared) {
-  for (int64_t a = blockIdx.x * blockDim.x + threadIdx.x; a < p.n_fluid; a += gridDim.x * blockDim.x) {
-    // h_local = h / (h_ratio * h / h_ref), as the reference rescales the ratio
-    const T h = p.has_ratio ? p.h / (ratio[a] * p.h_scale) : p.h;
-    const T sig = sigma_d<D, T>(h);
-    const T ca = p.has_corr ? corr[a] : T(1);
-    T xa[D];
+template <int D, class T, int L>
+__global__ void __launch_bounds__(kGatherBlock) v_gradient(VP<T> p, const T* __restrict__ pos,
+                                                           const T* __restrict__ vol, const T* __restrict__ ratio,
+                                                           const T* __restrict__ corr,
+                                                           const int64_t* __restrict__ rowptr,
+                                                           const uint32_t* __restrict__ ent, T* __restrict__ grad,
+                                                           T* __restrict__ squared) {
+  const RowLanes<L> me;
+  const int64_t a = me.row;
+  if (a >= p.n_fluid) return;
+  // h_local = h / (h_ratio * h / h_ref), as the reference rescales the ratio
+  const T h = p.has_ratio ? p.h / (ratio[a] * p.h_scale) : p.h;
+  const T inv_h = T(1) / h, sig_h = sigma_d<D, T>(h) * inv_h;
+  const T ca = p.has_corr ? corr[a] : T(1);
+  T xa[D];
 #pragma unroll
-    for (int k = 0; k < D; ++k) xa[k] = pos[D * a + k];
-    CSum<T> s[D];
-    for (int64_t e = rowptr[a]; e < rowptr[a + 1]; ++e) {
-      const int64_t b = ent[e] & kIndexMask;
-      T d[D], r2 = T(0);
-#pragma unroll
-      for (int k = 0; k < D; ++k) {
-        d[k] = xa[k] - pos[D * b + k];
-        r2 += d[k] * d[k];
-      }
-      const T r = sqrt(r2);
-      const T q = r / h;
-      const T ds = q < T(1) ? T(-3) * q + T(2.25) * q * q : (q < T(2) ? T(-0.75) * (T(2) - q) * (T(2) - q) : T(0));
-      const T scale = sig * ds / (h * (r > p.eps ? r : p.eps));
-      const T cb = p.has_corr ? corr[b] : T(1);
-      const T w = (b < p.n_fluid ? ca + cb : p.wall_factor * ca) * vol[b];
-#pragma unroll
-      for (int k = 0; k < D; ++k) s[k].add(w * (d[k] * scale));
-    }
-    T sq = T(0);
+  for (int k = 0; k < D; ++k) xa[k] = pos[D * a + k];
+  CSum<T> s[D];
+  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+    const int64_t b = e & kIndexMask;
+    T d[D], r2 = T(0);
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-      const T g = -s[k].value();
-      grad[D * a + k] = g;
-      sq += g * g;
+      d[k] = xa[k] - pos[D * b + k];
+      r2 += d[k] * d[k];
     }
-    squared[a] = sq;
+    T q, scale;
+    if (sizeof(T) == 8) {
+      // one reciprocal square root for r, r / h and 1 / (h r)
+      const T ir = r2 > p.eps * p.eps ? rsqrt(r2) : T(1) / p.eps;
+      q = r2 * ir * inv_h;
+      scale = sig_h * ir;
+    } else {
+      const T r = sqrt(r2);
+      q = r / h;
+      scale = sig_h / (r > p.eps ? r : p.eps);
+    }
+    const T t = T(2) - q;
+    const T ds = q < T(1) ? T(-3) * q + T(2.25) * q * q : (q < T(2) ? T(-0.75) * t * t : T(0));
+    scale = scale * ds;
+    const T cb = p.has_corr ? corr[b] : T(1);
+    const T w = (b < p.n_fluid ? ca + cb : p.wall_factor * ca) * vol[b];
+#pragma unroll
+    for (int k = 0; k < D; ++k) s[k].add(w * (d[k] * scale));
+  });
+  T g[D], sq = T(0);
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    g[k] = -me.sum(s[k]);
+    sq += g[k] * g[k];
   }
+  if (me.lane) return;
+#pragma unroll
+  for (int k = 0; k < D; ++k) grad[D * a + k] = g[k];
+  squared[a] = sq;
 }
 
 template <class T>
@@ -148,21 +162,25 @@ int run_gradient(const tsph_tvc_params& prm, const tsph_tvc_io& io, cudaStream_t
   p.h_scale = static_cast<T>(prm.h_ratio_scale);
   p.wall_factor = static_cast<T>(prm.wall_factor);
   p.eps = static_cast<T>(1e-12);
-  const unsigned g = grid_for(prm.n_fluid, 128);
   const T* pos = static_cast<const T*>(io.pos);
   const T* vol = static_cast<const T*>(io.volume);
   const T* ratio = static_cast<const T*>(io.h_ratio);
   const T* corr = static_cast<const T*>(io.correction);
   T* grad = static_cast<T*>(io.gradient);
   T* sq = static_cast<T*>(io.squared);
-  if (prm.dim == 1)
-    v_gradient<1, T><<<g, 128, 0, s>>>(p, pos, vol, ratio, corr, io.rowptr, io.entries, grad, sq);
-  else if (prm.dim == 2)
-    v_gradient<2, T><<<g, 128, 0, s>>>(p, pos, vol, ratio, corr, io.rowptr, io.entries, grad, sq);
-  else
-    v_gradient<3, T><<<g, 128, 0, s>>>(p, pos, vol, ratio, corr, io.rowptr, io.entries, grad, sq);
-  TSPH_LAUNCH_CHECK();
-  return TSPH_OK;
+  auto go = [&](auto dim) {
+    constexpr int D = decltype(dim)::value;
+    return with_lanes<D>(prm.n_fluid, [&](auto lanes) -> int {
+      constexpr int LN = decltype(lanes)::value;
+      v_gradient<D, T, LN><<<row_grid(prm.n_fluid, LN), kGatherBlock, 0, s>>>(p, pos, vol, ratio, corr, io.rowptr,
+                                                                             io.entries, grad, sq);
+      TSPH_LAUNCH_CHECK();
+      return TSPH_OK;
+    });
+  };
+  if (prm.dim == 1) return go(std::integral_constant<int, 1>{});
+  if (prm.dim == 2) return go(std::integral_constant<int, 2>{});
+  return go(std::integral_constant<int, 3>{});
 }
 
 template <class T>

@@ -121,14 +121,14 @@ __global__ void __launch_bounds__(kGatherBlock) density_kernel(WP<T> p, const Q4
     s.add(pb.w * f);
     if (renorm) kt.add(f);
   });
-  T rho = p.k.times_sigma(me.sum(s));
+  T rho = p.k.times_sigma(me.total(s));
   rho = rho > p.rho_floor ? rho : p.rho_floor;
   if (p.has_offset) {
     rho = rho + offset[a];
     rho = rho > p.rho_floor ? rho : p.rho_floor;
   }
   if (renorm) {
-    T total = p.k.times_sigma(me.sum(kt)) + p.w0;
+    T total = p.k.times_sigma(me.total(kt)) + p.w0;
     total = total > T(1e-12) ? total : T(1e-12);
     rho = rho * (p.lattice_sum / total);
     rho = rho > p.rho_floor ? rho : p.rho_floor;

@@ -73,3 +73,57 @@ def test_rhs_lanes_3d(gpu, dtype, tol, n):
     close(got[1], want[1], bulk, 20 * tol)
     close(got[2], want[2], np.abs(want[2]).max(), 100 * tol)
     close(got[3], want[3], np.abs(want[3]).max(), 100 * tol)
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-11), (torch.float32, 2e-4)])
+@pytest.mark.parametrize("n", [49152, 49153])
+def test_periodic_operators(gpu, dtype, tol, n):
+    """accelerations (psi diffusion, order 4, images on every axis) and csf_fields3 on a
+    jittered block with a free face in a periodic box."""
+    from oracle import csf3 as oc
+    from oracle.neighbors import periodic_pairs
+    from tensorsph_b200.threed import accelerations
+    from tensorsph_b200.threed.csf3 import csf_fields3
+    side, dx = 37, 1.0 / 37
+    h = 1.3 * dx
+    g = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    rng = np.random.default_rng(n)
+    x = ((g + 0.1 * rng.uniform(-1, 1, g.shape)) * dx) % 1.0
+    v = rng.normal(0, 1e-3, x.shape)
+    m = np.full(n, 1000.0 * dx ** 3)
+    t = [torch.from_numpy(a).to(gpu, dtype) for a in (x, v, m)]
+    d = [a.double().cpu().numpy() for a in t]
+    pairs = periodic_pairs(d[0], [1.0] * 3, 2.0 * h)
+    kw = dict(rho0=1000.0, sound_speed=1.0, viscosity=1e-2, viscous_order=4, density_diffusion=0.1, dt=1e-4,
+              gravity=(0.0, -9.81, 0.0))
+    p = torch.from_numpy(pairs).to(gpu)
+    got = accelerations(*t, h, p, box=[1.0] * 3, **kw)
+    want = op.accelerations(*d, h, pairs, box=[1.0] * 3, **kw)
+    close(got[0], want[0], np.abs(want[0]).max(), 10 * tol)
+    close(got[1], want[1], 1000.0, tol)
+    close(got[2], want[2], 1000.0, 10 * tol)
+    got = csf_fields3(t[0], t[2], h, p, rho0=1000.0, box=[1.0] * 3)
+    want = oc.csf_fields3(d[0], d[2], h, pairs, rho0=1000.0, box=[1.0] * 3)
+    for name in ("color", "grad_c", "delta_s"):
+        close(getattr(got, name), want[name], max(np.abs(want[name]).max(), 1.0), tol)
+    if dtype == torch.float64:
+        close(got.kappa, want["kappa"], np.abs(want["kappa"]).max(), 1e-8)
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-12), (torch.float32, 2e-5)])
+@pytest.mark.parametrize("dim,n", [(1, 2000), (2, 49152), (2, 49153), (3, 49152), (3, 49153)])
+def test_tvc_lanes(gpu, dtype, tol, dim, n):
+    from oracle import tvc as ot
+    from tensorsph_b200.transport_velocity_correction import kernel_gradient_integral
+    side = int(np.ceil(n ** (1.0 / dim)))
+    g = np.stack(np.meshgrid(*[np.arange(side)] * dim, indexing="ij"), -1).reshape(-1, dim)[:n]
+    rng = np.random.default_rng(n + dim)
+    x = (g + 0.1 * rng.uniform(-1, 1, g.shape)) * 0.01
+    t = torch.from_numpy(x[rng.permutation(n)]).to(gpu, dtype)
+    x = t.double().cpu().numpy()
+    vol = np.full(n, 0.01 ** dim)
+    pairs = cell_linked_pairs_batched(x, 0.026)
+    got = kernel_gradient_integral(t, torch.from_numpy(vol).to(gpu, dtype), 0.013, wall_count=n // 10,
+                                   pairs=torch.from_numpy(pairs).to(gpu))
+    want = ot.kernel_gradient_integral(x, vol, 0.013, pairs, wall_count=n // 10)
+    close(got, want, np.abs(want).max(), tol)
