@@ -402,24 +402,68 @@ __device__ __forceinline__ uint4 ld_group(const uint32_t* nbr, int64_t rows, int
 // hardware reciprocal, within 2 ulp.
 __device__ __forceinline__ float rcp_pair(float x) { return __fdividef(1.f, x); }
 
+// The lanes that share a row in the kernels of small batches: kRowLanes
+// neighbouring lanes of a warp, of which lane 0 writes.
+constexpr int kRowLanes = 4;
+// Rows (fluid, or wall for the wall pass) up to which they do.
+constexpr int kFewRows = 49152;
+
+template <int L>
+struct Lanes {
+  int lane = 0;
+  unsigned group = 0xffffffffu;
+  __device__ __forceinline__ Lanes() {
+    if (L > 1) {
+      lane = threadIdx.x & (L - 1);
+      group = ((1u << L) - 1u) << (threadIdx.x & 31 & ~(L - 1));
+    }
+  }
+  // Adds the lanes' batch sums in batch order, in every lane: the sum is that of
+  // one thread walking the row, to the bit, so a case does not depend on whether
+  // its batch is small enough for lanes.
+  __device__ __forceinline__ void add(CSum<float>& s, float part) const {
+    if (L == 1) {
+      s.add(part);
+    } else {
+#pragma unroll
+      for (int q = 0; q < L; ++q) s.add(__shfl_sync(group, part, q, L));
+    }
+  }
+};
+
+// Rows of this thread: a row per thread, or per L lanes.
+template <int L>
+__device__ __forceinline__ int first_row() {
+  return static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) / L);
+}
+template <int L>
+__device__ __forceinline__ int row_step() {
+  return static_cast<int>(gridDim.x * blockDim.x / L);
+}
+
 // Walk row a in batches of KB entries (KB a multiple of 4: whole groups; the
 // last group is padded with null-row entries by the builder, groups past the
 // row read as null-row entries); the loads of a batch are all issued before
 // any use.  KB (the batch depth: neighbour records in flight per thread) is
-// a tuning parameter of the hot kernels.
-template <int KB = kBatch, class Body>
-__device__ __forceinline__ void walk_row(const Dev& e, int64_t a, Body&& body) {
+// a tuning parameter of the hot kernels.  L lanes take the batches in turn; all
+// of them call body equally often (a batch past the row's end is all null rows).
+template <int KB = kBatch, int L = 1, class Body>
+__device__ __forceinline__ void walk_row(const Dev& e, int64_t a, Body&& body, int lane = 0) {
   static_assert(KB % 4 == 0, "batches of whole groups");
   constexpr int G = KB / 4;
   const int groups = (e.cnt[a] + 3) >> 2;
   const uint4 padg = make_uint4(e.pad, e.pad, e.pad, e.pad);
+  const int mine = L == 1 ? 0 : lane * G;  // this lane's groups of a round
   // the entries of the next batch are loaded while the current one is used
   uint4 cur[G], nxt[G];
 #pragma unroll
-  for (int j = 0; j < G; ++j) cur[j] = j < groups ? ld_group(e.nbr, e.rows, a, j) : padg;
-  for (int g = 0; g < groups; g += G) {
+  for (int j = 0; j < G; ++j) cur[j] = mine + j < groups ? ld_group(e.nbr, e.rows, a, mine + j) : padg;
+  for (int g = 0; g < groups; g += G * L) {
 #pragma unroll
-    for (int j = 0; j < G; ++j) nxt[j] = (g + G + j < groups) ? ld_group(e.nbr, e.rows, a, g + G + j) : padg;
+    for (int j = 0; j < G; ++j) {
+      const int k = g + G * L + mine + j;
+      nxt[j] = k < groups ? ld_group(e.nbr, e.rows, a, k) : padg;
+    }
     uint32_t ent[KB];
 #pragma unroll
     for (int j = 0; j < G; ++j) {
@@ -457,23 +501,56 @@ __device__ __forceinline__ const CaseDev& case_of(const Dev& e, int64_t a) {
 
 // ------------------------------------------------------------ rebuild ---
 
-__global__ void k_check(Dev e, int shift_pass) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= e.n_slots) return;
-  CaseCtl& t = e.ctl[c];
-  if (!t.active) {
-    t.rebuild = 0;
-    return;
+// Step start of one case: clear the per-step meters, fix the step size.
+__device__ __forceinline__ void step_begin(const CaseDev& C, CaseCtl& t) {
+  t.rho_max = t.speed_max = t.front_max = 0;
+  t.ke = t.pe = 0;
+  t.force[0] = t.force[1] = t.force[2] = 0;
+  t.disp[0] = 0;
+  if (!t.active) return;
+  if (C.adaptive) {
+    // dam_break.py:379-408: step_dt = min(dt, target - elapsed); the step at
+    // which elapsed reaches the target records the final meters and is not
+    // integrated; after it the case stays frozen
+    const bool final_now = !t.finished && t.elapsed >= C.target_time - C.time_tol;
+    t.dt_step = t.finished ? 0.0 : fmin(t.dt_now, C.target_time - t.elapsed);
+    t.dt_int = (t.finished || final_now) ? 0.0 : t.dt_step;
+    if (final_now) {
+      t.finished = 1;
+      t.final_step = static_cast<int>(t.steps);
+    }
+  } else {
+    t.dt_step = t.dt_int = C.dt;
   }
-  const double d = __longlong_as_double(static_cast<long long>(t.shift_done ? t.disp[1] : t.disp[0]));
-  const int go = t.first || d > e.cases[c].skin_half;
-  t.rebuild = go;
-  if (go) {
-    t.rebuilds += 1;
-    t.first = 0;
-    atomicOr(e.any_rebuild, 1);
+}
+
+// The skin test of every case, the flag that switches the rebuild on (and its
+// conditional node in a step graph) and, in the first pass, the step start (the
+// rebuild in between reads none of what that sets): one block, one launch, for a
+// memset and three kernels of 3-4 us each in a small batch's step.
+__global__ void __launch_bounds__(1024) k_check(Dev e, int first_pass, cudaGraphConditionalHandle handle,
+                                                int conditional) {
+  int any = 0;
+  for (int c = threadIdx.x; c < e.n_slots; c += blockDim.x) {
+    CaseCtl& t = e.ctl[c];
+    int go = 0;
+    if (t.active) {
+      const double d = __longlong_as_double(static_cast<long long>(t.shift_done ? t.disp[1] : t.disp[0]));
+      go = t.first || d > e.cases[c].skin_half;
+      if (go) {
+        t.rebuilds += 1;
+        t.first = 0;
+      }
+    }
+    t.rebuild = go;
+    any |= go;
+    if (first_pass) step_begin(e.cases[c], t);
   }
-  (void)shift_pass;
+  any = __syncthreads_or(any);
+  if (threadIdx.x == 0) {
+    *e.any_rebuild = any ? 1 : 0;
+    if (conditional) cudaGraphSetConditional(handle, any ? 1u : 0u);
+  }
 }
 
 __global__ void k_keys(Dev e) {
@@ -829,38 +906,12 @@ __global__ void k_rebuilt(Dev e) {
   e.ctl[c].disp[1] = 0;
 }
 
-// Per-case step start: clear the per-step meters.
-__global__ void k_step_begin(Dev e) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= e.n_slots) return;
-  CaseCtl& t = e.ctl[c];
-  t.rho_max = t.speed_max = t.front_max = 0;
-  t.ke = t.pe = 0;
-  t.force[0] = t.force[1] = t.force[2] = 0;
-  t.disp[0] = 0;
-  if (!t.active) return;
-  const CaseDev& C = e.cases[c];
-  if (C.adaptive) {
-    // dam_break.py:379-408: step_dt = min(dt, target - elapsed); the step at
-    // which elapsed reaches the target records the final meters and is not
-    // integrated; after it the case stays frozen
-    const bool final_now = !t.finished && t.elapsed >= C.target_time - C.time_tol;
-    t.dt_step = t.finished ? 0.0 : fmin(t.dt_now, C.target_time - t.elapsed);
-    t.dt_int = (t.finished || final_now) ? 0.0 : t.dt_step;
-    if (final_now) {
-      t.finished = 1;
-      t.final_step = static_cast<int>(t.steps);
-    }
-  } else {
-    t.dt_step = t.dt_int = C.dt;
-  }
-}
-
 // ------------------------------------------------------------- physics ---
 
-template <bool kOne, int KB>
+template <bool kOne, int KB, int L>
 __global__ void __launch_bounds__(kMaxBlock) k_density(const __grid_constant__ Dev e) {
-  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < e.nf; a += gridDim.x * blockDim.x) {
+  const Lanes<L> lanes;
+  for (int a = first_row<L>(); a < e.nf; a += row_step<L>()) {
     const CaseDev& C = case_of<kOne>(e, a);
     const float sigma = C.sigma, inv_h = C.inv_h, qf = C.qf, floor_ = C.rho_floor;
     const Rec la = e.lp[a];
@@ -870,7 +921,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_density(const __grid_constant__ D
     s.add(-C.rho0);
     s.add(la.w * sigma);
     const bool renorm = C.renorm != 0, comp = C.comp != 0;
-    walk_row<KB>(e, a, [&](const uint32_t* ent) {
+    walk_row<KB, L>(e, a, [&](const uint32_t* ent) {
       float2 part = f2(0.f), wsum = f2(0.f);
 #pragma unroll
       for (int j = 0; j < KB; j += 2) {
@@ -884,10 +935,11 @@ __global__ void __launch_bounds__(kMaxBlock) k_density(const __grid_constant__ D
         part = __ffma2_rn(make_float2(l0.w, l1.w), W, part);
         if (renorm) wsum = __fadd2_rn(wsum, W);
       }
-      s.add(part.x + part.y);
-      if (renorm) kt.add(wsum.x + wsum.y);
-      if (comp) nb.add(part.x + part.y);
-    });
+      lanes.add(s, part.x + part.y);
+      if (renorm) lanes.add(kt, wsum.x + wsum.y);
+      if (comp) lanes.add(nb, part.x + part.y);
+    }, lanes.lane);
+    if (lanes.lane) continue;
     const float dfloor = floor_ - C.rho0;
     float d = s.value();
     if (comp) {
@@ -1091,9 +1143,10 @@ __global__ void __launch_bounds__(kMaxBlock) k_density_gradient(const __grid_con
   }
 }
 
-template <bool kOne, int KB>
+template <bool kOne, int KB, int L>
 __global__ void __launch_bounds__(kMaxBlock) k_diffusion_eos(const __grid_constant__ Dev e) {
-  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < e.nf; a += gridDim.x * blockDim.x) {
+  const Lanes<L> lanes;
+  for (int a = first_row<L>(); a < e.nf; a += row_step<L>()) {
     const CaseDev& C = case_of<kOne>(e, a);
     const float2 ra = e.rs[a];  // (rho - rho0, m / rho)
     const Rec la = e.lp[a];
@@ -1107,7 +1160,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_diffusion_eos(const __grid_consta
       const int NF = e.NF;
       const float2 q2 = f2(qf), inv_h2 = f2(inv_h), gscale = f2(-sigma * inv_h);
       CSum<float> rate;
-      walk_row<KB>(e, a, [&](const uint32_t* ent) {
+      walk_row<KB, L>(e, a, [&](const uint32_t* ent) {
         float2 part = f2(0.f);
 #pragma unroll
         for (int j = 0; j < KB; j += 2) {
@@ -1133,8 +1186,8 @@ __global__ void __launch_bounds__(kMaxBlock) k_diffusion_eos(const __grid_consta
           const float2 w = make_float2(-dscale * r0.y, -dscale * r1.y);
           part = __ffma2_rn(w, coupling, part);
         }
-        rate.add(part.x + part.y);
-      });
+        lanes.add(rate, part.x + part.y);
+      }, lanes.lane);
       const float dfloor = C.rho_floor - C.rho0;
       const float dtf = C.adaptive ? static_cast<float>(e.ctl[kOne ? e.one_slot : e.cid[a]].dt_step) : C.dtf;
       d = ra.x + dtf * rate.value();
@@ -1144,7 +1197,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_diffusion_eos(const __grid_consta
       const int NF = e.NF;
       const float2 q2 = f2(qf), inv_h2 = f2(inv_h), gscale = f2(-sigma * inv_h);
       CSum<float> rate;
-      walk_row<KB>(e, a, [&](const uint32_t* ent) {
+      walk_row<KB, L>(e, a, [&](const uint32_t* ent) {
         float2 part = f2(0.f);
 #pragma unroll
         for (int j = 0; j < KB; j += 2) {
@@ -1166,13 +1219,14 @@ __global__ void __launch_bounds__(kMaxBlock) k_diffusion_eos(const __grid_consta
           const float2 w = make_float2(-dscale * r0.y, -dscale * r1.y);
           part = __ffma2_rn(w, coupling, part);
         }
-        rate.add(part.x + part.y);
-      });
+        lanes.add(rate, part.x + part.y);
+      }, lanes.lane);
       const float dtf = C.adaptive ? static_cast<float>(e.ctl[kOne ? e.one_slot : e.cid[a]].dt_step) : C.dtf;
       const float dfloor = C.rho_floor - C.rho0;
       d = ra.x + dtf * rate.value();
       d = d > dfloor ? d : dfloor;
     }
+    if (lanes.lane) continue;
     e.dlt[a] = d;
     const float rho = C.rho0 + d;
     const float p = tait_dev(d, C.rho0, C.bulk, C.gamma);
@@ -1232,16 +1286,17 @@ __global__ void __launch_bounds__(kMaxBlock) k_bcd(const __grid_constant__ Dev e
   }
 }
 
-template <bool kOne, int KB>
+template <bool kOne, int KB, int L>
 __global__ void __launch_bounds__(kMaxBlock) k_walls(const __grid_constant__ Dev e) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < e.nw; t += gridDim.x * blockDim.x) {
+  const Lanes<L> lanes;
+  for (int t = first_row<L>(); t < e.nw; t += row_step<L>()) {
     const int64_t a = e.NF + t;
     const CaseDev& C = case_of<kOne>(e, a);
     const float sigma = C.sigma, inv_h = C.inv_h, qf = C.qf, grav = C.grav;
     const int f0 = C.fluid_begin;
     const Rec la = e.lp[a];
     CSum<float> num, den;
-    walk_row<KB>(e, a, [&](const uint32_t* ent) {
+    walk_row<KB, L>(e, a, [&](const uint32_t* ent) {
       float pn = 0.f, pd = 0.f;
 #pragma unroll
       for (int j = 0; j < KB; ++j) {
@@ -1256,9 +1311,10 @@ __global__ void __launch_bounds__(kMaxBlock) k_walls(const __grid_constant__ Dev
         pn += src * W;
         pd += W;
       }
-      num.add(pn);
-      den.add(pd);
-    });
+      lanes.add(num, pn);
+      lanes.add(den, pd);
+    }, lanes.lane);
+    if (lanes.lane) continue;
     const float dd = den.value();
     float p = num.value() / (dd > 1e-30f ? dd : 1e-30f);
     p = p > 0.f ? p : 0.f;
@@ -1274,9 +1330,10 @@ __global__ void __launch_bounds__(kMaxBlock) k_walls(const __grid_constant__ Dev
 // At most 80 registers (three 256-thread blocks per SM): the depth-8 and -16
 // instances then keep one more block resident without spilling (measured on
 // the 2 M case: 0.530 -> 0.505 ms at depth 8, 0.516 -> 0.508 at 16).
-template <bool kOne, int KB>
+template <bool kOne, int KB, int L>
 __global__ void __launch_bounds__(kMaxBlock, 3) k_force(const __grid_constant__ Dev e) {
-  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < e.nf; a += gridDim.x * blockDim.x) {
+  const Lanes<L> lanes;
+  for (int a = first_row<L>(); a < e.nf; a += row_step<L>()) {
     const CaseDev& C = case_of<kOne>(e, a);
     const float sigma = C.sigma, inv_h = C.inv_h, qf = C.qf, nu2 = C.nu2, nu2f = C.nu2f,
                 eta2 = C.visc_eps;
@@ -1286,7 +1343,7 @@ __global__ void __launch_bounds__(kMaxBlock, 3) k_force(const __grid_constant__ 
     const float Pa = e.pq[a];
     const float2 q2 = f2(qf), inv_h2 = f2(inv_h), gscale = f2(sigma * inv_h);
     CSum<float> ax, ay, az;
-    walk_row<KB>(e, a, [&](const uint32_t* ent) {
+    walk_row<KB, L>(e, a, [&](const uint32_t* ent) {
       float2 px = f2(0.f), py = f2(0.f), pz = f2(0.f);
 #pragma unroll
       for (int j = 0; j < KB; j += 2) {
@@ -1313,10 +1370,11 @@ __global__ void __launch_bounds__(kMaxBlock, 3) k_force(const __grid_constant__ 
         py = __ffma2_rn(fp, dy, __ffma2_rn(coef, sub2(f2(va.y), make_float2(v0.y, v1.y)), py));
         pz = __ffma2_rn(fp, dz, __ffma2_rn(coef, sub2(f2(va.z), make_float2(v0.z, v1.z)), pz));
       }
-      ax.add(px.x + px.y);
-      ay.add(py.x + py.y);
-      az.add(pz.x + pz.y);
-    });
+      lanes.add(ax, px.x + px.y);
+      lanes.add(ay, py.x + py.y);
+      lanes.add(az, pz.x + pz.y);
+    }, lanes.lane);
+    if (lanes.lane) continue;
     float sx = 0.f, sy = 0.f;
     if (C.csf) {
       const float2 st = e.st[a];
@@ -2954,21 +3012,18 @@ int enqueue_rebuild_body(tsph_engine* E, cudaStream_t s) {
   return TSPH_OK;
 }
 
-__global__ void k_set_rebuild_condition(cudaGraphConditionalHandle h, const int* any_rebuild) {
-  cudaGraphSetConditional(h, *any_rebuild ? 1u : 0u);
-}
-
 // Skin test, then the rebuild.  While a step graph is being captured
 // (`conditional`), the rebuild goes into the body of a conditional node that
 // the skin test's flag switches on, so that steps without a rebuild skip its
 // ~20 launches.
 int enqueue_rebuild(tsph_engine* E, cudaStream_t s, int pass, bool conditional) {
   Dev& d = E->d;
-  const unsigned gc = grid_for(d.n_slots, 128);
-  TSPH_CUDA_CHECK(cudaMemsetAsync(d.any_rebuild, 0, sizeof(int), s));
-  k_check<<<gc, 128, 0, s>>>(d, pass);
-  TSPH_LAUNCH_CHECK();
-  if (!conditional) return enqueue_rebuild_body(E, s);
+  const int threads = std::min(1024, (d.n_slots + 31) / 32 * 32);
+  if (!conditional) {
+    k_check<<<1, threads, 0, s>>>(d, pass == 0, cudaGraphConditionalHandle{}, 0);
+    TSPH_LAUNCH_CHECK();
+    return enqueue_rebuild_body(E, s);
+  }
   cudaStreamCaptureStatus status;
   cudaGraph_t graph = nullptr;
   const cudaGraphNode_t* deps = nullptr;
@@ -2977,7 +3032,7 @@ int enqueue_rebuild(tsph_engine* E, cudaStream_t s, int pass, bool conditional) 
   if (status != cudaStreamCaptureStatusActive) return TSPH_ERR_CUDA;
   cudaGraphConditionalHandle handle;
   TSPH_CUDA_CHECK(cudaGraphConditionalHandleCreate(&handle, graph, 0, 0));
-  k_set_rebuild_condition<<<1, 1, 0, s>>>(handle, d.any_rebuild);
+  k_check<<<1, threads, 0, s>>>(d, pass == 0, handle, 1);
   TSPH_LAUNCH_CHECK();
   TSPH_CUDA_CHECK(cudaStreamGetCaptureInfo(s, &status, nullptr, &graph, &deps, &ndeps));
   cudaGraphNodeParams params{};
@@ -3024,7 +3079,6 @@ int enqueue_step(tsph_engine* E, cudaStream_t s, cudaEvent_t* marks = nullptr, b
   int rc = enqueue_rebuild(E, s, 0, graph);
   if (rc) return rc;
   const unsigned gc = grid_for(d.n_slots, 128);
-  k_step_begin<<<gc, 128, 0, s>>>(d);
   mark();
   const int B = E->block;
   const unsigned g = grid_for(d.nf, B);
@@ -3033,11 +3087,17 @@ int enqueue_step(tsph_engine* E, cudaStream_t s, cudaEvent_t* marks = nullptr, b
 #define TSPH_PICK(K)                                                                     \
   (one ? (depth == 16 ? K<true, 16> : (depth == 8 ? K<true, 8> : K<true, 4>))            \
        : (depth == 16 ? K<false, 16> : (depth == 8 ? K<false, 8> : K<false, 4>)))
-  TSPH_PICK(k_density)<<<g, B, 0, s>>>(d);
+  const bool few = d.nf <= kFewRows, few_walls = d.nw <= kFewRows;
+  const unsigned gl = few ? grid_for(static_cast<int64_t>(d.nf) * kRowLanes, B) : g;
+#define TSPH_PICK_DEPTH(K, O, L) (depth == 16 ? K<O, 16, L> : (depth == 8 ? K<O, 8, L> : K<O, 4, L>))
+#define TSPH_PICK_ROWS(K)                                                                           \
+  (one ? (few ? TSPH_PICK_DEPTH(K, true, kRowLanes) : TSPH_PICK_DEPTH(K, true, 1))                   \
+       : (few ? TSPH_PICK_DEPTH(K, false, kRowLanes) : TSPH_PICK_DEPTH(K, false, 1)))
+  TSPH_PICK_ROWS(k_density)<<<gl, B, 0, s>>>(d);
   if (d.has_comp) k_compression_average<<<d.n_slots, 1024, 0, s>>>(d);
   if (d.has_psi) TSPH_PICK(k_density_gradient)<<<g, B, 0, s>>>(d);
   mark();
-  TSPH_PICK(k_diffusion_eos)<<<g, B, 0, s>>>(d);
+  TSPH_PICK_ROWS(k_diffusion_eos)<<<gl, B, 0, s>>>(d);
   if (d.closure_passes > 0) {
     k_closure_init<<<g, B, 0, s>>>(d);
     float* pres[2] = {d.pr, d.pbuf};
@@ -3051,11 +3111,14 @@ int enqueue_step(tsph_engine* E, cudaStream_t s, cudaEvent_t* marks = nullptr, b
   mark();
   // the wall pass (rows of ~40 fluid neighbours) is fastest at depth <= 8
   // (measured on the 2 M case: 0.033 ms at 8, 0.039 ms at 16)
-#define TSPH_PICK_WALLS(K) (one ? (depth == 4 ? K<true, 4> : K<true, 8>) : (depth == 4 ? K<false, 4> : K<false, 8>))
-  if (d.nw) TSPH_PICK_WALLS(k_walls)<<<grid_for(d.nw, B), B, 0, s>>>(d);
+#define TSPH_PICK_WALL_DEPTH(O, L) (depth == 4 ? k_walls<O, 4, L> : k_walls<O, 8, L>)
+  const unsigned gw = grid_for(static_cast<int64_t>(d.nw) * (few_walls ? kRowLanes : 1), B);
+  const auto walls = one ? (few_walls ? TSPH_PICK_WALL_DEPTH(true, kRowLanes) : TSPH_PICK_WALL_DEPTH(true, 1))
+                         : (few_walls ? TSPH_PICK_WALL_DEPTH(false, kRowLanes) : TSPH_PICK_WALL_DEPTH(false, 1));
+  if (d.nw) walls<<<gw, B, 0, s>>>(d);
   if (d.has_bcd && d.nw) {
     TSPH_PICK(k_bcd)<<<g, B, 0, s>>>(d);
-    TSPH_PICK_WALLS(k_walls)<<<grid_for(d.nw, B), B, 0, s>>>(d);
+    walls<<<gw, B, 0, s>>>(d);
   }
   if (d.has_csf) {
     const unsigned gf = static_cast<unsigned>((d.nf + B - 1) / B);
@@ -3083,9 +3146,11 @@ int enqueue_step(tsph_engine* E, cudaStream_t s, cudaEvent_t* marks = nullptr, b
     TSPH_LAUNCH_CHECK();
   }
   mark();  // walls + surface tension
-  TSPH_PICK(k_force)<<<g, B, 0, s>>>(d);
+  TSPH_PICK_ROWS(k_force)<<<gl, B, 0, s>>>(d);
 #undef TSPH_PICK
-#undef TSPH_PICK_WALLS
+#undef TSPH_PICK_DEPTH
+#undef TSPH_PICK_ROWS
+#undef TSPH_PICK_WALL_DEPTH
   mark();
   if (d.n_ob) k_reaction<<<static_cast<unsigned>((d.n_ob + B - 1) / B), B, 0, s>>>(d);
   mark();
