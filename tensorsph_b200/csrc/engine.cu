@@ -98,6 +98,7 @@ struct CaseDev {
   unsigned long long rows_lim;  // (list cutoff / q + 2)^2 rounded up: the rows' test in squared units
   int stencil_cells;       // cells each side covering the 4h fit stencil
   double sigma_st, h_d, inv_h_d, sigma2d_d, vol_scale;  // CSF: sigma, h, 1/h, 10/(7 pi h^2), 1/rho0
+  double sigma2d_h;        // sigma2d_d / h
   double stencil2;         // (4h)^2
   double fit_rc2;          // (4h + skin)^2, the fit rows' list cutoff
   int tvc_every;           // transport-velocity correction every k steps (0: off)
@@ -196,6 +197,12 @@ struct Dev {
   Rec* lpv;          // shifting: position + volume m/rho after the Euler update
   float* tmp_v;      // the volume carried through a rebuild's permutation
   float2* tmp_rp;    // the last density and pressure carried through it (read back by id)
+  // CSF: the fluid rows' x and y, volume m / rho0 and colour (after the divergence
+  // the fit weight), dense so that a warp's gathers touch half the lines that
+  // 32-byte records cost; in tmp4a, which only a rebuild uses
+  double2* csX;
+  double* csV;
+  double* csC;
   double4* csA;      // CSF: colour, M00, M01, M11
   double4* csB;      // CSF: grad c x, y, |grad c|, |det M|
   double2* csN0;     // CSF: raw normal
@@ -214,8 +221,7 @@ struct Dev {
   float* pbuf;            // closure: the other pressure buffer of its Jacobi passes
   uint8_t* known;         // closure: [2][NF] known-pressure flags of the passes
   int has_tvc, tvc_late;  // tvc_late: the correction runs after the second list pass
-  int csf_kinds;          // CSF options present in the batch: fits 1 quadratic, 2 circle,
-                          // 16 quadratic + local_range, 32 circle + local_range; 4 local_range,
+  int csf_kinds;          // CSF options present in the batch: fits 1 quadratic, 2 circle; 4 local_range,
                           // 8 wall traction (only those passes are launched)
   uint32_t* nbr4;    // CSF fit rows (fluid neighbours within 4h + skin), k-major over NF
   int32_t* cnt4;
@@ -1507,12 +1513,20 @@ __device__ __forceinline__ bool row_nearest_wall(const Dev& e, int a, double ax,
   }
   return any;
 }
+// One reciprocal square root gives r and 1 / r (the division by r and the root
+// took about 45 of a term's 60 FP64 instructions).  64 droplet cases, 0.95 M
+// rows: colour 162 -> 111 us, gradient 190 -> 144, divergence 208 -> 146, the
+// normal passes unchanged; with the dense arrays of k_csf_begin 97, 119 and 131,
+// the normal passes 123 and 127 -> 105 and 112.  L1 is then 60-70 % busy, the
+// FP64 pipe 35-55 %.  Below r = 1e-12, where the reference divides by that, q is
+// as good as r / h: W is W(0) to the last bit.
 __device__ __forceinline__ KD kernel_d(double dx, double dy, const CaseDev& C) {
-  const double r = sqrt(dx * dx + dy * dy);
-  const double q = r * C.inv_h_d;
+  const double r2 = dx * dx + dy * dy;
+  const double ir = r2 > 1e-24 ? rsqrt(r2) : 1e12;
+  const double q = r2 * ir * C.inv_h_d;
   KD k;
   k.w = C.sigma2d_d * shape_d(q);
-  k.gs = C.sigma2d_d * dshape_d(q) * C.inv_h_d / fmax(r, 1e-12);
+  k.gs = C.sigma2d_h * dshape_d(q) * ir;
   return k;
 }
 
@@ -1554,30 +1568,30 @@ __global__ void __launch_bounds__(kMaxBlock) k_csf_colour(const __grid_constant_
   for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < e.nf; a += gridDim.x * blockDim.x) {
     const CaseDev& C = e.cases[e.cid[a]];
     if (!C.csf) continue;
-    const double4 pa = ld4(e.pos, a);
-    double c = pa.w * C.vol_scale * C.sigma2d_d, m00 = 0.0, m01 = 0.0, m11 = 0.0;
+    const double2 pa = e.csX[a];
+    double c = e.csV[a] * C.sigma2d_d, m00 = 0.0, m01 = 0.0, m11 = 0.0;
     fluid_row(e, a, [&](const int* b, const bool* ok) {
       double2 pb[4];
-      double mb[4];
+      double vb[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        pb[j] = ld_xy(e.pos, b[j]);
-        mb[j] = ld_w(e.pos, b[j]);
+        pb[j] = e.csX[b[j]];
+        vb[j] = e.csV[b[j]];
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         if (!ok[j]) continue;
         const double dx = pa.x - pb[j].x, dy = pa.y - pb[j].y;
         const KD k = kernel_d(dx, dy, C);
-        const double vb = mb[j] * C.vol_scale;
-        c += vb * k.w;
-        const double g = -vb * k.gs;  // M += V_b (-d) (x) (d gs)
+        c += vb[j] * k.w;
+        const double g = -vb[j] * k.gs;  // M += V_b (-d) (x) (d gs)
         m00 += g * (dx * dx);
         m01 += g * (dx * dy);
         m11 += g * (dy * dy);
       }
     });
     c = c < 0.0 ? 0.0 : (c > 1.0 ? 1.0 : c);
+    e.csC[a] = c;
     e.csA[a] = make_double4(c, m00, m01, m11);
     e.csB[a] = make_double4(0.0, 0.0, 0.0, fabs(m00 * m11 - m01 * m01));
   }
@@ -1660,6 +1674,76 @@ __global__ void k_csf_pick(const __grid_constant__ Dev e, int shift) {
   for (int i = 0; i < 8; ++i) h[lane * 8 + i] = 0;
 }
 
+// The same select for cases of up to kSelectRows rows, all eight digits in one
+// launch: a block per case copies the case's keys into shared memory and counts
+// them there.  Most keys of a pass share their digit (|det M| is near 1 in the
+// bulk), so a warp whose lanes agree adds once.  64 cases of 7.7-20.5 k rows:
+// 47 us against 135 for the 16 launches.
+constexpr int kSelectRows = 28000;  // 8-byte keys that fit a block's 227 KB beside the bins
+
+__global__ void __launch_bounds__(1024) k_csf_select(const __grid_constant__ Dev e) {
+  extern __shared__ unsigned long long skeys[];
+  __shared__ unsigned int h[256];
+  __shared__ unsigned long long prefix;
+  __shared__ long long rank;
+  const int c = blockIdx.x;
+  CaseCtl& t = e.ctl[c];
+  const CaseDev& C = e.cases[c];
+  if (!t.active || !C.csf) return;
+  const int n = C.n_fluid, lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < n; i += blockDim.x)
+    skeys[i] = static_cast<unsigned long long>(__double_as_longlong(e.csB[C.fluid_begin + i].w));
+  if (threadIdx.x == 0) {
+    prefix = 0;
+    rank = (n - 1) / 2;
+  }
+  for (int shift = 56; shift >= 0; shift -= 8) {
+    if (threadIdx.x < 256) h[threadIdx.x] = 0;
+    __syncthreads();
+    const unsigned long long pre = prefix;
+    for (int i0 = 0; i0 < n; i0 += blockDim.x) {
+      const int i = i0 + static_cast<int>(threadIdx.x);
+      const unsigned long long key = i < n ? skeys[i] : 0;
+      const bool in = i < n && (shift == 56 || (key >> (shift + 8)) == (pre >> (shift + 8)));
+      const unsigned int digit = static_cast<unsigned int>((key >> shift) & 255u);
+      const unsigned int lanes = __ballot_sync(0xffffffffu, in);
+      if (!lanes) continue;
+      const int lead = __ffs(lanes) - 1;
+      const unsigned int d0 = __shfl_sync(0xffffffffu, digit, lead);
+      if (__any_sync(0xffffffffu, in && digit != d0)) {
+        if (in) atomicAdd(&h[digit], 1u);
+      } else if (lane == lead) {
+        atomicAdd(&h[d0], static_cast<unsigned int>(__popc(lanes)));
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      unsigned int mine[8];
+      long long local = 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        mine[i] = h[lane * 8 + i];
+        local += mine[i];
+      }
+      const long long incl = warp_inclusive_scan(local), excl = incl - local, k0 = rank;
+      const unsigned int holds = __ballot_sync(0xffffffffu, k0 >= excl && k0 < incl);
+      const int owner = holds ? __ffs(holds) - 1 : 31;
+      if (lane == owner) {
+        long long k = k0 - excl;
+        int d = lane * 8;
+        for (int i = 0; i < 8; ++i, ++d) {
+          if (k < static_cast<long long>(mine[i]) || i == 7) break;
+          k -= mine[i];
+        }
+        prefix = pre | (static_cast<unsigned long long>(d) << shift);
+        rank = k;
+      }
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) t.csf_med = __longlong_as_double(static_cast<long long>(prefix));
+}
+
 // M' = M, or the identity where |det M| <= 1e-4 median |det M| (csf_consistent.py:106-113)
 __device__ __forceinline__ void csf_matrix(const Dev& e, int c, const double4& A, double detabs, double& p,
                                            double& q, double& r) {
@@ -1688,24 +1772,24 @@ __global__ void __launch_bounds__(kMaxBlock) k_csf_grad(const __grid_constant__ 
     c = e.cid[a];
     const CaseDev& C = e.cases[c];
     if (C.csf) {
-      const double4 pa = ld4(e.pos, a);
+      const double2 pa = e.csX[a];
       const double4 A = e.csA[a];
       double gx = 0.0, gy = 0.0;
       fluid_row(e, a, [&](const int* b, const bool* ok) {
         double2 pb[4];
-        double mb[4], cb[4];
+        double vb[4], cb[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          pb[j] = ld_xy(e.pos, b[j]);
-          mb[j] = ld_w(e.pos, b[j]);
-          cb[j] = e.csA[b[j]].x;
+          pb[j] = e.csX[b[j]];
+          vb[j] = e.csV[b[j]];
+          cb[j] = e.csC[b[j]];
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           if (!ok[j]) continue;
           const double dx = pa.x - pb[j].x, dy = pa.y - pb[j].y;
           const KD k = kernel_d(dx, dy, C);
-          const double w = mb[j] * C.vol_scale * (cb[j] - A.x) * k.gs;
+          const double w = vb[j] * (cb[j] - A.x) * k.gs;
           gx += w * dx;
           gy += w * dy;
         }
@@ -1771,17 +1855,17 @@ __global__ void __launch_bounds__(kMaxBlock) k_csf_range(const __grid_constant__
     c = e.cid[a];
     const CaseDev& C = e.cases[c];
     if (C.csf && C.csf_range) {
-      const double ca = e.csA[a].x;
+      const double ca = e.csC[a];
       double hi = ca, lo = ca;
       if (C.csf_fit) {
-        const double4 pa = ld4(e.pos, a);
+        const double2 pa = e.csX[a];
         const int n4 = e.cnt4[a];
         for (int k = 0; k < n4; ++k) {
           const int b = static_cast<int>(e.nbr4[static_cast<int64_t>(k) * e.NF + a]);
-          const double2 pb = ld_xy(e.pos, b);
+          const double2 pb = e.csX[b];
           const double dx = pa.x - pb.x, dy = pa.y - pb.y;
           if (!(dx * dx + dy * dy <= C.stencil2)) continue;
-          const double cv = e.csA[b].x;
+          const double cv = e.csC[b];
           hi = cv > hi ? cv : hi;
           lo = cv < lo ? cv : lo;
         }
@@ -1790,7 +1874,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_csf_range(const __grid_constant__
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             if (!ok[j]) continue;
-            const double cv = e.csA[b[j]].x;
+            const double cv = e.csC[b[j]];
             hi = cv > hi ? cv : hi;
             lo = cv < lo ? cv : lo;
           }
@@ -1816,21 +1900,21 @@ __global__ void __launch_bounds__(kMaxBlock) k_csf_smooth(const __grid_constant_
   for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < e.nf; a += gridDim.x * blockDim.x) {
     const CaseDev& C = e.cases[e.cid[a]];
     if (!C.csf) continue;
-    const double4 pa = ld4(e.pos, a);
-    double nx = 0.0, ny = 0.0, den = pa.w * C.vol_scale * C.sigma2d_d;
+    const double2 pa = e.csX[a];
+    double nx = 0.0, ny = 0.0, den = e.csV[a] * C.sigma2d_d;
     fluid_row(e, a, [&](const int* b, const bool* ok) {
       double2 pb[4], nb[4];
-      double mb[4];
+      double vb[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        pb[j] = ld_xy(e.pos, b[j]);
-        mb[j] = ld_w(e.pos, b[j]);
+        pb[j] = e.csX[b[j]];
+        vb[j] = e.csV[b[j]];
         nb[j] = src[b[j]];
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         if (!ok[j]) continue;
-        const double w = mb[j] * C.vol_scale * kernel_d(pa.x - pb[j].x, pa.y - pb[j].y, C).w;
+        const double w = vb[j] * kernel_d(pa.x - pb[j].x, pa.y - pb[j].y, C).w;
         nx += w * nb[j].x;
         ny += w * nb[j].y;
         den += w;
@@ -1857,23 +1941,23 @@ __global__ void __launch_bounds__(kMaxBlock) k_csf_div(const __grid_constant__ D
     const int c = e.cid[a];
     const CaseDev& C = e.cases[c];
     if (!C.csf) continue;
-    const double4 pa = ld4(e.pos, a);
+    const double2 pa = e.csX[a];
     const double2 na = e.csN[a];
     double s00 = 0.0, s01 = 0.0, s10 = 0.0, s11 = 0.0;
     fluid_row(e, a, [&](const int* b, const bool* ok) {
       double2 pb[4], nb[4];
-      double mb[4];
+      double vb[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        pb[j] = ld_xy(e.pos, b[j]);
-        mb[j] = ld_w(e.pos, b[j]);
+        pb[j] = e.csX[b[j]];
+        vb[j] = e.csV[b[j]];
         nb[j] = e.csN[b[j]];
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         if (!ok[j]) continue;
         const double dx = pa.x - pb[j].x, dy = pa.y - pb[j].y;
-        const double gs = mb[j] * C.vol_scale * kernel_d(dx, dy, C).gs;
+        const double gs = vb[j] * kernel_d(dx, dy, C).gs;
         const double g0 = gs * dx, g1 = gs * dy;
         const double dn0 = nb[j].x - na.x, dn1 = nb[j].y - na.y;
         s00 += dn0 * g0;
@@ -1889,16 +1973,25 @@ __global__ void __launch_bounds__(kMaxBlock) k_csf_div(const __grid_constant__ D
     double4 K = e.csK[a];
     K.x = (s00 * r - s01 * q - s10 * q + s11 * p) / det;
     e.csK[a] = K;
+    if (C.csf_fit) {
+      // the fit weight delta_s / max delta_s (legacy: |grad c| / max |grad c|)
+      const CaseCtl& t = e.ctl[c];
+      const double top = __longlong_as_double(static_cast<long long>(C.csf_range ? t.csf_dmax : t.csf_gmax));
+      const double w = (C.csf_range ? e.csD[a] : e.csB[a].z) * (1.0 / fmax(top, 1e-30));
+      e.csC[a] = w < 0.0 ? 0.0 : (w > 1.0 ? 1.0 : w);
+    }
   }
 }
 
 // Q7: weighted fit v = c + b u + a u^2 in the frame (t, n) of row a over the
 // fluid particles within 4h (cells within stencil_cells of the home cell),
 // weights w_b = |grad c|_b / max |grad c| (= delta_s / max delta_s).
-// kFit: 1 the quadratic fit, 2 the circle fit; kRange: local_range weights.
-// Each instance serves the cases of its kind (separate instances keep the
-// default one's registers).
-template <int kFit, bool kRange>
+// kFit: 1 the quadratic fit, 2 the circle fit.  Each instance serves the cases
+// of its kind (separate instances keep the default one's registers).  Bound by
+// the loads' passes through L1: 64 droplet cases, 0.95 M rows, 301 us gathering
+// 32-byte position and gradient records with the weight scaled and clipped per
+// term, 273 with one record of position and weight, 228 from dense arrays.
+template <int kFit>
 __global__ void __launch_bounds__(kMaxBlock) k_csf_fit(const __grid_constant__ Dev e) {
   __shared__ double red[kMaxBlock / 32];
   const int a0 = blockIdx.x * blockDim.x;
@@ -1911,14 +2004,9 @@ __global__ void __launch_bounds__(kMaxBlock) k_csf_fit(const __grid_constant__ D
   if (a < e.nf) {
     c = e.cid[a];
     const CaseDev& C = e.cases[c];
-    if (C.csf && C.csf_fit == kFit && (C.csf_range != 0) == kRange) {
-      // the fit weights: delta_s_b / max delta_s (legacy: |grad c| / max |grad c|)
-      constexpr bool rng = kRange;
-      const double gmax = fmax(__longlong_as_double(static_cast<long long>(rng ? e.ctl[c].csf_dmax : e.ctl[c].csf_gmax)),
-                               1e-30);
-      const double inv_g = 1.0 / gmax;
+    if (C.csf && C.csf_fit == kFit) {
       const double st2 = C.stencil2;
-      const double4 pa = ld4(e.pos, a);
+      const double2 pa = e.csX[a];
       const double2 na = e.csN[a];
       const double tx = -na.y, ty = na.x;
       double s0 = 0, s1 = 0, s2 = 0, s3 = 0, s4 = 0, s5 = 0, s6 = 0, s7 = 0, s8 = 0;
@@ -1935,19 +2023,17 @@ __global__ void __launch_bounds__(kMaxBlock) k_csf_fit(const __grid_constant__ D
           nb4[j] = k + 4 + j < n4 ? static_cast<int>(e.nbr4[static_cast<int64_t>(k + 4 + j) * e.NF + a]) : a;
         }
         double2 pb[4];
-        double mg[4];
+        double wb[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          pb[j] = ld_xy(e.pos, b[j]);
-          mg[j] = rng ? e.csD[b[j]] : e.csB[b[j]].z;
+          pb[j] = e.csX[b[j]];
+          wb[j] = e.csC[b[j]];
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const double ddx = pa.x - pb[j].x, ddy = pa.y - pb[j].y;
           // padding (b == a) and points beyond the 4h stencil get no weight
-          double w = mg[j] * inv_g;
-          w = w < 0.0 ? 0.0 : (w > 1.0 ? 1.0 : w);
-          w = (k + j < n4 && ddx * ddx + ddy * ddy <= st2) ? w : 0.0;
+          const double w = (k + j < n4 && ddx * ddx + ddy * ddy <= st2) ? wb[j] : 0.0;
           if (kFit == 2) {
             // circle moments of the offset (x, y) = x_b - x_a, f = x^2 + y^2
             const double x = -ddx, y = -ddy, f = x * x + y * y;
@@ -1974,8 +2060,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_csf_fit(const __grid_constant__ D
           s7 += w * (uu * uu);
         }
       }
-      double wa = (rng ? e.csD[a] : e.csB[a].z) * inv_g;
-      wa = wa < 0.0 ? 0.0 : (wa > 1.0 ? 1.0 : wa);
+      const double wa = e.csC[a];
       s0 += wa;
       if (kFit == 2) {
         // Pratt: x^2 + y^2 + D x + E y + F = 0, [[s3 s4 s1] [s4 s5 s2] [s1 s2 s0]]
@@ -2094,12 +2179,21 @@ __global__ void k_csf_final(const __grid_constant__ Dev e) {
   }
 }
 
-__global__ void k_csf_clear(Dev e) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= e.n_slots) return;
-  e.ctl[c].csf_gmax = 0;
-  e.ctl[c].csf_fmax = 0;
-  e.ctl[c].csf_dmax = 0;
+// The CSF passes' start: the cases' maxima to zero, the fluid rows' dense arrays.
+__global__ void k_csf_begin(const __grid_constant__ Dev e) {
+  const int i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  for (int c = i0; c < e.n_slots; c += step) {
+    e.ctl[c].csf_gmax = 0;
+    e.ctl[c].csf_fmax = 0;
+    e.ctl[c].csf_dmax = 0;
+  }
+  for (int a = i0; a < e.nf; a += step) {
+    const CaseDev& C = e.cases[e.cid[a]];
+    if (!C.csf) continue;
+    const double4 p = ld4(e.pos, a);
+    e.csX[a] = make_double2(p.x, p.y);
+    e.csV[a] = p.w * C.vol_scale;
+  }
 }
 
 // Semi-implicit Euler, box and obstacle clamps, per-case meters (of the state
@@ -2833,6 +2927,7 @@ struct tsph_engine {
   int64_t instantiations = 0;  // step graphs instantiated
   int64_t updates = 0;         // batch changes absorbed by cudaGraphExecUpdate
   int sms = 148;               // multiprocessors of the device (grid-stride launch caps)
+  int select_rows = 0;          // largest case k_csf_select takes (0: the device refused its shared memory)
   int integrate_per_sm[3] = {1, 1, 1};  // resident k_integrate<true> blocks of 64, 128, 256 threads
 };
 
@@ -2899,6 +2994,9 @@ size_t carve(const tsph_engine_params& p, Dev* d, char* base, CaseDev** cases, c
   t.vals = static_cast<int32_t*>(take(nsort * sizeof(int32_t)));
   t.vals_tmp = static_cast<int32_t*>(take(nsort * sizeof(int32_t)));
   t.tmp4a = static_cast<double4*>(take(nsort * sizeof(double4)));
+  t.csX = reinterpret_cast<double2*>(t.tmp4a);
+  t.csV = reinterpret_cast<double*>(t.csX + NF);
+  t.csC = t.csV + NF;
   t.tmp4b = static_cast<double4*>(take(nsort * sizeof(double4)));
   t.tmp_id = static_cast<int32_t*>(take(nsort * sizeof(int32_t)));
   t.tmp_v = static_cast<float*>(take(nsort * sizeof(float)));
@@ -2976,7 +3074,7 @@ void batch_changed(tsph_engine* E) {
     d.has_comp |= c.dev.comp;
     if (c.dev.closure) d.closure_passes = std::max(d.closure_passes, c.dev.closure_passes);
     if (c.dev.csf)
-      d.csf_kinds |= (c.dev.csf_fit ? (c.dev.csf_fit == 1 ? 1 : 2) << (c.dev.csf_range ? 4 : 0) : 0) |
+      d.csf_kinds |= (c.dev.csf_fit ? (c.dev.csf_fit == 1 ? 1 : 2) : 0) |
                      (c.dev.csf_range ? 4 : 0) | (c.dev.csf_contact >= 2 ? 8 : 0);
     d.has_tvc |= c.dev.tvc_every > 0 ? 1 : 0;
   }
@@ -3122,23 +3220,27 @@ int enqueue_step(tsph_engine* E, cudaStream_t s, cudaEvent_t* marks = nullptr, b
   }
   if (d.has_csf) {
     const unsigned gf = static_cast<unsigned>((d.nf + B - 1) / B);
-    k_csf_clear<<<gc, 128, 0, s>>>(d);
+    k_csf_begin<<<g, B, 0, s>>>(d);
     k_csf_colour<<<g, B, 0, s>>>(d);
     const unsigned gh = static_cast<unsigned>((d.nf + 255) / 256);
     const unsigned gp = static_cast<unsigned>((d.n_slots + 3) / 4);
-    for (int shift = 56; shift >= 0; shift -= 8) {
-      k_csf_hist<<<gh, 256, 0, s>>>(d, shift);
-      k_csf_pick<<<gp, 128, 0, s>>>(d, shift);
+    int most = 0;
+    for (const CaseHost& c : E->order) most = std::max(most, c.dev.n_fluid);
+    if (most <= E->select_rows) {
+      k_csf_select<<<d.n_slots, 1024, static_cast<size_t>(most) * sizeof(unsigned long long), s>>>(d);
+    } else {
+      for (int shift = 56; shift >= 0; shift -= 8) {
+        k_csf_hist<<<gh, 256, 0, s>>>(d, shift);
+        k_csf_pick<<<gp, 128, 0, s>>>(d, shift);
+      }
     }
     k_csf_grad<<<gf, B, 0, s>>>(d);
     if (d.csf_kinds & 4) k_csf_range<<<gf, B, 0, s>>>(d);
     k_csf_smooth<false><<<g, B, 0, s>>>(d);
     k_csf_smooth<true><<<g, B, 0, s>>>(d);
     k_csf_div<<<g, B, 0, s>>>(d);
-    if (d.csf_kinds & 1) k_csf_fit<1, false><<<gf, B, 0, s>>>(d);
-    if (d.csf_kinds & 16) k_csf_fit<1, true><<<gf, B, 0, s>>>(d);
-    if (d.csf_kinds & 2) k_csf_fit<2, false><<<gf, B, 0, s>>>(d);
-    if (d.csf_kinds & 32) k_csf_fit<2, true><<<gf, B, 0, s>>>(d);
+    if (d.csf_kinds & 1) k_csf_fit<1><<<gf, B, 0, s>>>(d);
+    if (d.csf_kinds & 2) k_csf_fit<2><<<gf, B, 0, s>>>(d);
     if (d.csf_kinds & 8)
       k_csf_final<true><<<g, B, 0, s>>>(d);
     else
@@ -3320,6 +3422,7 @@ CaseDev make_case_dev(const tsph_case_params& p, int64_t* ncells) {
   c.h_d = p.h;
   c.inv_h_d = 1.0 / p.h;
   c.sigma2d_d = 10.0 / (7.0 * M_PI * p.h * p.h);
+  c.sigma2d_h = c.sigma2d_d / p.h;
   c.vol_scale = 1.0 / p.rho0;
   c.stencil_cells = static_cast<int>(std::ceil((4.0 * p.h + p.skin) / cell));
   c.stencil2 = 16.0 * p.h * p.h;
@@ -3473,6 +3576,11 @@ int tsph_engine_create(const tsph_engine_params* prm, void* arena, int64_t arena
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_integrate<true>, blocks[k], 0) == cudaSuccess && n > 0)
         E->integrate_per_sm[k] = n;
     }
+    if (cudaFuncSetAttribute(k_csf_select, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kSelectRows * static_cast<int>(sizeof(unsigned long long))) == cudaSuccess)
+      E->select_rows = kSelectRows;
+    else
+      cudaGetLastError();
   }
   carve(*prm, &E->d, E->arena, &E->cases_dev, &E->radix_scratch);
   Dev& d = E->d;

@@ -138,3 +138,26 @@ def test_engine_csf_contact_angle_matches_oracle(model, theta, gpu):
         ulp = float(np.spacing(np.float32(np.abs(got / cfg.dt).max())))
         terr = np.abs(t_dev - t_ref).max()
         assert terr <= 4 * ulp + 1e-5 * np.abs(t_ref).max(), (terr, ulp, np.abs(t_ref).max())
+
+
+@pytest.mark.parametrize("neighbour_dx", [0.0005, 0.00025, 0.0002])
+def test_csf_median_select_routes_agree(neighbour_dx, gpu):
+    """A case's median |det M| comes from one launch when every case of the
+    batch has at most 28,000 rows, else from a launch per digit: the same drop
+    beside a drop of 7.7 k, 30.5 k or 48 k rows, and alone, bit for bit."""
+    from dataclasses import replace
+
+    from tensorsph_b200.engine import BatchEngine, capacity_for, droplet_impact_case
+    spec = droplet_impact_case(drop_config(0.0728))
+    big = droplet_impact_case(replace(drop_config(0.0728), dx=neighbour_dx, dt=0.25 * 1.3 * neighbour_dx / 20.0))
+    assert (big.x.shape[0] > 28000) == (neighbour_dx < 0.0005)
+    got = []
+    for specs in ([spec], [spec, big], [big, spec]):
+        eng = BatchEngine(**capacity_for(specs, max_neighbors=64, diag_ring=8))
+        ids = {id(s): eng.add(s) for s in specs}
+        eng.step(4)
+        got.append([t.cpu() for t in eng.read(ids[id(spec)])])
+        eng.close()
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert torch.equal(a, b)
