@@ -55,6 +55,30 @@ struct RowLanes {
 #pragma unroll 2
     for (int k = lane; k < len; k += L) use(row_ent[k]);
   }
+  // The same with the next two entries on their way while two are used, for the
+  // passes that wait on their gathers: a term's chain is one load instead of two
+  // (FP64, 3-D, us a launch: 480 k rows, colour 219 -> 188, gradient 231 -> 194,
+  // kappa 241 -> 219; 262 k rows, density 102 -> 83, moments 143 -> 117, diffusion
+  // 179 -> 156; FP32 densities 54 -> 50 and 56 -> 51).  The passes bound by issue or
+  // by registers lose by it (FP64 3-D force 193 -> 210, FP32 diffusion 79 -> 85).
+  // Loading the records as well a step ahead was no faster (202, 195, 210).
+  template <class Use>
+  __device__ __forceinline__ void walk_ahead(const uint32_t* __restrict__ ent, int64_t beg, int64_t end,
+                                             Use&& use) const {
+    const uint32_t* __restrict__ row_ent = ent + beg;
+    const int len = static_cast<int>(end - beg);
+    int k = lane;
+    if (k >= len) return;
+    uint32_t e0 = row_ent[k], e1 = row_ent[min(k + L, len - 1)];
+    for (; k + L < len; k += 2 * L) {
+      const uint32_t n0 = row_ent[min(k + 2 * L, len - 1)], n1 = row_ent[min(k + 3 * L, len - 1)];
+      use(e0);
+      use(e1);
+      e0 = n0;
+      e1 = n1;
+    }
+    if (k < len) use(e0);
+  }
 };
 
 template <class T>

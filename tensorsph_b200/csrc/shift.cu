@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(kGatherBlock) s_gradient(int64_t n, Cubic<T> k
   const Q4<T> pa = pv[a];
   const T ca = c[a];
   CSum<T> g[3];
-  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+  me.walk_ahead(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
     const uint32_t b = e & kIndexMask;
     const Q4<T> pb = pv[b];
     const T d[3] = {pa.x - pb.x, pa.y - pb.y, pa.z - pb.z};

@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(kGatherBlock) t_density(TP<T> p, const Q4<T>* 
   if (a >= p.n) return;
   const Q4<T> pa = pm[a];
   CSum<T> s;
-  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+  me.walk_ahead(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
     const Q4<T> pb = pm[e & kIndexMask];
     T d[3];
     sep(pa, pb, p, d);
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kGatherBlock) t_gradient(TP<T> p, const Q4<T>*
   const Q4<T> pa = pm[a];
   const T ra = rv[a].x;
   CSum<T> G[3], M[6];
-  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+  me.walk_ahead(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
     const uint32_t b = e & kIndexMask;
     if (b >= p.nf) return;
     const Q4<T> pb = pm[b];
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kGatherBlock) t_diffusion(TP<T> p, const Q4<T>
   if (a < p.nf) {
     const Q4<T> pa = pm[a];
     const Q4<T> ga = p.form == 1 ? grad[a] : Q4<T>{T(0), T(0), T(0), T(0)};
-    me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+    me.walk_ahead(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
       const uint32_t b = e & kIndexMask;
       if (b >= p.nf) return;
       const Q4<T> pb = pm[b];
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kGatherBlock) t_walls(TP<T> p, const Q4<T>* __
   if (a >= p.n) return;
   const Q4<T> pa = pm[a];
   CSum<T> num, den;
-  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+  me.walk_ahead(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
     const uint32_t f = e & kIndexMask;
     if (f >= p.nf) return;
     const Q4<T> pb = pm[f];
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kGatherBlock) t_moments(TP<T> p, const Q4<T>* 
   const Q4<T> pa = pm[a];
   const T ra = st[a].x;
   CSum<T> k2, k4;
-  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+  me.walk_ahead(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
     const uint32_t b = e & kIndexMask;
     const Q4<T> pb = pm[b];
     T d[3];

@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kGatherBlock) v_gradient(VP<T> p, const T* __r
 #pragma unroll
   for (int k = 0; k < D; ++k) xa[k] = pos[D * a + k];
   CSum<T> s[D];
-  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+  me.walk_ahead(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
     const int64_t b = e & kIndexMask;
     T d[D], r2 = T(0);
 #pragma unroll

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kGatherBlock) density_kernel(WP<T> p, const Q4
   CSum<T> s, kt;
   if (me.lane == 0) s.add(pa.w);  // W(0) = sigma
   const bool renorm = p.flags & TSPH_RHS_RENORMALIZE;
-  me.walk(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
+  me.walk_ahead(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
     const Q4<T> pb = pm[e & kIndexMask];
     T d[3];
     separation<T, D>(pa, pb, p, d);
