@@ -132,7 +132,10 @@ int tsph_max_displacement(const void* pos, const void* anchor, int64_t n, int64_
 /* Every pair (i, j) puts j in row i and i in row j; entry = neighbour index */
 /* | (1u << 31 when the row is the pair's second element).  Rows are sorted. */
 /* ------------------------------------------------------------------------ */
+/* A workspace larger than tsph_csr_workspace_bytes by up to                  */
+/* tsph_csr_slot_bytes saves a pass over a sorted list.                       */
 int64_t tsph_csr_workspace_bytes(int64_t npairs, int64_t nrows);
+int64_t tsph_csr_slot_bytes(int64_t npairs, int64_t nrows);
 int tsph_csr_from_pairs(const int64_t* pairs, int64_t npairs, int64_t nrows, int64_t* rowptr,
                         uint32_t* entries, void* ws, int64_t ws_bytes, tsph_stream stream);
 

@@ -203,6 +203,7 @@ _SIGNATURES = {
     "tsph_max_displacement": (c_int, [c_void_p, c_void_p, c_int64, c_int64, c_int64, c_void_p,
                                       c_void_p, c_void_p]),
     "tsph_csr_workspace_bytes": (c_int64, [c_int64, c_int64]),
+    "tsph_csr_slot_bytes": (c_int64, [c_int64, c_int64]),
     "tsph_csr_from_pairs": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p,
                                     c_int64, c_void_p]),
     "tsph_wcsph_workspace_bytes": (c_int64, [POINTER(WcsphParams)]),

@@ -13,20 +13,27 @@
 //
 //   sorted list (what the searches of this library return, and the
 //   reference's): the pairs of row i are one run of the list, already in
-//   order, so only the second halves need counting, scattering and sorting:
-//     A  list_degrees  run boundaries, one atomic per pair that also hands out
-//                      the pair's slot in row j (kept in 16 bits)
+//   order, so only the second halves need counting, collecting and sorting:
+//     A  list_place  run boundaries; one atomic per pair counts row j's second
+//                    halves and hands out a place among the row's slots, where
+//                    i goes at once
 //     scan of the degrees
-//     B  list_fill     the first half copied in place (coalesced), the second
-//                      scattered to its slots
-//     C  rows_sort     the second halves only
+//     B  rows_sort   the second halves from the slots to their place, sorted;
+//                    the same warp copies the rows' runs (coalesced)
+//     A row with more second halves than slots is filled by another pass over
+//     the list (list_rest) and sorted where it lies.
 //   any other list: two atomics per pair to count, two to fill, rows sorted whole.
 //
-// What bounds the first route: the L2 atomics of A (one per pair), the
-// scattered 4-byte stores of B, instruction issue in C.  18.6 M pairs of a
-// periodic column (480 k rows): A 0.13, scan 0.01, B 0.15, C 0.11 ms, against
-// 0.22 + 0.01 + 0.36 + 0.60 ms by the second route with a rank sort of whole
-// rows; 10.6 M pairs of a 2-D column (1.04 M rows): 0.26 against 0.53 ms.
+// What bounds the first route: the L2 atomics of A (one per pair) with the
+// scattered 4-byte stores behind them, instruction issue and the copies' loads
+// in B.  18.6 M pairs of a periodic column (480 k rows): A 0.18, scan 0.01,
+// B 0.14 ms; counting first (0.13), filling by another pass over the list (0.15)
+// and sorting (0.11) took 0.41, the second route with a rank sort of whole rows
+// 1.2 ms.  13.1 M pairs of a block in mixed order 0.31 against 0.45, 10.6 M of a
+// 2-D column (1.04 M rows) 0.24 against 0.26.  The copies in a launch of their own
+// (0.09) or 32 pairs at a time (0.07 more than 128) lose to B's.
+#include <algorithm>
+
 #include "common.cuh"
 #include "rowsort.cuh"
 
@@ -37,7 +44,7 @@ constexpr uint32_t kSecond = 0x80000000u;
 constexpr int kBlock = 256;
 // One pair per thread: the loads of a warp are one contiguous 512-byte run.
 
-enum { kBad = 1, kUnsorted = 2, kLongRow = 4 };
+enum { kBad = 1, kUnsorted = 2, kOver = 4 };  // kOver: a row has more second halves than slots
 
 // kWide: the list starts on a 16-byte boundary (one load per pair).
 template <bool kWide>
@@ -51,10 +58,11 @@ __device__ __forceinline__ longlong2 ld_pair(const int64_t* __restrict__ pairs, 
 // goes through the L1, so a block may still miss the flag; it is no more than a
 // short cut, and the host reads the flag after the kernel.
 template <bool kWide>
-__global__ void __launch_bounds__(kBlock) list_degrees(const int64_t* __restrict__ pairs, int64_t npairs,
-                                                       int64_t nrows, int2* __restrict__ run,
-                                                       unsigned int* __restrict__ second,
-                                                       uint16_t* __restrict__ slot, unsigned int* found) {
+__global__ void __launch_bounds__(kBlock) list_place(const int64_t* __restrict__ pairs, int64_t npairs,
+                                                     int64_t nrows, int2* __restrict__ run,
+                                                     unsigned int* __restrict__ second,
+                                                     uint32_t* __restrict__ slots, unsigned int per_row,
+                                                     unsigned int* found) {
   if (*found & kUnsorted) return;
   const int64_t p = static_cast<int64_t>(blockIdx.x) * kBlock + threadIdx.x;
   if (p >= npairs) return;
@@ -75,8 +83,10 @@ __global__ void __launch_bounds__(kBlock) list_degrees(const int64_t* __restrict
   }
   if (p == npairs - 1) run[i].y = static_cast<int>(npairs);
   const unsigned int s = atomicAdd(&second[j], 1u);
-  if (s > 0xffffu) atomicOr(found, kLongRow);
-  slot[p] = static_cast<uint16_t>(s);
+  if (s < per_row)
+    slots[j * per_row + s] = static_cast<uint32_t>(i) | kSecond;
+  else if (s == per_row)
+    atomicOr(found, kOver);
 }
 
 __global__ void list_rows(const int2* __restrict__ run, const unsigned int* __restrict__ second, int64_t nrows,
@@ -85,29 +95,64 @@ __global__ void list_rows(const int2* __restrict__ run, const unsigned int* __re
   if (r < nrows) deg[r] = run[r].y - run[r].x + static_cast<int32_t>(second[r]);
 }
 
-// B
+// The second halves of the rows without enough slots, in any order to where they belong.
 template <bool kWide>
-__global__ void __launch_bounds__(kBlock) list_fill(const int64_t* __restrict__ pairs, int64_t npairs,
+__global__ void __launch_bounds__(kBlock) list_rest(const int64_t* __restrict__ pairs, int64_t npairs,
                                                     const int2* __restrict__ run, const int64_t* __restrict__ rowptr,
-                                                    const uint16_t* __restrict__ slot,
+                                                    const unsigned int* __restrict__ second, unsigned int per_row,
+                                                    unsigned int* __restrict__ placed,
                                                     uint32_t* __restrict__ entries) {
   const int64_t p = static_cast<int64_t>(blockIdx.x) * kBlock + threadIdx.x;
   if (p >= npairs) return;
   const longlong2 me = ld_pair<kWide>(pairs, p);
-  entries[rowptr[me.x] + (p - run[me.x].x)] = static_cast<uint32_t>(me.y);
+  if (second[me.y] <= per_row) return;
   const int2 rj = run[me.y];
-  entries[rowptr[me.y] + (rj.y - rj.x) + slot[p]] = static_cast<uint32_t>(me.x) | kSecond;
+  entries[rowptr[me.y] + (rj.y - rj.x) + atomicAdd(&placed[me.y], 1u)] = static_cast<uint32_t>(me.x) | kSecond;
 }
 
 // The second-element halves of the rows.
+template <bool kWide>
 struct SecondHalves {
   uint32_t* entries;
   const int64_t* rowptr;
   const int2* run;
+  const unsigned int* second;
+  uint32_t* slots;
+  unsigned int per_row;
+  const int64_t* pairs;
   __device__ __forceinline__ int64_t dst(int64_t r) const { return rowptr[r] + (run[r].y - run[r].x); }
-  __device__ __forceinline__ uint32_t* src(int64_t r) const { return entries + dst(r); }
-  __device__ __forceinline__ int64_t len(int64_t r) const { return rowptr[r + 1] - dst(r); }
+  __device__ __forceinline__ uint32_t* src(int64_t r) const {
+    return second[r] <= per_row ? slots + r * per_row : entries + dst(r);
+  }
+  __device__ __forceinline__ int64_t len(int64_t r) const { return second[r]; }
 };
+
+// The first halves: the runs of rows r0 .. r0 + 7 are one stretch of the list.
+template <bool kWide>
+__device__ __forceinline__ void beside_rows(const SecondHalves<kWide>& rows, int64_t r0, int64_t n) {
+  const int lane = threadIdx.x & 31;
+  const int64_t r = r0 + (lane & 7);
+  const int2 q = r < n ? rows.run[r] : make_int2(0, 0);
+  const long long shift = r < n ? rows.rowptr[r] - q.x : 0;
+  int first = q.y > q.x ? q.x : 0x7fffffff, last = q.y > q.x ? q.y : 0;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
+    last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
+  }
+  // (eight rows without a run: first lies beyond last)
+  for (int64_t base = first; base < last; base += 128) {
+    const int64_t p0 = base + lane;
+    longlong2 me[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) me[u] = ld_pair<kWide>(rows.pairs, min(p0 + 32 * u, static_cast<int64_t>(last - 1)));
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long to = __shfl_sync(0xffffffffu, shift, static_cast<int>(me[u].x - r0));
+      if (p0 + 32 * u < last) rows.entries[to + p0 + 32 * u] = static_cast<uint32_t>(me[u].y);
+    }
+  }
+}
 
 __global__ void csr_degree(const int64_t* __restrict__ pairs, int64_t npairs, int64_t nrows,
                            int32_t* __restrict__ deg, unsigned int* __restrict__ found) {
@@ -140,12 +185,21 @@ struct CsrWs {
   int64_t* cursor;       // nrows + 1 (any list); run: int2 per row (sorted list)
   unsigned int* second;  // nrows
   unsigned int* found;   // right after `second`: one memset clears both
-  uint16_t* slot;        // npairs
   char* scan;
   char* sort;
+  uint32_t* slots;       // last, as many per row as the workspace has room for
 };
 
-size_t csr_layout(int64_t npairs, int64_t nrows, CsrWs* w, void* base) {
+// Slots per row: twice the mean number of second halves and eight (an interior
+// row of a cloud with free faces, or in a shuffled order, has more than the
+// mean), at most 128 and 4 GiB in all.
+int64_t slots_wanted(int64_t npairs, int64_t nrows) {
+  if (nrows <= 0 || npairs <= 0) return 0;
+  const int64_t k = std::min<int64_t>((2 * npairs / nrows + 15) / 8 * 8, 128);
+  return std::min(k, (int64_t(4) << 30) / (nrows * static_cast<int64_t>(sizeof(uint32_t))));
+}
+
+size_t csr_layout(int64_t nrows, CsrWs* w, void* base) {
   char* cur = static_cast<char*>(base);
   size_t used = 0;
   auto take = [&](size_t bytes) -> char* {
@@ -158,9 +212,9 @@ size_t csr_layout(int64_t npairs, int64_t nrows, CsrWs* w, void* base) {
   t.cursor = reinterpret_cast<int64_t*>(take((nrows + 1) * sizeof(int64_t)));
   t.second = reinterpret_cast<unsigned int*>(take((nrows + 1) * sizeof(unsigned int)));
   t.found = t.second ? t.second + nrows : nullptr;
-  t.slot = reinterpret_cast<uint16_t*>(take(npairs * sizeof(uint16_t)));
   t.scan = take(scan_scratch_bytes(nrows + 1));
   t.sort = take(segsort_scratch_bytes(nrows));
+  t.slots = reinterpret_cast<uint32_t*>(cur + used);
   if (w) *w = t;
   return used;
 }
@@ -172,19 +226,19 @@ int read_found(const unsigned int* found, unsigned int* host, cudaStream_t s) {
 }
 
 // Returns with *taken false, and nothing written to the outputs, when the list
-// is not sorted (or a row has more than 65,536 second-element entries).
+// is not sorted.
 template <bool kWide>
 int rows_of_sorted(const int64_t* pairs, int64_t npairs, int64_t nrows, int64_t* rowptr, uint32_t* entries,
-                   const CsrWs& w, bool* taken, cudaStream_t s) {
+                   const CsrWs& w, unsigned int per_row, bool* taken, cudaStream_t s) {
   int2* run = reinterpret_cast<int2*>(w.cursor);
   TSPH_CUDA_CHECK(cudaMemsetAsync(run, 0, nrows * sizeof(int2), s));
   TSPH_CUDA_CHECK(cudaMemsetAsync(w.second, 0, (nrows + 1) * sizeof(unsigned int), s));
   const unsigned g = static_cast<unsigned>((npairs + kBlock - 1) / kBlock);
-  list_degrees<kWide><<<g, kBlock, 0, s>>>(pairs, npairs, nrows, run, w.second, w.slot, w.found);
+  list_place<kWide><<<g, kBlock, 0, s>>>(pairs, npairs, nrows, run, w.second, w.slots, per_row, w.found);
   TSPH_LAUNCH_CHECK();
   unsigned int found = 0;
   int rc = read_found(w.found, &found, s);
-  *taken = rc != TSPH_OK || found == 0;
+  *taken = true;
   // an index out of range behind an unsorted stretch is found by the general route
   if (found & kUnsorted) *taken = false;
   if (!*taken) return TSPH_OK;
@@ -193,9 +247,14 @@ int rows_of_sorted(const int64_t* pairs, int64_t npairs, int64_t nrows, int64_t*
   TSPH_LAUNCH_CHECK();
   rc = exclusive_scan_i32_to_i64(w.deg, rowptr, nrows, rowptr + nrows, w.scan, s);
   if (rc) return rc;
-  list_fill<kWide><<<g, kBlock, 0, s>>>(pairs, npairs, run, rowptr, w.slot, entries);
-  TSPH_LAUNCH_CHECK();
-  return sort_rows(SecondHalves{entries, rowptr, run}, nrows, npairs, AsEntries{entries}, w.sort, s);
+  if (found & kOver) {
+    unsigned int* placed = reinterpret_cast<unsigned int*>(w.deg);
+    TSPH_CUDA_CHECK(cudaMemsetAsync(placed, 0, nrows * sizeof(unsigned int), s));
+    list_rest<kWide><<<g, kBlock, 0, s>>>(pairs, npairs, run, rowptr, w.second, per_row, placed, entries);
+    TSPH_LAUNCH_CHECK();
+  }
+  return sort_rows(SecondHalves<kWide>{entries, rowptr, run, w.second, w.slots, per_row, pairs}, nrows,
+                   found & kOver ? npairs : per_row, AsEntries{entries}, w.sort, s);
 }
 
 }  // namespace
@@ -205,8 +264,12 @@ using namespace tsph;
 
 extern "C" {
 
-int64_t tsph_csr_workspace_bytes(int64_t npairs, int64_t nrows) {
-  return static_cast<int64_t>(csr_layout(npairs, nrows, nullptr, nullptr));
+int64_t tsph_csr_workspace_bytes(int64_t, int64_t nrows) {
+  return static_cast<int64_t>(csr_layout(nrows, nullptr, nullptr));
+}
+
+int64_t tsph_csr_slot_bytes(int64_t npairs, int64_t nrows) {
+  return nrows * slots_wanted(npairs, nrows) * static_cast<int64_t>(sizeof(uint32_t));
 }
 
 int tsph_csr_from_pairs(const int64_t* pairs, int64_t npairs, int64_t nrows, int64_t* rowptr,
@@ -215,7 +278,7 @@ int tsph_csr_from_pairs(const int64_t* pairs, int64_t npairs, int64_t nrows, int
   if (ws_bytes < tsph_csr_workspace_bytes(npairs, nrows)) return TSPH_ERR_WORKSPACE;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   CsrWs w;
-  csr_layout(npairs, nrows, &w, ws);
+  csr_layout(nrows, &w, ws);
   if (nrows == 0 || npairs == 0) {
     TSPH_CUDA_CHECK(cudaMemsetAsync(rowptr, 0, (nrows + 1) * sizeof(int64_t), s));
     return TSPH_OK;
@@ -223,8 +286,11 @@ int tsph_csr_from_pairs(const int64_t* pairs, int64_t npairs, int64_t nrows, int
   if (npairs < (int64_t(1) << 31)) {
     bool taken = false;
     const bool wide = reinterpret_cast<uintptr_t>(pairs) % 16 == 0;
-    int rc = wide ? rows_of_sorted<true>(pairs, npairs, nrows, rowptr, entries, w, &taken, s)
-                  : rows_of_sorted<false>(pairs, npairs, nrows, rowptr, entries, w, &taken, s);
+    const int64_t room = (ws_bytes - tsph_csr_workspace_bytes(npairs, nrows)) /
+                         (nrows * static_cast<int64_t>(sizeof(uint32_t)));
+    const unsigned int per_row = static_cast<unsigned int>(std::min(room, slots_wanted(npairs, nrows)));
+    int rc = wide ? rows_of_sorted<true>(pairs, npairs, nrows, rowptr, entries, w, per_row, &taken, s)
+                  : rows_of_sorted<false>(pairs, npairs, nrows, rowptr, entries, w, per_row, &taken, s);
     if (rc || taken) return rc;
   }
   TSPH_CUDA_CHECK(cudaMemsetAsync(w.deg, 0, nrows * sizeof(int32_t), s));

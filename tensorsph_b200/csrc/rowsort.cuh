@@ -141,6 +141,10 @@ struct Bounded {
   }
 };
 
+// What a warp does besides for its rows r0 .. r0 + 7 (below n); all lanes call it.
+template <class Rows>
+__device__ __forceinline__ void beside_rows(const Rows&, int64_t, int64_t) {}
+
 // The rows may lie where the output goes: a row is read whole before any of it
 // is written, and rows do not overlap.
 template <class Rows, class Out>
@@ -152,6 +156,7 @@ __global__ void __launch_bounds__(kSortBlock, 8) rows_sort(Rows rows, int64_t n,
   for (int64_t w = (static_cast<int64_t>(blockIdx.x) * kSortBlock + threadIdx.x) >> 5; 8 * w < n; w += warps) {
     const int64_t r0 = 8 * w, r = r0 + (lane & 7);
     const int64_t len = r < n ? rows.len(r) : 0;
+    beside_rows(rows, r0, n);
     int64_t longest = len;
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));

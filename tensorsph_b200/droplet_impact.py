@@ -405,7 +405,11 @@ def symmetric_rows(pairs: torch.Tensor, nrows: int):
     npairs = int(pairs.shape[0])
     rowptr = torch.empty(nrows + 1, dtype=torch.long, device=dev)
     entries = torch.empty(max(2 * npairs, 1), dtype=torch.int32, device=dev)
-    ws = _lib.workspace(L.tsph_csr_workspace_bytes(npairs, nrows), dev)
+    need = L.tsph_csr_workspace_bytes(npairs, nrows)
+    try:
+        ws = _lib.workspace(need + L.tsph_csr_slot_bytes(npairs, nrows), dev)
+    except torch.OutOfMemoryError:  # the slots only save a pass
+        ws = _lib.workspace(need, dev)
     rc = L.tsph_csr_from_pairs(pairs.data_ptr(), npairs, nrows, rowptr.data_ptr(),
                                entries.data_ptr(), ws.data_ptr(), ws.numel(), _lib.stream(dev))
     if rc == _lib.ERR_INDEX:

@@ -127,3 +127,28 @@ def test_tvc_lanes(gpu, dtype, tol, dim, n):
                                    pairs=torch.from_numpy(pairs).to(gpu))
     want = ot.kernel_gradient_integral(x, vol, 0.013, pairs, wall_count=n // 10)
     close(got, want, np.abs(want).max(), tol)
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-12), (torch.float32, 2e-5)])
+@pytest.mark.parametrize("dim,copies", [(2, 1), (2, 300), (2, 3000), (3, 1), (3, 300)])
+def test_short_rows(gpu, dtype, tol, dim, copies):
+    """Rows of 0 to 18 entries at each lane count: clusters of 1 to 19 particles, out of reach
+    of one another, all pairs of a cluster within the cutoff (the tail of a lane's part of a
+    row: no entry, one, an odd number)."""
+    from oracle import tvc as ot
+    from tensorsph_b200.transport_velocity_correction import kernel_gradient_integral
+    rng = np.random.default_rng(dim)
+    size = np.tile(np.arange(1, 20), copies)
+    n = int(size.sum())
+    start = np.concatenate(([0], np.cumsum(size)))
+    home = np.repeat(np.arange(size.size), size)
+    x = rng.uniform(0.0, 0.9, (n, dim))
+    x[:, 0] += 4.0 * (home % 64)
+    x[:, 1] += 4.0 * (home // 64)
+    pairs = np.concatenate([start[c] + np.stack(np.triu_indices(s, 1), -1) for c, s in enumerate(size)])
+    t = torch.from_numpy(x).to(gpu, dtype)
+    x, vol = t.double().cpu().numpy(), np.full(n, 0.5)
+    got = kernel_gradient_integral(t, torch.from_numpy(vol).to(gpu, dtype), 1.0,
+                                   pairs=torch.from_numpy(pairs).to(gpu))
+    want = ot.kernel_gradient_integral(x, vol, 1.0, pairs)
+    close(got, want, np.abs(want).max(), tol)

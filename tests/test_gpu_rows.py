@@ -58,3 +58,47 @@ def test_rows_refuse_bad_indices(gpu, bad):
     from tensorsph_b200.droplet_impact import symmetric_rows
     with pytest.raises(ValueError):
         symmetric_rows(torch.tensor(bad, dtype=torch.int64, device=gpu), 9)
+
+
+@pytest.mark.parametrize("per_row", [0, 1, 7, 19, 20, 10 ** 6])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_rows_at_slot_counts(gpu, per_row, mixed):
+    """Workspaces with room for no, few, almost enough, just enough and more slots than a
+    row's second halves (at most 20 here) give the same rows."""
+    from tensorsph_b200 import _lib
+    rng = np.random.default_rng(per_row)
+    n = 1003
+    p = np.stack((np.repeat(np.arange(n), 20), (np.arange(n)[:, None] + 1 + np.arange(20)).reshape(-1)), axis=1)
+    p = p[p[:, 1] < n]
+    if mixed:
+        p = np.sort(rng.permutation(n)[p], axis=1)
+        p = p[np.lexsort((p[:, 1], p[:, 0]))]
+    L = _lib.lib()
+    t = torch.from_numpy(p).to(gpu)
+    ptr = torch.empty(n + 1, dtype=torch.long, device=gpu)
+    entries = torch.empty(2 * p.shape[0], dtype=torch.int32, device=gpu)
+    least = L.tsph_csr_workspace_bytes(p.shape[0], n)
+    room = min(4 * n * per_row, L.tsph_csr_slot_bytes(p.shape[0], n))
+    ws = _lib.workspace(least + room, gpu)
+    args = (t.data_ptr(), p.shape[0], n, ptr.data_ptr(), entries.data_ptr(), ws.data_ptr())
+    _lib.check(L.tsph_csr_from_pairs(*args, least + room, _lib.stream(gpu)), "tsph_csr_from_pairs")
+    want_ptr, want = expected_rows(p, n)
+    assert np.array_equal(ptr.cpu().numpy(), want_ptr)
+    assert np.array_equal(entries.cpu().numpy().view(np.uint32).astype(np.int64), want)
+    assert L.tsph_csr_from_pairs(*args, least - 1, _lib.stream(gpu)) != 0
+
+
+def test_rows_without_memory_for_slots(gpu, monkeypatch):
+    from tensorsph_b200 import _lib
+    plain, refused = _lib.workspace, []
+
+    def tight(nbytes, device):
+        if not refused:
+            refused.append(nbytes)
+            raise torch.OutOfMemoryError("no room")
+        return plain(nbytes, device)
+
+    monkeypatch.setattr(_lib, "workspace", tight)
+    p = np.sort(np.random.default_rng(0).integers(0, 500, (9000, 2)), axis=1)
+    check(p[np.lexsort((p[:, 1], p[:, 0]))], 500, gpu)
+    assert refused
