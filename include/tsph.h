@@ -390,6 +390,10 @@ typedef struct {
 /* replaces kernel_gradient_integral (transport_velocity_correction.py:285-410):
  * gradient and squared */
 int tsph_tvc_gradient(const tsph_tvc_params* prm, const tsph_tvc_io* io, tsph_stream stream);
+/* the same, faster with a workspace (NULL or tsph_tvc_workspace_bytes) */
+int64_t tsph_tvc_workspace_bytes(const tsph_tvc_params* prm);
+int tsph_tvc_gradient_ws(const tsph_tvc_params* prm, const tsph_tvc_io* io, void* ws, int64_t ws_bytes,
+                         tsph_stream stream);
 /* replaces the displacement of transport_velocity_correction
  * (transport_velocity_correction.py:413-513): limiter, shift, clipped count */
 int tsph_tvc_shift(const tsph_tvc_params* prm, const tsph_tvc_io* io, tsph_stream stream);

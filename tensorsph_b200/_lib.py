@@ -222,6 +222,8 @@ _SIGNATURES = {
     "tsph_csf2_contact_boundary": (c_int, [POINTER(Csf2Params), c_void_p, c_void_p, c_void_p, c_void_p,
                                            c_void_p, c_int64, c_void_p]),
     "tsph_tvc_gradient": (c_int, [POINTER(TvcParams), POINTER(TvcIO), c_void_p]),
+    "tsph_tvc_workspace_bytes": (c_int64, [POINTER(TvcParams)]),
+    "tsph_tvc_gradient_ws": (c_int, [POINTER(TvcParams), POINTER(TvcIO), c_void_p, c_int64, c_void_p]),
     "tsph_tvc_shift": (c_int, [POINTER(TvcParams), POINTER(TvcIO), c_void_p]),
     "tsph_csf3_workspace_bytes": (c_int64, [POINTER(Csf3Params)]),
     "tsph_csf3_fields": (c_int, [POINTER(Csf3Params), POINTER(Csf3IO), c_void_p, c_int64, c_void_p]),

@@ -35,9 +35,21 @@ __device__ __forceinline__ T sigma_d(T h) {
   return T(1) / (T(M_PI) * h * h * h);
 }
 
-template <int D, class T, int L>
+// Position and volume in one record.
+template <int D, class T>
+__global__ void v_pack(const T* __restrict__ pos, const T* __restrict__ vol, int64_t n, Q4<T>* __restrict__ rec) {
+  for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < n;
+       a += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    rec[a] = Q4<T>{pos[D * a], D > 1 ? pos[D * a + 1] : T(0), D > 2 ? pos[D * a + 2] : T(0), vol[a]};
+}
+
+// kPacked: the neighbours come from rec, else from pos and vol.  In mixed order a
+// term's gathers are what it waits for: 328 k rows of 80 entries, FP64, 278 us from
+// the two arrays (three to four sectors a term), 138 from records (one).
+template <int D, class T, int L, bool kPacked>
 __global__ void __launch_bounds__(kGatherBlock) v_gradient(VP<T> p, const T* __restrict__ pos,
-                                                           const T* __restrict__ vol, const T* __restrict__ ratio,
+                                                           const T* __restrict__ vol, const Q4<T>* __restrict__ rec,
+                                                           const T* __restrict__ ratio,
                                                            const T* __restrict__ corr,
                                                            const int64_t* __restrict__ rowptr,
                                                            const uint32_t* __restrict__ ent, T* __restrict__ grad,
@@ -55,10 +67,21 @@ __global__ void __launch_bounds__(kGatherBlock) v_gradient(VP<T> p, const T* __r
   CSum<T> s[D];
   me.walk_ahead(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
     const int64_t b = e & kIndexMask;
-    T d[D], r2 = T(0);
+    T xb[D], vb, d[D], r2 = T(0);
+    if (kPacked) {
+      const Q4<T> q = rec[b];
+      xb[0] = q.x;
+      if (D > 1) xb[D > 1 ? 1 : 0] = q.y;
+      if (D > 2) xb[D > 2 ? 2 : 0] = q.z;
+      vb = q.w;
+    } else {
+#pragma unroll
+      for (int k = 0; k < D; ++k) xb[k] = pos[D * b + k];
+      vb = vol[b];
+    }
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-      d[k] = xa[k] - pos[D * b + k];
+      d[k] = xa[k] - xb[k];
       r2 += d[k] * d[k];
     }
     T q, scale;
@@ -76,7 +99,7 @@ __global__ void __launch_bounds__(kGatherBlock) v_gradient(VP<T> p, const T* __r
     const T ds = q < T(1) ? T(-3) * q + T(2.25) * q * q : (q < T(2) ? T(-0.75) * t * t : T(0));
     scale = scale * ds;
     const T cb = p.has_corr ? corr[b] : T(1);
-    const T w = (b < p.n_fluid ? ca + cb : p.wall_factor * ca) * vol[b];
+    const T w = (b < p.n_fluid ? ca + cb : p.wall_factor * ca) * vb;
 #pragma unroll
     for (int k = 0; k < D; ++k) s[k].add(w * (d[k] * scale));
   });
@@ -152,7 +175,7 @@ bool params_ok(const tsph_tvc_params* p) {
 }
 
 template <class T>
-int run_gradient(const tsph_tvc_params& prm, const tsph_tvc_io& io, cudaStream_t s) {
+int run_gradient(const tsph_tvc_params& prm, const tsph_tvc_io& io, Q4<T>* rec, cudaStream_t s) {
   VP<T> p{};
   p.n_total = prm.n_total;
   p.n_fluid = prm.n_fluid;
@@ -172,8 +195,15 @@ int run_gradient(const tsph_tvc_params& prm, const tsph_tvc_io& io, cudaStream_t
     constexpr int D = decltype(dim)::value;
     return with_lanes<D>(prm.n_fluid, [&](auto lanes) -> int {
       constexpr int LN = decltype(lanes)::value;
-      v_gradient<D, T, LN><<<row_grid(prm.n_fluid, LN), kGatherBlock, 0, s>>>(p, pos, vol, ratio, corr, io.rowptr,
-                                                                             io.entries, grad, sq);
+      const unsigned g = row_grid(prm.n_fluid, LN);
+      if (rec) {
+        v_pack<D, T><<<grid_for(prm.n_total, 256), 256, 0, s>>>(pos, vol, prm.n_total, rec);
+        v_gradient<D, T, LN, true><<<g, kGatherBlock, 0, s>>>(p, pos, vol, rec, ratio, corr, io.rowptr, io.entries,
+                                                              grad, sq);
+      } else {
+        v_gradient<D, T, LN, false><<<g, kGatherBlock, 0, s>>>(p, pos, vol, rec, ratio, corr, io.rowptr, io.entries,
+                                                               grad, sq);
+      }
       TSPH_LAUNCH_CHECK();
       return TSPH_OK;
     });
@@ -215,15 +245,27 @@ using namespace tsph;
 
 extern "C" {
 
-int tsph_tvc_gradient(const tsph_tvc_params* prm, const tsph_tvc_io* io, tsph_stream stream) {
+int64_t tsph_tvc_workspace_bytes(const tsph_tvc_params* prm) {
+  if (!params_ok(prm)) return 0;
+  return prm->n_total * 4 * static_cast<int64_t>(prm->dtype == TSPH_F64 ? sizeof(double) : sizeof(float));
+}
+
+int tsph_tvc_gradient_ws(const tsph_tvc_params* prm, const tsph_tvc_io* io, void* ws, int64_t ws_bytes,
+                         tsph_stream stream) {
   if (!params_ok(prm) || !io) return TSPH_ERR_ARG;
   if (prm->n_fluid == 0) return TSPH_OK;
   if (!io->pos || !io->volume || !io->rowptr || !io->entries || !io->gradient || !io->squared ||
       (prm->has_ratio && !io->h_ratio))
     return TSPH_ERR_ARG;
+  if (ws && ws_bytes < tsph_tvc_workspace_bytes(prm)) return TSPH_ERR_WORKSPACE;
+  if (reinterpret_cast<uintptr_t>(ws) % 32) ws = nullptr;  // the records' boundary
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (prm->dtype == TSPH_F64) return run_gradient<double>(*prm, *io, s);
-  return run_gradient<float>(*prm, *io, s);
+  if (prm->dtype == TSPH_F64) return run_gradient<double>(*prm, *io, static_cast<Q4<double>*>(ws), s);
+  return run_gradient<float>(*prm, *io, static_cast<Q4<float>*>(ws), s);
+}
+
+int tsph_tvc_gradient(const tsph_tvc_params* prm, const tsph_tvc_io* io, tsph_stream stream) {
+  return tsph_tvc_gradient_ws(prm, io, nullptr, 0, stream);
 }
 
 int tsph_tvc_shift(const tsph_tvc_params* prm, const tsph_tvc_io* io, tsph_stream stream) {

@@ -174,8 +174,13 @@ def _gradient(positions, volume, h, pairs, ratio, h_scale, wall_count, wall_fact
     io.h_ratio = 0 if R is None else R.data_ptr()
     io.correction = 0 if C is None else C.data_ptr()
     io.gradient, io.squared = grad.data_ptr(), squared.data_ptr()
-    _lib.check(_lib.lib().tsph_tvc_gradient(ctypes.byref(prm), ctypes.byref(io), _lib.stream(dev)),
-               "tsph_tvc_gradient")
+    L = _lib.lib()
+    try:
+        ws = _lib.workspace(L.tsph_tvc_workspace_bytes(ctypes.byref(prm)), dev)
+    except torch.OutOfMemoryError:  # the records only save time
+        ws = None
+    _lib.check(L.tsph_tvc_gradient_ws(ctypes.byref(prm), ctypes.byref(io), 0 if ws is None else ws.data_ptr(),
+                                      0 if ws is None else ws.numel(), _lib.stream(dev)), "tsph_tvc_gradient")
     return prm, io, grad, squared, R, (rowptr, entries, P, Vol, C)
 
 

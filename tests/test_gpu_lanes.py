@@ -152,3 +152,36 @@ def test_short_rows(gpu, dtype, tol, dim, copies):
                                    pairs=torch.from_numpy(pairs).to(gpu))
     want = ot.kernel_gradient_integral(x, vol, 1.0, pairs)
     close(got, want, np.abs(want).max(), tol)
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-12), (torch.float32, 2e-5)])
+@pytest.mark.parametrize("dim,options", [(1, False), (2, True), (3, False), (3, True)])
+def test_tvc_without_records(gpu, monkeypatch, dtype, tol, dim, options):
+    """Without memory for the packed records the sums come from the caller's arrays."""
+    from oracle import tvc as ot
+    from tensorsph_b200 import _lib
+    from tensorsph_b200.transport_velocity_correction import kernel_gradient_integral
+    n = 1331
+    rng = np.random.default_rng(dim)
+    side = int(np.ceil(n ** (1.0 / dim)))
+    g = np.stack(np.meshgrid(*[np.arange(side)] * dim, indexing="ij"), -1).reshape(-1, dim)[:n]
+    t = torch.from_numpy(((g + 0.1 * rng.uniform(-1, 1, g.shape)) * 0.01)[rng.permutation(n)]).to(gpu, dtype)
+    vol = torch.from_numpy(0.01 ** dim * rng.uniform(0.5, 2.0, n)).to(gpu, dtype)
+    kw = dict(wall_count=100) if options else {}
+    corr = torch.from_numpy(rng.uniform(0.9, 1.1, n)).to(gpu, dtype) if options else None
+    pairs = cell_linked_pairs_batched(t.double().cpu().numpy(), 0.026)
+    plain, refused = _lib.workspace, []
+
+    def tight(nbytes, device):
+        if nbytes == n * 4 * t.element_size():
+            refused.append(nbytes)
+            raise torch.OutOfMemoryError("no room")
+        return plain(nbytes, device)
+
+    want = ot.kernel_gradient_integral(t.double().cpu().numpy(), vol.double().cpu().numpy(), 0.013, pairs,
+                                       correction=None if corr is None else corr.double().cpu().numpy(), **kw)
+    for route in (plain, tight):
+        monkeypatch.setattr(_lib, "workspace", route)
+        got = kernel_gradient_integral(t, vol, 0.013, pairs=torch.from_numpy(pairs).to(gpu), correction=corr, **kw)
+        close(got, want, np.abs(want).max(), tol)
+    assert refused
