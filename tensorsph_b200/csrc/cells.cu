@@ -49,9 +49,9 @@ struct GridDev {
 struct BuildWs {
   uint64_t* keys;      // n (radix), or the key and slot of every particle (dense)
   uint64_t* keys_tmp;  // n
-  int32_t* order;      // n (sorted position -> particle)
+  int32_t* order;      // n, sorted: the particle (dense: in 3-D)
   int32_t* order_tmp;  // n
-  float4* rec;         // n, sorted: position from the grid's corner and the particle
+  float* rec;          // n, sorted: position from the grid's corner (rec_at)
   int32_t* cell;       // n * dim, sorted: cell coordinates relative to origin
   int32_t* counts;     // total_cells (dense) or 0, then
   int32_t* longest;    // 1: 0, or the longest row when it has outgrown its slots
@@ -89,7 +89,7 @@ size_t build_layout(const tsph_grid& g, BuildWs* w, void* base) {
   t.keys_tmp = reinterpret_cast<uint64_t*>(take(n * sizeof(uint64_t)));
   t.order = reinterpret_cast<int32_t*>(take(n * sizeof(int32_t)));
   t.order_tmp = reinterpret_cast<int32_t*>(take(n * sizeof(int32_t)));
-  t.rec = reinterpret_cast<float4*>(take(n * sizeof(float4)));
+  t.rec = reinterpret_cast<float*>(take((n + 3) / 4 * 4 * sizeof(float4)));
   t.cell = reinterpret_cast<int32_t*>(take(n * g.dim * sizeof(int32_t)));
   t.counts = reinterpret_cast<int32_t*>(take((cells + 1) * sizeof(int32_t)));
   t.longest = t.counts ? t.counts + (g.dense ? g.total_cells : 0) : nullptr;
@@ -103,6 +103,17 @@ size_t build_layout(const tsph_grid& g, BuildWs* w, void* base) {
   if (w) *w = t;
   return used;
 }
+
+// Where record t's first coordinate is and how far apart the others are.  In 3-D
+// records stand in blocks of four, four x, four y, four z, so that four candidates
+// are loaded 16 bytes at a time and computed two to an instruction; below, where a
+// run holds a dozen candidates, one record is 16 bytes (position and particle).
+template <int D>
+__device__ __forceinline__ int64_t rec_at(int64_t t) {
+  return D == 3 ? (t >> 2) * 12 + (t & 3) : 4 * t;
+}
+template <int D>
+constexpr int kRecStep = D == 3 ? 4 : 1;
 
 GridDev to_dev(const tsph_grid& g) {
   GridDev d{};
@@ -247,8 +258,8 @@ __global__ void cell_count(const T* __restrict__ pos, int64_t n, GridDev g, int3
 // Records in cell order: to start[key] + slot (dense), or from the sorted order.
 template <class T, int D, bool kDense>
 __global__ void cell_scatter(const T* __restrict__ pos, int64_t n, GridDev g, const int64_t* __restrict__ start,
-                             const int32_t* __restrict__ slots, const int32_t* __restrict__ order,
-                             float4* __restrict__ rec, int32_t* __restrict__ cell) {
+                             const int32_t* __restrict__ slots, int32_t* __restrict__ order,
+                             float* __restrict__ rec, int32_t* __restrict__ cell) {
   for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < n;
        t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t a = kDense ? t : order[t];
@@ -256,7 +267,13 @@ __global__ void cell_scatter(const T* __restrict__ pos, int64_t n, GridDev g, co
     float x[3] = {0.f, 0.f, 0.f};
     const uint64_t key = key_of<T, D>(pos, a, g, c, x);
     const int64_t at = kDense ? start[key] + slots[a] : t;
-    rec[at] = make_float4(x[0], x[1], x[2], __int_as_float(static_cast<int>(a)));
+    if (D < 3) {
+      reinterpret_cast<float4*>(rec)[at] = make_float4(x[0], x[1], 0.f, __int_as_float(static_cast<int>(a)));
+    } else {
+#pragma unroll
+      for (int k = 0; k < D; ++k) rec[rec_at<D>(at) + 4 * k] = x[k];
+      if (kDense) order[at] = static_cast<int>(a);
+    }
 #pragma unroll
     for (int k = 0; k < D; ++k) cell[at * D + k] = c[k];
   }
@@ -325,11 +342,39 @@ Band band_of(const tsph_grid& g) {
 }
 
 struct Cells {
-  const float4* rec;
+  const float* rec;
+  const int32_t* id;
   const int32_t* cell;
   const int64_t* start;   // dense
   const uint64_t* keys;   // not dense: sorted
 };
+
+// Two FP32 operations in one instruction, each rounded as its scalar form.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+// bits <- bits, sign of the low half, sign of the high half
+__device__ __forceinline__ void push_signs(uint32_t& bits, uint64_t v) {
+  const uint32_t lo = static_cast<uint32_t>(v), hi = static_cast<uint32_t>(v >> 32);
+  bits = __funnelshift_l(hi, __funnelshift_l(lo, bits, 1), 1);
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
 
 // What a row holds: kForward b > a (the list's pairs (a, b)); kBoth every
 // neighbour whose pair's first index is below the limit, as gather-row entries
@@ -345,12 +390,12 @@ enum RowPass { kCount, kSlot, kFill };
 // slots (in any order) and raises `longest` where that was not all, kFill, run
 // when it was raised, writes the rows from rowptr on.
 //
-// What bounds it: instruction issue (6 FP32 operations, the record load and
-// the tests per candidate; the 3-D list at 2.05 h scans ~500 candidates for
-// ~80 hits) and, with the stores of kSlot, scattered 4-byte writes.  1.0 M FP64
-// particles in 3-D: 0.54 ms (0.39 when it only counts), against 1.55 ms to
-// count and 1.65 to write with a thread per particle in the caller's order,
-// FP64 distances for every candidate and 27 cells by division.
+// What bounds it: instruction issue (in 3-D three to four instructions a candidate
+// and twenty a hit; the list at 2.05 h scans ~500 candidates for ~80 hits) and, with
+// the stores of kSlot, scattered 4-byte writes.  1.0 M FP64 particles in 3-D: 0.48
+// ms; with compares and predicates in place of the signs 0.55, and 1.55 ms to
+// count and 1.65 to write with a thread per particle in the caller's order, FP64
+// distances for every candidate and 27 cells by division.
 template <class T, int D, RowKind kKind, RowPass kPass, int kLanes>
 __global__ void __launch_bounds__(128) scan_rows(const T* __restrict__ pos, int64_t n, int64_t row_limit, GridDev g,
                                                  Cells cs, Band band, T c2, int32_t* __restrict__ rowcount,
@@ -363,13 +408,13 @@ __global__ void __launch_bounds__(128) scan_rows(const T* __restrict__ pos, int6
   const unsigned group = kLanes == 1 ? 1u << lane : ((kLanes == 32 ? 0u : 1u << kLanes) - 1u) << (lane - gl);
   const int64_t t = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / kLanes;
   if (t >= n) return;
-  const float4 ra = cs.rec[t];
-  const int64_t a = __float_as_int(ra.w);
+  const float* ra = cs.rec + rec_at<D>(t);
+  const int64_t a = D == 3 ? cs.id[t] : __float_as_int(ra[3]);
   if (kKind == kForward && kPass == kFill && a >= row_limit) return;
   int c[3] = {0, 0, 0};
 #pragma unroll
   for (int k = 0; k < D; ++k) c[k] = cs.cell[t * D + k];
-  const float xa[3] = {ra.x, ra.y, ra.z};
+  const float xa[3] = {ra[0], D > 1 ? ra[kRecStep<D>] : 0.f, D > 2 ? ra[2 * kRecStep<D>] : 0.f};
   int count = 0;
   const int64_t slot = kPass == kFill ? rowptr[a] : a * slots;
 
@@ -380,46 +425,117 @@ __global__ void __launch_bounds__(128) scan_rows(const T* __restrict__ pos, int6
     if (kPass == kSlot && at >= slots) return;
     out[slot + at] = kKind == kBoth && b < me ? static_cast<uint32_t>(b) | kSecond : static_cast<uint32_t>(b);
   };
-  // kBatch candidates at once: the tests against the outer bound are predicates,
-  // and one branch per batch looks at those between the bounds
-  auto run = [&](int beg, int end, float x, float y, float z) {
-    constexpr int kBatch = kLanes == 1 ? 4 : 1;
-    for (int p0 = beg; p0 < end; p0 += kBatch * kLanes) {
-      float4 rb[kBatch];
-      bool hit[kBatch];
+  const auto wanted = [&](int b) { return kKind == kForward ? b > me : b != me && (first || b < limit); };
+  // A thread's own row, 1-D and 2-D: four candidates at once; the tests against the
+  // outer bound are predicates, and one branch per batch looks at those between the
+  // bounds (by signs a 2-D pass of 200 k rows takes 47 us, so 38).
+  auto run_batch = [&](int beg, int end, float x, float y) {
+    const float4* recs = reinterpret_cast<const float4*>(cs.rec);
+    for (int p0 = beg; p0 < end; p0 += 4) {
+      float4 rb[4];
+      bool hit[4];
       bool unsure = false;
 #pragma unroll
-      for (int j = 0; j < kBatch; ++j) rb[j] = cs.rec[min(p0 + j + gl, end - 1)];
+      for (int j = 0; j < 4; ++j) rb[j] = recs[min(p0 + j, end - 1)];
 #pragma unroll
-      for (int j = 0; j < kBatch; ++j) {
-        const int b = __float_as_int(rb[j].w);
-        const float dx = x - rb[j].x, dy = y - rb[j].y, dz = z - rb[j].z;
+      for (int j = 0; j < 4; ++j) {
+        const float dx = x - rb[j].x, dy = y - rb[j].y;
         float d2 = dx * dx;
         if (D > 1) d2 = fmaf(dy, dy, d2);
-        if (D > 2) d2 = fmaf(dz, dz, d2);
-        const bool want = kKind == kForward ? b > me : b != me && (first || b < limit);
-        hit[j] = d2 < band.out && want && p0 + j + gl < end;
+        hit[j] = d2 < band.out && wanted(__float_as_int(rb[j].w)) && p0 + j < end;
         unsure |= hit[j] && d2 > band.in;
       }
       if (unsure) {
 #pragma unroll
-        for (int j = 0; j < kBatch; ++j)
+        for (int j = 0; j < 4; ++j)
           if (hit[j]) hit[j] = pair_d2<T, D>(px, a, __float_as_int(rb[j].w), g) <= c2;
       }
-      if (kLanes == 1) {
 #pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-          if (kPass != kCount && hit[j]) put(count, __float_as_int(rb[j].w));
-          count += hit[j];
-        }
-      } else if (kPass != kCount) {
-        const unsigned m = __ballot_sync(group, hit[0]) & group;
-        if (hit[0]) put(count + __popc(m & ((1u << lane) - 1u)), __float_as_int(rb[0].w));
-        count += __popc(m);
-      } else {
-        count += hit[0];
+      for (int j = 0; j < 4; ++j) {
+        if (kPass != kCount && hit[j]) put(count, __float_as_int(rb[j].w));
+        count += hit[j];
       }
     }
+  };
+  // A thread's own row, 3-D.  Up to 32 candidates leave the signs of d^2 - out and
+  // d^2 - in in a word each (a subtraction, two to an instruction, and a shift, where
+  // a compare and its predicate logic cost three on the integer pipe, which bounded
+  // the pass), and of a - b; then the few that are in are looked at one by one.
+  auto run_signs = [&](int beg, int end, float x, float y, float z) {
+    const uint64_t xx = pack2(x, x), yy = pack2(y, y), zz = pack2(z, z);
+    const uint64_t in2 = pack2(band.in, band.in), out2 = pack2(band.out, band.out);
+    for (int q = beg & ~3; q < end; q += 32) {
+      const ulonglong2* blk = reinterpret_cast<const ulonglong2*>(cs.rec + rec_at<3>(q));
+      const int blocks = min(8, (end - q + 3) >> 2);
+      uint32_t hits = 0, sure = 0, after = 0;
+      const int4* ids = reinterpret_cast<const int4*>(cs.id + q);
+#pragma unroll 2
+      for (int i = 0; i < blocks; ++i, blk += 3) {
+        const ulonglong2 bx = blk[0], by = blk[1], bz = blk[2];
+        uint64_t d0 = sub2(xx, bx.x), d1 = sub2(xx, bx.y);
+        const uint64_t e0 = sub2(yy, by.x), e1 = sub2(yy, by.y), f0 = sub2(zz, bz.x), f1 = sub2(zz, bz.y);
+        d0 = fma2(f0, f0, fma2(e0, e0, mul2(d0, d0)));
+        d1 = fma2(f1, f1, fma2(e1, e1, mul2(d1, d1)));
+        push_signs(hits, sub2(d0, out2));
+        push_signs(hits, sub2(d1, out2));
+        push_signs(sure, sub2(d0, in2));
+        push_signs(sure, sub2(d1, in2));
+        if (kKind == kForward) {
+          const int4 b = ids[i];
+          after = __funnelshift_l(me - b.x, after, 1);
+          after = __funnelshift_l(me - b.y, after, 1);
+          after = __funnelshift_l(me - b.z, after, 1);
+          after = __funnelshift_l(me - b.w, after, 1);
+        }
+      }
+      if (kKind == kForward) hits &= after;
+      hits <<= 32 - 4 * blocks;
+      sure <<= 32 - 4 * blocks;
+      // the blocks at the run's ends hold other cells' particles too
+      if (q < beg) hits &= 0xffffffffu >> (beg - q);
+      if (end - q < 32) hits &= ~(0xffffffffu >> (end - q));
+      for (uint32_t doubt = hits & ~sure; doubt;) {
+        const int k = __clz(doubt);
+        doubt ^= 0x80000000u >> k;
+        if (!(pair_d2<T, D>(px, a, cs.id[q + k], g) <= c2)) hits ^= 0x80000000u >> k;
+      }
+      while (hits) {
+        const int k = __clz(hits);
+        hits ^= 0x80000000u >> k;
+        const int b = cs.id[q + k];
+        const bool in = kKind == kForward || wanted(b);
+        if (kPass != kCount && in) put(count, b);
+        count += in;
+      }
+    }
+  };
+  auto run_shared = [&](int beg, int end, float x, float y, float z) {
+    for (int p0 = beg; p0 < end; p0 += kLanes) {
+      const int at = min(p0 + gl, end - 1);
+      const float* rb = cs.rec + rec_at<D>(at);
+      const int b = D == 3 ? cs.id[at] : __float_as_int(rb[3]);
+      const float dx = x - rb[0];
+      float d2 = dx * dx;
+      if (D > 1) d2 = fmaf(y - rb[kRecStep<D>], y - rb[kRecStep<D>], d2);
+      if (D > 2) d2 = fmaf(z - rb[2 * kRecStep<D>], z - rb[2 * kRecStep<D>], d2);
+      bool hit = d2 < band.out && wanted(b) && p0 + gl < end;
+      if (hit && d2 > band.in) hit = pair_d2<T, D>(px, a, b, g) <= c2;
+      if (kPass != kCount) {
+        const unsigned m = __ballot_sync(group, hit) & group;
+        if (hit) put(count + __popc(m & ((1u << lane) - 1u)), b);
+        count += __popc(m);
+      } else {
+        count += hit;
+      }
+    }
+  };
+  auto run = [&](int beg, int end, float x, float y, float z) {
+    if constexpr (kLanes > 1)
+      run_shared(beg, end, x, y, z);
+    else if constexpr (D == 3)
+      run_signs(beg, end, x, y, z);
+    else
+      run_batch(beg, end, x, y);
   };
   // first sorted position of cells [k0, k1] of the key space
   auto cells = [&](int64_t k0, int64_t k1, float x, float y, float z) {
@@ -491,7 +607,7 @@ template <class T, int D, RowKind kKind, RowPass kPass>
 int launch_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, const BuildWs& w, const int64_t* rowptr,
                 uint32_t* out, cudaStream_t s) {
   const int64_t n = grid.n;
-  const Cells cs{w.rec, w.cell, w.start, w.keys};
+  const Cells cs{w.rec, w.order, w.cell, w.start, w.keys};
   const T c2 = static_cast<T>(grid.cutoff * grid.cutoff);
   const T* p = static_cast<const T*>(pos);
   const int slots = static_cast<int>(row_slots(grid));
@@ -729,7 +845,8 @@ int tsph_grid_build(const void* pos, const tsph_grid* grid, void* ws, int64_t ws
       int rc2 = exclusive_scan_i32_to_i64(w.counts, w.start, grid->total_cells, w.start + grid->total_cells,
                                           w.scan_scratch, s);
       if (rc2) return rc2;
-      cell_scatter<T, D, true><<<grid_for(n, kBlock), kBlock, 0, s>>>(p, n, g, w.start, slots, nullptr, w.rec, w.cell);
+      cell_scatter<T, D, true><<<grid_for(n, kBlock), kBlock, 0, s>>>(p, n, g, w.start, slots, w.order, w.rec,
+                                                                          w.cell);
     } else {
       cell_scatter<T, D, false><<<grid_for(n, kBlock), kBlock, 0, s>>>(p, n, g, nullptr, nullptr, w.order, w.rec, w.cell);
     }

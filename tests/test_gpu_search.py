@@ -117,3 +117,27 @@ def test_rows_at_their_slots(gpu, count, dim):
     (ptr, entries, total), (ptr2, entries2), pairs = rows_and_pairs(pos, 0.02, pos.shape[0], gpu)
     assert np.array_equal(pairs.cpu().numpy(), on.cell_linked_pairs(pos, 0.02))
     assert torch.equal(ptr, ptr2) and torch.equal(entries[:total], entries2[:total])
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("box,lattice_points,offset", [(None, False, 0.0), (None, True, 0.0), (None, False, 3.0e3),
+                                                       (1.0, False, 0.0), (1.0, True, 0.0)])
+def test_runs_of_any_length(gpu, dtype, box, lattice_points, offset):
+    """The 3-D pass of a row per thread: runs of candidates from none to several words of
+    32, starting anywhere in a block of four, with distances at the cutoff (the lattice) and
+    with many candidates to decide exactly (the far origin)."""
+    from oracle.neighbors import cell_linked_pairs_batched
+    rng = np.random.default_rng(8)
+    if lattice_points:
+        pos = lattice((32, 32, 32), 1.0 / 32, dtype, 0.0)[:25000]
+        cutoff = 2.0 / 32
+    else:
+        pos = rng.random((25000, 3)) ** [1.0, 1.0, 3.0]       # dense at one face, sparse at the other
+        pos = (pos + offset).astype(dtype)
+        cutoff = 0.052
+    pos = pos[rng.permutation(pos.shape[0])]
+    want = cell_linked_pairs_batched(pos, cutoff) if box is None else on.periodic_pairs(pos, [box] * 3, cutoff)
+    assert np.array_equal(search(pos, cutoff, gpu, None if box is None else [box] * 3), want)
+    if box is None:
+        (ptr, entries, count), (ptr2, entries2), _ = rows_and_pairs(pos, cutoff, pos.shape[0] // 2, gpu)
+        assert torch.equal(ptr, ptr2) and torch.equal(entries[:count], entries2[:count])
