@@ -508,25 +508,28 @@ __device__ __forceinline__ const CaseDev& case_of(const Dev& e, int64_t a) {
 // ------------------------------------------------------------ rebuild ---
 
 // Step start of one case: clear the per-step meters, fix the step size.
-__device__ __forceinline__ void step_begin(const CaseDev& C, CaseCtl& t) {
-  t.rho_max = t.speed_max = t.front_max = 0;
-  t.ke = t.pe = 0;
-  t.force[0] = t.force[1] = t.force[2] = 0;
-  t.disp[0] = 0;
+__device__ __forceinline__ void step_begin(const CaseDev& C, const CaseCtl& t, CaseCtl& out) {
+  const double dt = C.dt;
+  const int adaptive = C.adaptive;
+  out.rho_max = out.speed_max = out.front_max = 0;
+  out.ke = out.pe = 0;
+  out.force[0] = out.force[1] = out.force[2] = 0;
+  out.disp[0] = 0;
   if (!t.active) return;
-  if (C.adaptive) {
+  if (adaptive) {
     // dam_break.py:379-408: step_dt = min(dt, target - elapsed); the step at
     // which elapsed reaches the target records the final meters and is not
     // integrated; after it the case stays frozen
     const bool final_now = !t.finished && t.elapsed >= C.target_time - C.time_tol;
-    t.dt_step = t.finished ? 0.0 : fmin(t.dt_now, C.target_time - t.elapsed);
-    t.dt_int = (t.finished || final_now) ? 0.0 : t.dt_step;
+    const double step = t.finished ? 0.0 : fmin(t.dt_now, C.target_time - t.elapsed);
+    out.dt_step = step;
+    out.dt_int = (t.finished || final_now) ? 0.0 : step;
     if (final_now) {
-      t.finished = 1;
-      t.final_step = static_cast<int>(t.steps);
+      out.finished = 1;
+      out.final_step = static_cast<int>(t.steps);
     }
   } else {
-    t.dt_step = t.dt_int = C.dt;
+    out.dt_step = out.dt_int = dt;
   }
 }
 
@@ -538,19 +541,22 @@ __global__ void __launch_bounds__(1024) k_check(Dev e, int first_pass, cudaGraph
                                                 int conditional) {
   int any = 0;
   for (int c = threadIdx.x; c < e.n_slots; c += blockDim.x) {
-    CaseCtl& t = e.ctl[c];
+    // the state read whole first, as in k_finalize
+    CaseCtl& out = e.ctl[c];
+    const CaseCtl t = out;
+    const double half = e.cases[c].skin_half;
     int go = 0;
     if (t.active) {
       const double d = __longlong_as_double(static_cast<long long>(t.shift_done ? t.disp[1] : t.disp[0]));
-      go = t.first || d > e.cases[c].skin_half;
+      go = t.first || d > half;
       if (go) {
-        t.rebuilds += 1;
-        t.first = 0;
+        out.rebuilds = t.rebuilds + 1;
+        out.first = 0;
       }
     }
-    t.rebuild = go;
+    out.rebuild = go;
     any |= go;
-    if (first_pass) step_begin(e.cases[c], t);
+    if (first_pass) step_begin(e.cases[c], t, out);
   }
   any = __syncthreads_or(any);
   if (threadIdx.x == 0) {
@@ -1516,7 +1522,8 @@ __device__ __forceinline__ bool row_nearest_wall(const Dev& e, int a, double ax,
 // One reciprocal square root gives r and 1 / r (the division by r and the root
 // took about 45 of a term's 60 FP64 instructions).  64 droplet cases, 0.95 M
 // rows: colour 162 -> 111 us, gradient 190 -> 144, divergence 208 -> 146, the
-// normal passes unchanged; with the dense arrays of k_csf_begin 97, 119 and 131,
+// normal passes unchanged; with the dense arrays of k_csf_begin 97, 119 (109 at four
+// blocks an SM) and 131,
 // the normal passes 123 and 127 -> 105 and 112.  L1 is then 60-70 % busy, the
 // FP64 pipe 35-55 %.  Below r = 1e-12, where the reference divides by that, q is
 // as good as r / h: W is W(0) to the last bit.
@@ -1759,7 +1766,7 @@ __device__ __forceinline__ void csf_matrix(const Dev& e, int c, const double4& A
   }
 }
 
-__global__ void __launch_bounds__(kMaxBlock) k_csf_grad(const __grid_constant__ Dev e) {
+__global__ void __launch_bounds__(kMaxBlock, 4) k_csf_grad(const __grid_constant__ Dev e) {
   __shared__ double red[kMaxBlock / 32];
   const int a0 = blockIdx.x * blockDim.x;
   if (a0 >= e.nf) return;
@@ -2378,21 +2385,42 @@ __global__ void __launch_bounds__(kMaxBlock) k_integrate(const __grid_constant__
 // and potential energy, escapes, clamps, rebuilds, longest row, step, status,
 // obstacle impulse x, c_ref, the correction's log (16-19, written after the
 // update), obstacle impulse y and z, and the clamp impulse xyz.
+// What k_finalize reads of a case.
+struct FinalDev {
+  int adaptive, shift_every, tvc_every, tvc_bulk, comp;
+  double dt, courant_h, c0_d, dt_limit, dt_safety, dt_growth;
+  __device__ __forceinline__ explicit FinalDev(const CaseDev& C)
+      : adaptive(C.adaptive), shift_every(C.shift_every), tvc_every(C.tvc_every), tvc_bulk(C.tvc_bulk), comp(C.comp),
+        dt(C.dt), courant_h(C.courant_h), c0_d(C.c0_d), dt_limit(C.dt_limit), dt_safety(C.dt_safety),
+        dt_growth(C.dt_growth) {}
+};
+
+__device__ __forceinline__ unsigned int remainder_of(unsigned long long step, int m) {
+  return step >> 32 ? static_cast<unsigned int>(step % static_cast<unsigned long long>(m))
+                    : static_cast<unsigned int>(step) % static_cast<unsigned int>(m);
+}
+
+// The case's state is read whole before anything is written (one wait on memory
+// instead of one per field behind each store), with 32-bit remainders: 8.1 -> 3.3
+// us for one case, 13.4 -> 6.6 for 64.
 __global__ void k_finalize(Dev e) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= e.n_slots) return;
-  CaseCtl& t = e.ctl[c];
+  CaseCtl& out = e.ctl[c];
+  const CaseCtl t = out;
   if (!t.active) return;
-  const CaseDev& C = e.cases[c];
+  const FinalDev C(e.cases[c]);
   const unsigned long long step = t.steps;
-  double* row = e.diag + (static_cast<int64_t>(c) * e.diag_ring + static_cast<int64_t>(step % e.diag_ring)) * kDiag;
+  double* row = e.diag + (static_cast<int64_t>(c) * e.diag_ring + static_cast<int64_t>(remainder_of(step, e.diag_ring))) *
+                             kDiag;
   const double vmax = __longlong_as_double(static_cast<long long>(t.speed_max));
   row[0] = __longlong_as_double(static_cast<long long>(t.rho_max));
   row[1] = vmax;
   row[2] = __longlong_as_double(static_cast<long long>(t.front_max));
+  double impulse[3];
   for (int k = 0; k < 3; ++k) {
     row[3 + k] = t.force[k];
-    t.impulse[k] += t.force[k] * (C.adaptive ? t.dt_int : C.dt);
+    out.impulse[k] = impulse[k] = t.impulse[k] + t.force[k] * (C.adaptive ? t.dt_int : C.dt);
   }
   row[6] = t.ke;
   row[7] = t.pe;
@@ -2402,22 +2430,24 @@ __global__ void k_finalize(Dev e) {
   row[11] = static_cast<double>(t.row_max);
   row[12] = static_cast<double>(step);
   row[13] = static_cast<double>(t.status);
-  row[14] = t.impulse[0];
+  row[14] = impulse[0];
   row[15] = t.cref[0];
-  t.cref[1] = vmax;  // the shift's reference speed
-  t.steps = step + 1;
+  out.cref[1] = vmax;  // the shift's reference speed
+  out.steps = step + 1;
   // an adaptive case's final step records its meters and moves nothing
   const bool moves = !C.adaptive || t.dt_int > 0.0;
-  t.shift_now = moves && C.shift_every > 0 && step > 0 && (step % static_cast<unsigned long long>(C.shift_every)) == 0;
-  t.shift_done = 0;
-  t.tvc_now = moves && C.tvc_every > 0 && step > 0 && (step % static_cast<unsigned long long>(C.tvc_every)) == 0;
-  t.conc_now = t.shift_now || (t.tvc_now && C.tvc_bulk);
-  t.tvc_max = 0;
-  t.tvc_sum = 0.0;
-  t.tvc_kept = t.tvc_clipped = 0;
+  const bool shift = moves && C.shift_every > 0 && step > 0 && remainder_of(step, C.shift_every) == 0;
+  const bool tvc = moves && C.tvc_every > 0 && step > 0 && remainder_of(step, C.tvc_every) == 0;
+  out.shift_now = shift;
+  out.shift_done = 0;
+  out.tvc_now = tvc;
+  out.conc_now = shift || (tvc && C.tvc_bulk);
+  out.tvc_max = 0;
+  out.tvc_sum = 0.0;
+  out.tvc_kept = out.tvc_clipped = 0;
   row[16] = row[17] = row[18] = row[19] = 0.0;
-  row[20] = t.impulse[1];
-  row[21] = t.impulse[2];
+  row[20] = impulse[1];
+  row[21] = impulse[2];
   // k_integrate ran before this kernel: the clamp impulse through this
   // step's update, like the obstacle impulse through this step's force
   for (int k = 0; k < 3; ++k) row[22 + k] = t.clamp_impulse[k];
@@ -2427,13 +2457,13 @@ __global__ void k_finalize(Dev e) {
   row[27] = C.adaptive ? t.dt_now : C.dt;
   row[28] = C.comp ? t.comp_written : 0.0;
   row[29] = C.comp ? static_cast<double>(t.comp_counted) : 0.0;
-  t.elapsed += t.dt_int;
+  out.elapsed = t.elapsed + t.dt_int;
   if (C.adaptive && t.dt_int > 0.0) {
     // next_dt (droplet_impact.py:522-556) with the speed at the step's start
     const double stable = fmin(C.courant_h / (C.c0_d + fmax(0.0, vmax)), C.dt_limit);
     const double target = C.dt_safety * stable;
     const double grown = C.dt_growth >= 1.0 ? t.dt_now * C.dt_growth : target;
-    t.dt_now = fmin(fmin(target, grown), C.dt);
+    out.dt_now = fmin(fmin(target, grown), C.dt);
   }
 }
 
