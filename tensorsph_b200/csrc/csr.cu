@@ -26,11 +26,11 @@
 //
 // What bounds the first route: the L2 atomics of A (one per pair) with the
 // scattered 4-byte stores behind them, instruction issue and the copies' loads
-// in B.  18.6 M pairs of a periodic column (480 k rows): A 0.18, scan 0.01,
+// in B.  18.6 M pairs of a periodic column (480 k rows): A 0.17, scan 0.01,
 // B 0.14 ms; counting first (0.13), filling by another pass over the list (0.15)
 // and sorting (0.11) took 0.41, the second route with a rank sort of whole rows
 // 1.2 ms.  13.1 M pairs of a block in mixed order 0.31 against 0.45, 10.6 M of a
-// 2-D column (1.04 M rows) 0.24 against 0.26.  The copies in a launch of their own
+// 2-D column (1.04 M rows) 0.23 against 0.26.  The copies in a launch of their own
 // (0.09) or 32 pairs at a time (0.07 more than 128) lose to B's.
 #include <algorithm>
 
@@ -42,7 +42,10 @@ namespace {
 
 constexpr uint32_t kSecond = 0x80000000u;
 constexpr int kBlock = 256;
-// One pair per thread: the loads of a warp are one contiguous 512-byte run.
+// The loads of a warp are one contiguous 512-byte run.  A thread of list_place takes
+// two pairs, so that two atomics are on their way (18.6 M pairs 178 -> 166 us, 10.6 M
+// 2-D ones 97 -> 85, the same in mixed order; four: 170, 94 and 6 % slower there).
+constexpr int kPairs = 2;
 
 enum { kBad = 1, kUnsorted = 2, kOver = 4 };  // kOver: a row has more second halves than slots
 
@@ -64,29 +67,44 @@ __global__ void __launch_bounds__(kBlock) list_place(const int64_t* __restrict__
                                                      uint32_t* __restrict__ slots, unsigned int per_row,
                                                      unsigned int* found) {
   if (*found & kUnsorted) return;
-  const int64_t p = static_cast<int64_t>(blockIdx.x) * kBlock + threadIdx.x;
-  if (p >= npairs) return;
-  const longlong2 me = ld_pair<kWide>(pairs, p);
-  const int64_t i = me.x, j = me.y;
-  if (i < 0 || j < 0 || i >= nrows || j >= nrows) {
-    atomicOr(found, kBad);
-    return;
+  const int64_t p0 = static_cast<int64_t>(blockIdx.x) * (kPairs * kBlock) + threadIdx.x;
+  longlong2 me[kPairs], prev[kPairs];
+#pragma unroll
+  for (int u = 0; u < kPairs; ++u) {
+    const int64_t p = p0 + u * kBlock;
+    me[u] = p < npairs ? ld_pair<kWide>(pairs, p) : make_longlong2(-1, -1);
+    prev[u] = p > 0 && p < npairs ? ld_pair<kWide>(pairs, p - 1) : make_longlong2(-1, -1);
   }
-  const longlong2 prev = p > 0 ? ld_pair<kWide>(pairs, p - 1) : make_longlong2(-1, -1);
-  if (prev.x > i || (prev.x == i && prev.y > j)) {
-    atomicOr(found, kUnsorted);
-    return;
+  unsigned int s[kPairs];
+#pragma unroll
+  for (int u = 0; u < kPairs; ++u) {
+    const int64_t p = p0 + u * kBlock;
+    s[u] = 0xffffffffu;
+    if (p >= npairs) continue;
+    const int64_t i = me[u].x, j = me[u].y;
+    if (i < 0 || j < 0 || i >= nrows || j >= nrows) {
+      atomicOr(found, kBad);
+      continue;
+    }
+    if (prev[u].x > i || (prev[u].x == i && prev[u].y > j)) {
+      atomicOr(found, kUnsorted);
+      continue;
+    }
+    s[u] = atomicAdd(&second[j], 1u);
+    if (prev[u].x != i) {
+      run[i].x = static_cast<int>(p);
+      if (prev[u].x >= 0 && prev[u].x < nrows) run[prev[u].x].y = static_cast<int>(p);
+    }
+    if (p == npairs - 1) run[i].y = static_cast<int>(npairs);
   }
-  if (prev.x != i) {
-    run[i].x = static_cast<int>(p);
-    if (prev.x >= 0 && prev.x < nrows) run[prev.x].y = static_cast<int>(p);
+#pragma unroll
+  for (int u = 0; u < kPairs; ++u) {
+    if (s[u] == 0xffffffffu) continue;
+    if (s[u] < per_row)
+      slots[me[u].y * per_row + s[u]] = static_cast<uint32_t>(me[u].x) | kSecond;
+    else if (s[u] == per_row)
+      atomicOr(found, kOver);
   }
-  if (p == npairs - 1) run[i].y = static_cast<int>(npairs);
-  const unsigned int s = atomicAdd(&second[j], 1u);
-  if (s < per_row)
-    slots[j * per_row + s] = static_cast<uint32_t>(i) | kSecond;
-  else if (s == per_row)
-    atomicOr(found, kOver);
 }
 
 __global__ void list_rows(const int2* __restrict__ run, const unsigned int* __restrict__ second, int64_t nrows,
@@ -234,7 +252,7 @@ int rows_of_sorted(const int64_t* pairs, int64_t npairs, int64_t nrows, int64_t*
   TSPH_CUDA_CHECK(cudaMemsetAsync(run, 0, nrows * sizeof(int2), s));
   TSPH_CUDA_CHECK(cudaMemsetAsync(w.second, 0, (nrows + 1) * sizeof(unsigned int), s));
   const unsigned g = static_cast<unsigned>((npairs + kBlock - 1) / kBlock);
-  list_place<kWide><<<g, kBlock, 0, s>>>(pairs, npairs, nrows, run, w.second, w.slots, per_row, w.found);
+  list_place<kWide><<<static_cast<unsigned>((npairs + kPairs * kBlock - 1) / (kPairs * kBlock)), kBlock, 0, s>>>(pairs, npairs, nrows, run, w.second, w.slots, per_row, w.found);
   TSPH_LAUNCH_CHECK();
   unsigned int found = 0;
   int rc = read_found(w.found, &found, s);
