@@ -12,8 +12,8 @@
 //   bounds -> [host: grid]
 //   cell_count   key of every particle, its slot in its cell by an atomic
 //   scan         first sorted position of every cell
-//   cell_scatter a 16-byte record (x, y, z in FP32 from the grid's corner, id)
-//                per particle, cell by cell
+//   cell_scatter a 16-byte record (x, y, z in FP32 from the grid's corner, in
+//                cutoffs, and id) per particle, cell by cell
 //   scan_rows    per particle (in cell order) the neighbours among the
 //                candidates of its 3^D cells, into a fixed number of slots
 //   scan -> [host: list length]
@@ -44,6 +44,8 @@ struct GridDev {
   int64_t stride[kMaxDim];
   int64_t origin[kMaxDim];
   double cutoff, box[kMaxDim], width[kMaxDim];
+  double scale;          // records = lengths * scale: 1 / cutoff, or 0 (band_of)
+  float edge[kMaxDim];   // periodic box edges in records
 };
 
 struct BuildWs {
@@ -51,7 +53,7 @@ struct BuildWs {
   uint64_t* keys_tmp;  // n
   int32_t* order;      // n, sorted: the particle (dense: in 3-D)
   int32_t* order_tmp;  // n
-  float* rec;          // n, sorted: position from the grid's corner (rec_at)
+  float* rec;          // n, sorted: position from the grid's corner, in cutoffs (rec_at)
   int32_t* cell;       // n * dim, sorted: cell coordinates relative to origin
   int32_t* counts;     // total_cells (dense) or 0, then
   int32_t* longest;    // 1: 0, or the longest row when it has outgrown its slots
@@ -115,8 +117,45 @@ __device__ __forceinline__ int64_t rec_at(int64_t t) {
 template <int D>
 constexpr int kRecStep = D == 3 ? 4 : 1;
 
+// Which candidates the FP32 records decide.  Records are in units of the cutoff:
+// in the caller's units a squared FP32 distance overflows beyond 1.8e19 and
+// vanishes below 1e-23.  A record's coordinate is within 2^-24 of the extent of
+// its true value (and so is an image's shift), so a distance taken from two of
+// them in FP32, and the reference's own distance in its dtype, differ by less
+// than w = 2^-20 extent + 2e-6.  Below (1 - w)^2 a candidate is in, above
+// (1 + w)^2 it is out; between them (about one candidate in 10^4) the
+// reference's arithmetic on the given positions decides.  It decides for every
+// candidate where the band would be wide (a grid of many thousand cells on an
+// axis, or positions as many cutoffs outside their box), where a periodic axis
+// has three cells, so that a stencil cell's image need not be the nearest one,
+// and where the square of the cutoff leaves the dtype's range: the records are
+// zero then, which lies between the bounds.
+struct Band {
+  float in, out;
+  bool exact;
+};
+
+Band band_of(const tsph_grid& g) {
+  const double c2 = g.cutoff * g.cutoff, far = g.dtype == TSPH_F32 ? 1e30 : 1e280;
+  double extent = 0.0;
+  bool exact = !(c2 > 1.0 / far && c2 < far);
+  for (int k = 0; k < g.dim; ++k) {
+    if (g.periodic) {
+      extent = std::max(extent, std::max(g.box[k] / g.cutoff, 2.0 * static_cast<double>(g.origin[k])));
+      if (g.ncell[k] < 4) exact = true;
+    } else {
+      extent = std::max(extent, static_cast<double>(g.ncell[k]));
+    }
+  }
+  const double w = extent / 1048576.0 + 2e-6;
+  if (exact || !(w < 0.25)) return Band{-1.f, 1.f, true};
+  return Band{static_cast<float>((1.0 - w) * (1.0 - w) * (1.0 - 1e-6)),
+              static_cast<float>((1.0 + w) * (1.0 + w) * (1.0 + 1e-6)), false};
+}
+
 GridDev to_dev(const tsph_grid& g) {
   GridDev d{};
+  d.scale = band_of(g).exact ? 0.0 : 1.0 / g.cutoff;
   d.dim = static_cast<int>(g.dim);
   d.periodic = static_cast<int>(g.periodic);
   d.dense = static_cast<int>(g.dense);
@@ -126,6 +165,7 @@ GridDev to_dev(const tsph_grid& g) {
     d.origin[k] = g.origin[k];
     d.box[k] = g.box[k];
     d.width[k] = g.width[k];
+    d.edge[k] = static_cast<float>(g.box[k] * d.scale);
   }
   int64_t s = 1;
   for (int k = static_cast<int>(g.dim) - 1; k >= 0; --k) {
@@ -206,8 +246,12 @@ int plan_bounds(const void* pos, int64_t n, double cutoff, unsigned long long* d
 // ----------------------------------------------------------------- build ---
 
 // Cell of one coordinate (relative to the grid's origin, or wrapped into the
-// box) and the coordinate from the grid's corner, moved by whole boxes into
-// the same cell when periodic.
+// box) and its record: the coordinate from the grid's corner, moved by whole
+// boxes into the same cell when periodic, in cutoffs.
+__device__ __forceinline__ float record(double length, double scale) {
+  return scale == 0.0 ? 0.f : static_cast<float>(length * scale);
+}
+
 template <class T>
 __device__ __forceinline__ long long cell_of(T x, const GridDev& g, int k, float* local) {
   if (g.periodic) {
@@ -215,11 +259,11 @@ __device__ __forceinline__ long long cell_of(T x, const GridDev& g, int k, float
     long long c = raw % g.ncell[k];
     if (c < 0) c += g.ncell[k];
     if (local)
-      *local = static_cast<float>(static_cast<double>(x) - static_cast<double>((raw - c) / g.ncell[k]) *
-                                                               static_cast<double>(static_cast<T>(g.box[k])));
+      *local = record(static_cast<double>(x) - static_cast<double>((raw - c) / g.ncell[k]) *
+                                                   static_cast<double>(static_cast<T>(g.box[k])), g.scale);
     return c;
   }
-  if (local) *local = static_cast<float>(static_cast<double>(x) - static_cast<double>(g.origin[k]) * g.cutoff);
+  if (local) *local = record(static_cast<double>(x) - static_cast<double>(g.origin[k]) * g.cutoff, g.scale);
   return static_cast<long long>(floor(fp<T>::div(x, static_cast<T>(g.cutoff)))) - g.origin[k];
 }
 
@@ -307,38 +351,6 @@ __device__ __forceinline__ T pair_d2(const T* __restrict__ pos, int64_t a, int64
     acc = k == 0 ? sq : fp<T>::add(acc, sq);
   }
   return acc;
-}
-
-// Which candidates the FP32 records decide.  A record's coordinate is within
-// 2^-24 of the extent of its true value (and so is an image's shift), so a
-// distance taken from two of them in FP32, and the reference's own distance in
-// its dtype, differ by less than w = 2^-20 extent + 2e-6 cutoff.  Below
-// (cutoff - w)^2 a candidate is in, above (cutoff + w)^2 it is out; between
-// them (about one candidate in 10^4) the reference's arithmetic on the given
-// positions decides.  Where the band would be wide (coordinates many thousand
-// cutoffs from the corner), or a periodic axis has three cells, so that a
-// stencil cell's image need not be the nearest one, every candidate takes the
-// reference's arithmetic.
-struct Band {
-  float in, out;
-};
-
-Band band_of(const tsph_grid& g) {
-  double extent = 0.0;
-  bool exact = false;
-  for (int k = 0; k < g.dim; ++k) {
-    if (g.periodic) {
-      extent = std::max(extent, std::max(g.box[k], 2.0 * static_cast<double>(g.origin[k]) * g.cutoff));
-      if (g.ncell[k] < 4) exact = true;
-    } else {
-      extent = std::max(extent, static_cast<double>(g.ncell[k]) * g.cutoff);
-    }
-  }
-  const double w = extent / 1048576.0 + 2e-6 * g.cutoff;
-  if (exact || !(w < 0.25 * g.cutoff) || g.cutoff * g.cutoff < 1e-30 || extent > 1e15)
-    return Band{-1.f, INFINITY};
-  const double lo = g.cutoff - w, hi = g.cutoff + w;
-  return Band{static_cast<float>(lo * lo * (1.0 - 1e-6)), static_cast<float>(hi * hi * (1.0 + 1e-6))};
 }
 
 struct Cells {
@@ -560,8 +572,8 @@ __global__ void __launch_bounds__(128) scan_rows(const T* __restrict__ pos, int6
     for (int k = 0; k + 1 < D; ++k) {
       int64_t nc = c[k] + off[k];
       if (g.periodic) {
-        if (nc < 0) { nc += g.ncell[k]; x[k] += static_cast<float>(g.box[k]); }
-        else if (nc >= g.ncell[k]) { nc -= g.ncell[k]; x[k] -= static_cast<float>(g.box[k]); }
+        if (nc < 0) { nc += g.ncell[k]; x[k] += g.edge[k]; }
+        else if (nc >= g.ncell[k]) { nc -= g.ncell[k]; x[k] -= g.edge[k]; }
       } else if (nc < 0 || nc >= g.ncell[k]) {
         inside = false;
       }
@@ -572,7 +584,7 @@ __global__ void __launch_bounds__(128) scan_rows(const T* __restrict__ pos, int6
     const int64_t z0 = c[D - 1] > 0 ? c[D - 1] - 1 : 0, z1 = c[D - 1] < last ? c[D - 1] + 1 : last;
     cells(column + z0, column + z1, x[0], x[1], x[2]);
     if (g.periodic) {
-      const float edge = static_cast<float>(g.box[D - 1]);
+      const float edge = g.edge[D - 1];
       if (c[D - 1] == 0) {
         x[D - 1] += edge;
         cells(column + last, column + last, x[0], x[1], x[2]);

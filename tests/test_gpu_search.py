@@ -141,3 +141,24 @@ def test_runs_of_any_length(gpu, dtype, box, lattice_points, offset):
     if box is None:
         (ptr, entries, count), (ptr2, entries2), _ = rows_and_pairs(pos, cutoff, pos.shape[0] // 2, gpu)
         assert torch.equal(ptr, ptr2) and torch.equal(entries[:count], entries2[:count])
+
+
+@pytest.mark.parametrize("dtype,scale", [(np.float64, 1e-100), (np.float64, 1e-25), (np.float64, 1e-12), (np.float64, 1e18),
+                                         (np.float64, 1e20), (np.float64, 1e30), (np.float64, 1e45), (np.float64, 1e145),
+                                         (np.float32, 1e-20), (np.float32, 1e-12), (np.float32, 1e14), (np.float32, 1e20)])
+@pytest.mark.parametrize("counts", [(300,), (30000,), (24, 25), (160, 161), (8, 9, 10), (30, 30, 29)])
+def test_any_unit_of_length(gpu, dtype, scale, counts):
+    """Lengths whose squares leave the range of FP32, or of the positions' own dtype, on
+    both sides of the row count that switches lanes per row: lists, periodic lists, rows."""
+    pos = (lattice(counts, 1.0, np.float64, 0.2) * scale).astype(dtype)
+    pos = pos[np.random.default_rng(3).permutation(pos.shape[0])]
+    cutoff = 1.3 * scale
+    with np.errstate(over="ignore", under="ignore"):
+        want = on.cell_linked_pairs_batched(pos, cutoff)
+        box = [c * scale for c in counts]
+        periodic = on.periodic_pairs(pos, box, cutoff) if pos.shape[0] < 1000 else None
+    assert np.array_equal(search(pos, cutoff, gpu), want)
+    if periodic is not None:
+        assert np.array_equal(search(pos, cutoff, gpu, box), periodic)
+    (ptr, entries, count), (ptr2, entries2), _ = rows_and_pairs(pos, cutoff, pos.shape[0] // 2, gpu)
+    assert torch.equal(ptr, ptr2) and torch.equal(entries[:count], entries2[:count])
