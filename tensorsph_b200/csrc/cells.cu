@@ -612,7 +612,11 @@ __global__ void __launch_bounds__(128) scan_rows(const T* __restrict__ pos, int6
 // chip idle there, eight lanes leave a sixth of theirs idle in every run.  Whole
 // searches (FP32, 3-D, 2.05 h) with eight lanes / one: 8 k particles 132 / 156
 // us, 20 k 137 / 144, 40 k 177 / 154, 100 k 281 / 205; 2-D: the same up to 20 k,
-// 123 / 116 at 40 k.
+// 123 / 116 at 40 k.  Where every candidate takes the exact arithmetic, a thread
+// looks at its candidates one by one, and eight lanes pay at any number of rows
+// (FP32, three cells on two axes: 60 k rows of ~70 neighbours 366 / 488 us, of ~550
+// 2.9 / 4.5 ms; on all three axes 30 k rows of ~2900 22.8 / 45.2 ms), unless the cells
+// are found by bisection, which each lane would repeat (97 k rows 601 / 392 us).
 constexpr int64_t kLaneRows = 24576;
 
 template <class T, int D, RowKind kKind, RowPass kPass>
@@ -623,12 +627,13 @@ int launch_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, const
   const T c2 = static_cast<T>(grid.cutoff * grid.cutoff);
   const T* p = static_cast<const T*>(pos);
   const int slots = static_cast<int>(row_slots(grid));
-  if (n <= kLaneRows)
+  const Band band = band_of(grid);
+  if (n <= kLaneRows || (band.exact && grid.dense))
     scan_rows<T, D, kKind, kPass, 8><<<static_cast<unsigned>((n * 8 + 127) / 128), 128, 0, s>>>(
-        p, n, row_limit, to_dev(grid), cs, band_of(grid), c2, w.rowcount, rowptr, out, slots, w.longest);
+        p, n, row_limit, to_dev(grid), cs, band, c2, w.rowcount, rowptr, out, slots, w.longest);
   else
     scan_rows<T, D, kKind, kPass, 1><<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(
-        p, n, row_limit, to_dev(grid), cs, band_of(grid), c2, w.rowcount, rowptr, out, slots, w.longest);
+        p, n, row_limit, to_dev(grid), cs, band, c2, w.rowcount, rowptr, out, slots, w.longest);
   TSPH_LAUNCH_CHECK();
   return TSPH_OK;
 }

@@ -162,3 +162,21 @@ def test_any_unit_of_length(gpu, dtype, scale, counts):
         assert np.array_equal(search(pos, cutoff, gpu, box), periodic)
     (ptr, entries, count), (ptr2, entries2), _ = rows_and_pairs(pos, cutoff, pos.shape[0] // 2, gpu)
     assert torch.equal(ptr, ptr2) and torch.equal(entries[:count], entries2[:count])
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [24576, 24577, 30001])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_exact_grids_of_many_rows(gpu, dtype, n, dim):
+    """Three periodic cells on an axis (every candidate takes the exact arithmetic) and a
+    cloud with a far clump (the same, cells by bisection), on both sides of the row count
+    that switches lanes per row elsewhere."""
+    rng = np.random.default_rng(n)
+    box = [1.0] * (dim - 1) + [n / 3.0 ** dim / 12]
+    pos = (rng.random((n, dim)) * box).astype(dtype)
+    assert np.array_equal(search(pos, 0.333, gpu, box), on.periodic_pairs(pos, box, 0.333))
+    side = int(np.ceil(n ** (1.0 / dim)))
+    pos = lattice((side,) * dim, 1.0, np.float64, 0.2)[:n]
+    pos[-64:, 0] += 1.0e6
+    pos = pos.astype(dtype)[rng.permutation(n)]
+    assert np.array_equal(search(pos, 1.6, gpu), on.cell_linked_pairs_batched(pos, 1.6))
