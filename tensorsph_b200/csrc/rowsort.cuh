@@ -191,11 +191,12 @@ __global__ void __launch_bounds__(kSortBlock, 8) rows_sort(Rows rows, int64_t n,
 
 // The rows beyond kGroupRow: mid rows by one warp each (entry = register * 32 +
 // lane of the sorted order, as above with 32 lanes), longer ones by one block
-// each, in shared memory up to kMediumRow and beyond it directly where they
-// lie.  The global network is the
-// all-ascending form (the first step of each merge pairs t with t ^ (k - 1)),
-// so the minimum always lands on the lower index and the virtual +inf padding
-// beyond `len` never moves.
+// each, in shared memory up to kMediumRow and beyond it where they lie: stretches
+// of kMediumRow in shared memory, and directly only the steps between stretches
+// (21 of the 190 steps of 300 k entries, which bound such a row: 32.4 ms with all of
+// them in global memory).  The network is the all-ascending form (the first step of
+// each merge pairs t with t ^ (k - 1)), so the minimum always lands on the lower
+// index and the virtual +inf padding beyond `len` never moves.
 template <class Rows, class Out>
 __global__ void __launch_bounds__(kRestBlock, 1) rows_sort_rest(Rows rows, Out out, LongRows lists) {
   __shared__ uint32_t buf[kMediumRow];
@@ -214,41 +215,58 @@ __global__ void __launch_bounds__(kRestBlock, 1) rows_sort_rest(Rows rows, Out o
     for (int i = 0; i < 32; ++i)
       if (lane * 32 + i < len) out(r, dst + lane * 32 + i, v[i]);
   }
+  // the steps of merge k at distances j, j / 2, .., 1 over buf[0, p2)
+  auto merge = [&](int k, int j, int p2) {
+    for (; j > 0; j >>= 1) {
+      const int mask = 2 * j == k ? k - 1 : j;
+      for (int t = threadIdx.x; t < p2; t += blockDim.x) {
+        const int u = t ^ mask;
+        if (u > t) {
+          const uint32_t x = buf[t], y = buf[u];
+          if (x > y) { buf[t] = y; buf[u] = x; }
+        }
+      }
+      __syncthreads();
+    }
+  };
+  auto load = [&](const uint32_t* a, int64_t len, int p2) {
+    for (int t = threadIdx.x; t < p2; t += blockDim.x) buf[t] = t < len ? a[t] : 0xffffffffu;
+    __syncthreads();
+  };
   for (int64_t q = blockIdx.x; q < bigs; q += gridDim.x) {
     const int64_t r = lists.big[q], dst = rows.dst(r), len = rows.len(r);
     uint32_t* a = rows.src(r);
     int64_t p2 = 1;
     while (p2 < len) p2 <<= 1;
     if (len <= kMediumRow) {
-      for (int t = threadIdx.x; t < p2; t += blockDim.x) buf[t] = t < len ? a[t] : 0xffffffffu;
-      __syncthreads();
-      for (int k = 2; k <= p2; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-          for (int t = threadIdx.x; t < p2; t += blockDim.x) {
-            const int ixj = t ^ j;
-            if (ixj > t) {
-              const bool up = (t & k) == 0;
-              const uint32_t x = buf[t], y = buf[ixj];
-              if ((x > y) == up) { buf[t] = y; buf[ixj] = x; }
-            }
-          }
-          __syncthreads();
-        }
-      }
+      load(a, len, static_cast<int>(p2));
+      for (int k = 2; k <= p2; k <<= 1) merge(k, k >> 1, static_cast<int>(p2));
       for (int t = threadIdx.x; t < len; t += blockDim.x) out(r, dst + t, buf[t]);
     } else {
-      for (int64_t k = 2; k <= p2; k <<= 1) {
-        for (int64_t j = k >> 1; j > 0; j >>= 1) {
+      auto stretches = [&](auto&& steps) {
+        for (int64_t b = 0; b < len; b += kMediumRow) {
+          load(a + b, len - b, kMediumRow);
+          steps();
+          for (int t = threadIdx.x; t < kMediumRow && t < len - b; t += blockDim.x) a[b + t] = buf[t];
+          __syncthreads();
+        }
+      };
+      stretches([&] {
+        for (int k = 2; k <= kMediumRow; k <<= 1) merge(k, k >> 1, kMediumRow);
+      });
+      for (int64_t k = 2 * kMediumRow; k <= p2; k <<= 1) {
+        for (int64_t j = k >> 1; j >= kMediumRow; j >>= 1) {
           const int64_t mask = (j == (k >> 1)) ? (k - 1) : j;
           for (int64_t t = threadIdx.x; t < p2; t += blockDim.x) {
-            const int64_t ixj = t ^ mask;
-            if (ixj > t && t < len && ixj < len) {
-              const uint32_t x = a[t], y = a[ixj];
-              if (x > y) { a[t] = y; a[ixj] = x; }
+            const int64_t u = t ^ mask;
+            if (u > t && t < len && u < len) {
+              const uint32_t x = a[t], y = a[u];
+              if (x > y) { a[t] = y; a[u] = x; }
             }
           }
           __syncthreads();
         }
+        stretches([&] { merge(0, kMediumRow >> 1, kMediumRow); });
       }
       for (int64_t t = threadIdx.x; t < len; t += blockDim.x) out(r, dst + t, a[t]);
     }

@@ -102,3 +102,15 @@ def test_rows_without_memory_for_slots(gpu, monkeypatch):
     p = np.sort(np.random.default_rng(0).integers(0, 500, (9000, 2)), axis=1)
     check(p[np.lexsort((p[:, 1], p[:, 0]))], 500, gpu)
     assert refused
+
+
+@pytest.mark.parametrize("count", [8191, 8192, 8193, 16383, 16384, 16385, 24577, 40000, 131073])
+def test_rows_beyond_shared_memory(gpu, count):
+    """Two rows sorted by stretches of 8192 entries, in arbitrary order and with repeats; the
+    list sorted and shuffled."""
+    rng = np.random.default_rng(count)
+    n = count + 2
+    p = np.concatenate((np.stack((rng.integers(0, n - 2, count), np.full(count, n - 1)), axis=1),
+                        np.stack((rng.permutation(n - 2)[:count], np.full(count, n - 2)), axis=1)))
+    check(rng.permutation(p), n, gpu)
+    check(p[np.lexsort((p[:, 1], p[:, 0]))], n, gpu)
