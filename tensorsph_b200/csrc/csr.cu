@@ -56,24 +56,31 @@ __device__ __forceinline__ longlong2 ld_pair(const int64_t* __restrict__ pairs, 
   return make_longlong2(pairs[2 * p], pairs[2 * p + 1]);
 }
 
-// A: with `found` already raised by an earlier block the rest of the grid
-// returns at once (an unsorted list is seen within its first pairs).  The read
-// goes through the L1, so a block may still miss the flag; it is no more than a
-// short cut, and the host reads the flag after the kernel.
-template <bool kWide>
+// Lists of up to this many pairs also count the rows' degrees in A, so that an
+// unsorted one needs no second count (whole calls: 500 pairs 92 -> 70 us, 100 k 102 ->
+// 82; sorted ones the same within 1 us up to here).  A longer unsorted one pays A for
+// finding out: 1.0 M pairs 145 us, 140 by the general route alone.
+constexpr int64_t kSmallList = 131072;
+
+// A: with the list found unsorted by an earlier block the rest of the grid only
+// looks at the indices' range (an unsorted list is seen within its first pairs), so
+// that the host waits once for either route.  The read of `found` goes through the
+// L1, so a block may still miss the flag; it is no more than a short cut, and the
+// host reads the flags after the kernel.
+template <bool kWide, bool kDegrees>
 __global__ void __launch_bounds__(kBlock) list_place(const int64_t* __restrict__ pairs, int64_t npairs,
                                                      int64_t nrows, int2* __restrict__ run,
-                                                     unsigned int* __restrict__ second,
+                                                     int32_t* __restrict__ deg, unsigned int* __restrict__ second,
                                                      uint32_t* __restrict__ slots, unsigned int per_row,
                                                      unsigned int* found) {
-  if (*found & kUnsorted) return;
+  const bool range_only = !kDegrees && (*found & kUnsorted);
   const int64_t p0 = static_cast<int64_t>(blockIdx.x) * (kPairs * kBlock) + threadIdx.x;
   longlong2 me[kPairs], prev[kPairs];
 #pragma unroll
   for (int u = 0; u < kPairs; ++u) {
     const int64_t p = p0 + u * kBlock;
     me[u] = p < npairs ? ld_pair<kWide>(pairs, p) : make_longlong2(-1, -1);
-    prev[u] = p > 0 && p < npairs ? ld_pair<kWide>(pairs, p - 1) : make_longlong2(-1, -1);
+    prev[u] = !range_only && p > 0 && p < npairs ? ld_pair<kWide>(pairs, p - 1) : make_longlong2(-1, -1);
   }
   unsigned int s[kPairs];
 #pragma unroll
@@ -85,6 +92,11 @@ __global__ void __launch_bounds__(kBlock) list_place(const int64_t* __restrict__
     if (i < 0 || j < 0 || i >= nrows || j >= nrows) {
       atomicOr(found, kBad);
       continue;
+    }
+    if (range_only) continue;
+    if (kDegrees) {
+      atomicAdd(&deg[i], 1);
+      atomicAdd(&deg[j], 1);
     }
     if (prev[u].x > i || (prev[u].x == i && prev[u].y > j)) {
       atomicOr(found, kUnsorted);
@@ -199,10 +211,10 @@ __global__ void csr_fill(const int64_t* __restrict__ pairs, int64_t npairs, int6
 }
 
 struct CsrWs {
-  int32_t* deg;          // nrows
   int64_t* cursor;       // nrows + 1 (any list); run: int2 per row (sorted list)
-  unsigned int* second;  // nrows
-  unsigned int* found;   // right after `second`: one memset clears both
+  int32_t* deg;          // nrows
+  unsigned int* second;  // nrows, right after `deg`
+  unsigned int* found;   // right after `second`: one memset clears them
   char* scan;
   char* sort;
   uint32_t* slots;       // last, as many per row as the workspace has room for
@@ -226,9 +238,9 @@ size_t csr_layout(int64_t nrows, CsrWs* w, void* base) {
     return p;
   };
   CsrWs t{};
-  t.deg = reinterpret_cast<int32_t*>(take(nrows * sizeof(int32_t)));
   t.cursor = reinterpret_cast<int64_t*>(take((nrows + 1) * sizeof(int64_t)));
-  t.second = reinterpret_cast<unsigned int*>(take((nrows + 1) * sizeof(unsigned int)));
+  t.deg = reinterpret_cast<int32_t*>(take((2 * nrows + 1) * sizeof(int32_t)));
+  t.second = t.deg ? reinterpret_cast<unsigned int*>(t.deg + nrows) : nullptr;
   t.found = t.second ? t.second + nrows : nullptr;
   t.scan = take(scan_scratch_bytes(nrows + 1));
   t.sort = take(segsort_scratch_bytes(nrows));
@@ -244,23 +256,27 @@ int read_found(const unsigned int* found, unsigned int* host, cudaStream_t s) {
 }
 
 // Returns with *taken false, and nothing written to the outputs, when the list
-// is not sorted.
+// is not sorted; w.deg then holds the degrees of a small list's rows.
 template <bool kWide>
 int rows_of_sorted(const int64_t* pairs, int64_t npairs, int64_t nrows, int64_t* rowptr, uint32_t* entries,
                    const CsrWs& w, unsigned int per_row, bool* taken, cudaStream_t s) {
   int2* run = reinterpret_cast<int2*>(w.cursor);
   TSPH_CUDA_CHECK(cudaMemsetAsync(run, 0, nrows * sizeof(int2), s));
-  TSPH_CUDA_CHECK(cudaMemsetAsync(w.second, 0, (nrows + 1) * sizeof(unsigned int), s));
+  const bool small = npairs <= kSmallList;
+  if (small)
+    TSPH_CUDA_CHECK(cudaMemsetAsync(w.deg, 0, (2 * nrows + 1) * sizeof(unsigned int), s));
+  else
+    TSPH_CUDA_CHECK(cudaMemsetAsync(w.second, 0, (nrows + 1) * sizeof(unsigned int), s));
   const unsigned g = static_cast<unsigned>((npairs + kBlock - 1) / kBlock);
-  list_place<kWide><<<static_cast<unsigned>((npairs + kPairs * kBlock - 1) / (kPairs * kBlock)), kBlock, 0, s>>>(pairs, npairs, nrows, run, w.second, w.slots, per_row, w.found);
+  const unsigned gp = static_cast<unsigned>((npairs + kPairs * kBlock - 1) / (kPairs * kBlock));
+  const auto place = small ? list_place<kWide, true> : list_place<kWide, false>;
+  place<<<gp, kBlock, 0, s>>>(pairs, npairs, nrows, run, w.deg, w.second, w.slots, per_row, w.found);
   TSPH_LAUNCH_CHECK();
   unsigned int found = 0;
   int rc = read_found(w.found, &found, s);
-  *taken = true;
-  // an index out of range behind an unsorted stretch is found by the general route
-  if (found & kUnsorted) *taken = false;
-  if (!*taken) return TSPH_OK;
   if (rc) return rc;
+  *taken = !(found & kUnsorted);
+  if (!*taken) return TSPH_OK;
   list_rows<<<static_cast<unsigned>((nrows + kBlock - 1) / kBlock), kBlock, 0, s>>>(run, w.second, nrows, w.deg);
   TSPH_LAUNCH_CHECK();
   rc = exclusive_scan_i32_to_i64(w.deg, rowptr, nrows, rowptr + nrows, w.scan, s);
@@ -301,7 +317,8 @@ int tsph_csr_from_pairs(const int64_t* pairs, int64_t npairs, int64_t nrows, int
     TSPH_CUDA_CHECK(cudaMemsetAsync(rowptr, 0, (nrows + 1) * sizeof(int64_t), s));
     return TSPH_OK;
   }
-  if (npairs < (int64_t(1) << 31)) {
+  const bool checked = npairs < (int64_t(1) << 31);  // by list_place
+  if (checked) {
     bool taken = false;
     const bool wide = reinterpret_cast<uintptr_t>(pairs) % 16 == 0;
     const int64_t room = (ws_bytes - tsph_csr_workspace_bytes(npairs, nrows)) /
@@ -311,13 +328,14 @@ int tsph_csr_from_pairs(const int64_t* pairs, int64_t npairs, int64_t nrows, int
                   : rows_of_sorted<false>(pairs, npairs, nrows, rowptr, entries, w, per_row, &taken, s);
     if (rc || taken) return rc;
   }
-  TSPH_CUDA_CHECK(cudaMemsetAsync(w.deg, 0, nrows * sizeof(int32_t), s));
-  TSPH_CUDA_CHECK(cudaMemsetAsync(w.found, 0, sizeof(unsigned int), s));
-  csr_degree<<<grid_for(npairs, 256), 256, 0, s>>>(pairs, npairs, nrows, w.deg, w.found);
-  TSPH_LAUNCH_CHECK();
-  unsigned int found = 0;
-  int rc = read_found(w.found, &found, s);
-  if (rc) return rc;
+  int rc = TSPH_OK;
+  if (npairs > kSmallList) {
+    TSPH_CUDA_CHECK(cudaMemsetAsync(w.deg, 0, (2 * nrows + 1) * sizeof(int32_t), s));
+    csr_degree<<<grid_for(npairs, 256), 256, 0, s>>>(pairs, npairs, nrows, w.deg, w.found);
+    TSPH_LAUNCH_CHECK();
+    unsigned int found = 0;
+    if (!checked && (rc = read_found(w.found, &found, s))) return rc;
+  }
   rc = exclusive_scan_i32_to_i64(w.deg, rowptr, nrows, rowptr + nrows, w.scan, s);
   if (rc) return rc;
   TSPH_CUDA_CHECK(cudaMemcpyAsync(w.cursor, rowptr, nrows * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));

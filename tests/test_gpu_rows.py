@@ -114,3 +114,25 @@ def test_rows_beyond_shared_memory(gpu, count):
                         np.stack((rng.permutation(n - 2)[:count], np.full(count, n - 2)), axis=1)))
     check(rng.permutation(p), n, gpu)
     check(p[np.lexsort((p[:, 1], p[:, 0]))], n, gpu)
+
+
+@pytest.mark.parametrize("count", [511, 131071, 131072, 131073, 300000])
+def test_rows_where_degrees_are_counted_along(gpu, count):
+    """Sorted and unsorted lists around the size up to which the first pass also counts the
+    degrees, the order broken at the start, in the middle and by the last pair; an index out
+    of range as the last thing in each."""
+    from tensorsph_b200.droplet_impact import symmetric_rows
+    rng = np.random.default_rng(count)
+    n = count // 7
+    p = rng.integers(0, n, (count, 2))
+    p = p[np.lexsort((p[:, 1], p[:, 0]))]
+    p[-1], p[-2] = (n - 1, n - 1), (n - 1, n - 2)
+    for at in (None, 1, count // 2, count - 1):
+        q = p.copy()
+        if at is not None:
+            q[[at - 1, at]] = [[n - 1, 3], [0, 5]]
+        check(q, n, gpu)
+        for bad in (n, -1):
+            q[-1, 1] = bad
+            with pytest.raises(ValueError):
+                symmetric_rows(torch.from_numpy(q).to(gpu), n)
