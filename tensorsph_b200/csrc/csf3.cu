@@ -38,7 +38,7 @@ struct CP {
   int64_t n;
   int periodic, has_volume;
   T box[3], half[3];
-  T rho0, w0, sigma, cutoff;
+  T rho0, sigma, cutoff;
   Cubic<T> k;
 };
 
@@ -86,7 +86,8 @@ __global__ void c_pack(CP<T> p, const T* __restrict__ pos, const T* __restrict__
   }
 }
 
-// C1: colour, M (symmetric, 6 values) and |det M| (as its IEEE bits for the select)
+// C1: colour (a sum of shapes, times sigma in two floats: the rounding of a single
+// sigma is common to all rows of a call), M (symmetric, 6 values) and |det M| (as its IEEE bits for the select)
 template <class T, int L>
 __global__ void __launch_bounds__(kGatherBlock) c_colour(CP<T> p, const Q4<T>* __restrict__ pv,
                                                          const int64_t* __restrict__ rowptr,
@@ -101,10 +102,11 @@ __global__ void __launch_bounds__(kGatherBlock) c_colour(CP<T> p, const Q4<T>* _
   CSum<T> m[6];
   me.walk_ahead(ent, rowptr[a], rowptr[a + 1], [&](uint32_t e) {
     const Q4<T> pb = pv[e & kIndexMask];
-    T d[3], w, g;
+    T d[3];
     sep(pa, pb, p, d);
-    p.k.wg2(norm2(d), w, g);
-    c.add(pb.w * w);
+    const auto R = p.k.radial(norm2(d));
+    const T g = p.k.g2(R);
+    c.add(pb.w * p.k.shape(R.q));
     // V_b (x_b - x_a) (x) grad_a W = -V_b g d (x) d
     const T s = -pb.w * g;
     m[0].add(s * d[0] * d[0]);
@@ -114,8 +116,8 @@ __global__ void __launch_bounds__(kGatherBlock) c_colour(CP<T> p, const Q4<T>* _
     m[4].add(s * d[1] * d[2]);
     m[5].add(s * d[2] * d[2]);
   });
-  if (me.lane == 0) c.add(pa.w * p.w0);
-  const T cv = me.sum(c);
+  if (me.lane == 0) c.add(pa.w);  // W(0) = sigma
+  const T cv = p.k.times_sigma(me.total(c));
   T mv[6];
 #pragma unroll
   for (int k = 0; k < 6; ++k) mv[k] = me.sum(m[k]);
@@ -351,7 +353,6 @@ CP<T> make_cp(const tsph_csf3_params& prm) {
   }
   p.rho0 = static_cast<T>(prm.rho0);
   const double sigma3 = 1.0 / (M_PI * prm.h * prm.h * prm.h);
-  p.w0 = static_cast<T>(sigma3);
   p.sigma = static_cast<T>(prm.sigma);
   p.cutoff = static_cast<T>(prm.cutoff);
   p.k = make_cubic<T>(prm.h, sigma3);

@@ -132,3 +132,24 @@ def test_csf3_axisym_matches_reference(golden, gpu):
         acc = surface_tension_acceleration3(st, dev(g[f"c{k}_rho"]), 0.0728).cpu().numpy()
         ra = g[f"c{k}_acc"]
         assert np.abs(acc - ra).max() <= tol * np.abs(ra).max(), k
+
+
+@pytest.mark.parametrize("dx", [0.01, 0.0138, 0.03])
+def test_csf3_fp32_colour_has_no_common_error(gpu, dx):
+    """FP32 colours lie about the 64-bit ones: rounding a single sigma = 1 / (pi h^3), by 2.7 to
+    4.0e-8 here, would shift every colour of a call.  The volumes are exact (m / rho0 = 2^-20),
+    there is no box (whose own rounding to FP32 does shift the pairs across it), and what is left
+    rounds either way: the mean of the relative errors of 5832 rows is below a sixth of FP32's half
+    ulp."""
+    from tensorsph_b200.neighbor_search import cell_linked_pairs
+    from tensorsph_b200.threed.csf3 import csf_fields3
+    side = 18
+    g = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    rng = np.random.default_rng(4)
+    x = torch.from_numpy((g + 0.5 + 0.1 * rng.uniform(-1, 1, g.shape)) * dx).to(gpu, torch.float32)
+    m = torch.full((x.shape[0],), 1000.0 * 2.0 ** -20, device=gpu)
+    h = 1.3 * dx
+    pairs = cell_linked_pairs(x, 2.0 * h)
+    low = csf_fields3(x, m, h, pairs, rho0=1000.0).color.double()
+    high = csf_fields3(x.double(), m.double(), h, pairs, rho0=1000.0).color
+    assert abs(float(((low - high) / high).mean())) < 1e-8
