@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kGatherBlock) v_gradient(VP<T> p, const T* __r
   if (a >= p.n_fluid) return;
   // h_local = h / (h_ratio * h / h_ref), as the reference rescales the ratio
   const T h = p.has_ratio ? p.h / (ratio[a] * p.h_scale) : p.h;
-  const T inv_h = T(1) / h, sig_h = sigma_d<D, T>(h) * inv_h;
+  const T inv_h = T(1) / h, sig = sigma_d<D, T>(h);
   const T ca = p.has_corr ? corr[a] : T(1);
   T xa[D];
 #pragma unroll
@@ -84,20 +84,20 @@ __global__ void __launch_bounds__(kGatherBlock) v_gradient(VP<T> p, const T* __r
       d[k] = xa[k] - xb[k];
       r2 += d[k] * d[k];
     }
-    T q, scale;
+    // FP64: one reciprocal square root for r, r / h and 1 / (h r).  FP32 keeps the
+    // divisions: their roundings differ from term to term, those of sigma / h and
+    // 1 / h are common to the row.
+    T q, ir = T(0), r = T(0);
     if (sizeof(T) == 8) {
-      // one reciprocal square root for r, r / h and 1 / (h r)
-      const T ir = r2 > p.eps * p.eps ? rsqrt(r2) : T(1) / p.eps;
+      ir = r2 > p.eps * p.eps ? rsqrt(r2) : T(1) / p.eps;
       q = r2 * ir * inv_h;
-      scale = sig_h * ir;
     } else {
-      const T r = sqrt(r2);
+      r = sqrt(r2);
       q = r / h;
-      scale = sig_h / (r > p.eps ? r : p.eps);
     }
     const T t = T(2) - q;
     const T ds = q < T(1) ? T(-3) * q + T(2.25) * q * q : (q < T(2) ? T(-0.75) * t * t : T(0));
-    scale = scale * ds;
+    const T scale = sizeof(T) == 8 ? sig * inv_h * ir * ds : sig * ds / (h * (r > p.eps ? r : p.eps));
     const T cb = p.has_corr ? corr[b] : T(1);
     const T w = (b < p.n_fluid ? ca + cb : p.wall_factor * ca) * vb;
 #pragma unroll
