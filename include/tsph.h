@@ -106,7 +106,10 @@ int tsph_pairs_emit(const void* pos, const tsph_grid* grid, int64_t row_limit, v
  * first index is below row_limit, without the list in between: after
  * tsph_grid_build, tsph_rows_count writes rowptr (n + 1 int64) and returns the
  * entry count on the host (synchronises), tsph_rows_emit writes the entries
- * (entry_count uint32).  Same rows as tsph_csr_from_pairs makes of the list. */
+ * (entry_count uint32).  Same rows as tsph_csr_from_pairs makes of the list.
+ * An emit takes the row_limit and the rowptr (the list: its row_limit and count)
+ * of one count on the same built grid.  Other counts may lie in between; they
+ * cost the emit a second scan. */
 int tsph_rows_count(const void* pos, const tsph_grid* grid, int64_t row_limit, void* ws,
                     int64_t ws_bytes, int64_t* rowptr, int64_t* entry_count, tsph_stream stream);
 int tsph_rows_emit(const void* pos, const tsph_grid* grid, int64_t row_limit, void* ws,

@@ -48,6 +48,20 @@ struct GridDev {
   float edge[kMaxDim];   // periodic box edges in records
 };
 
+// What the last count left in the slots: rows of this limit (kAllForward: the
+// list's), this many slots each (0: none), the longest row if some row has more.
+struct alignas(16) RowState {
+  int longest, slots;
+  long long limit;
+};
+constexpr long long kAllForward = -1;
+
+__device__ __forceinline__ bool in_slots(const RowState* state, int slots, long long limit) {
+  const int4 v = *reinterpret_cast<const int4*>(state);
+  const long long counted = static_cast<long long>(static_cast<uint64_t>(static_cast<uint32_t>(v.w)) << 32 | static_cast<uint32_t>(v.z));
+  return slots > 0 && v.y == slots && v.x <= slots && counted == limit;
+}
+
 struct BuildWs {
   uint64_t* keys;      // n (radix), or the key and slot of every particle (dense)
   uint64_t* keys_tmp;  // n
@@ -55,8 +69,8 @@ struct BuildWs {
   int32_t* order_tmp;  // n
   float* rec;          // n, sorted: position from the grid's corner, in cutoffs (rec_at)
   int32_t* cell;       // n * dim, sorted: cell coordinates relative to origin
-  int32_t* counts;     // total_cells (dense) or 0, then
-  int32_t* longest;    // 1: 0, or the longest row when it has outgrown its slots
+  int32_t* counts;     // total_cells (dense) or 1, then
+  RowState* state;     // 1
   int64_t* start;      // total_cells + 1 (dense) or 1: first sorted position of a cell
   int64_t* rowptr;     // n + 1 (pair rows)
   int32_t* rowcount;   // n
@@ -93,8 +107,8 @@ size_t build_layout(const tsph_grid& g, BuildWs* w, void* base) {
   t.order_tmp = reinterpret_cast<int32_t*>(take(n * sizeof(int32_t)));
   t.rec = reinterpret_cast<float*>(take((n + 3) / 4 * 4 * sizeof(float4)));
   t.cell = reinterpret_cast<int32_t*>(take(n * g.dim * sizeof(int32_t)));
-  t.counts = reinterpret_cast<int32_t*>(take((cells + 1) * sizeof(int32_t)));
-  t.longest = t.counts ? t.counts + (g.dense ? g.total_cells : 0) : nullptr;
+  t.counts = reinterpret_cast<int32_t*>(take(cells * sizeof(int32_t)));
+  t.state = reinterpret_cast<RowState*>(take(sizeof(RowState)));
   t.start = reinterpret_cast<int64_t*>(take((cells + 1) * sizeof(int64_t)));
   t.rowptr = reinterpret_cast<int64_t*>(take((n + 1) * sizeof(int64_t)));
   t.rowcount = reinterpret_cast<int32_t*>(take(n * sizeof(int32_t)));
@@ -399,8 +413,10 @@ enum RowPass { kCount, kSlot, kFill };
 // cells c - 1 .. c + 1 of the last axis are consecutive keys: a column's
 // candidates are one run (two at a periodic seam), 3^(D-1) runs in all.
 // kCount counts them, kSlot also writes the first `slots` of each row to its
-// slots (in any order) and raises `longest` where that was not all, kFill, run
-// when it was raised, writes the rows from rowptr on.
+// slots (in any order), raises state->longest where that was not all and notes
+// what the slots hold; kFill, for rows that the slots do not hold, writes them
+// from rowptr on, each within its own part (a rowptr of another limit would not
+// fit: what is missing there becomes the row itself, so that no pass reads out of range).
 //
 // What bounds it: instruction issue (in 3-D three to four instructions a candidate
 // and twenty a hit; the list at 2.05 h scans ~500 candidates for ~80 hits) and, with
@@ -412,14 +428,19 @@ template <class T, int D, RowKind kKind, RowPass kPass, int kLanes>
 __global__ void __launch_bounds__(128) scan_rows(const T* __restrict__ pos, int64_t n, int64_t row_limit, GridDev g,
                                                  Cells cs, Band band, T c2, int32_t* __restrict__ rowcount,
                                                  const int64_t* __restrict__ rowptr, uint32_t* __restrict__ out,
-                                                 int slots, int* longest) {
-  if (kPass == kFill && *longest <= slots) return;
+                                                 int slots, RowState* state) {
+  const long long rows_of = kKind == kForward ? kAllForward : static_cast<long long>(row_limit);
+  if (kPass == kFill && in_slots(state, slots, rows_of)) return;
   constexpr int kColumns = D == 1 ? 1 : (D == 2 ? 3 : 9);
   constexpr uint32_t kSecond = 0x80000000u;
   const int lane = threadIdx.x & 31, gl = lane & (kLanes - 1);
   const unsigned group = kLanes == 1 ? 1u << lane : ((kLanes == 32 ? 0u : 1u << kLanes) - 1u) << (lane - gl);
   const int64_t t = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / kLanes;
   if (t >= n) return;
+  if (kPass == kSlot && t == 0 && gl == 0) {
+    state->slots = slots;
+    state->limit = rows_of;
+  }
   const float* ra = cs.rec + rec_at<D>(t);
   const int64_t a = D == 3 ? cs.id[t] : __float_as_int(ra[3]);
   if (kKind == kForward && kPass == kFill && a >= row_limit) return;
@@ -429,12 +450,13 @@ __global__ void __launch_bounds__(128) scan_rows(const T* __restrict__ pos, int6
   const float xa[3] = {ra[0], D > 1 ? ra[kRecStep<D>] : 0.f, D > 2 ? ra[2 * kRecStep<D>] : 0.f};
   int count = 0;
   const int64_t slot = kPass == kFill ? rowptr[a] : a * slots;
+  const int room = kPass == kFill ? static_cast<int>(rowptr[a + 1] - slot) : slots;
 
   const int me = static_cast<int>(a), limit = static_cast<int>(row_limit);
   const bool first = me < limit;  // kBoth: a row below the limit takes every neighbour
   const T* __restrict__ px = pos;
   auto put = [&](int at, int b) {
-    if (kPass == kSlot && at >= slots) return;
+    if (at >= room) return;
     out[slot + at] = kKind == kBoth && b < me ? static_cast<uint32_t>(b) | kSecond : static_cast<uint32_t>(b);
   };
   const auto wanted = [&](int b) { return kKind == kForward ? b > me : b != me && (first || b < limit); };
@@ -596,14 +618,16 @@ __global__ void __launch_bounds__(128) scan_rows(const T* __restrict__ pos, int6
       }
     }
   }
-  if (kPass != kFill) {
+  if (kPass == kFill) {
+    for (int k = count + gl; k < room; k += kLanes) out[slot + k] = static_cast<uint32_t>(me);
+  } else {
     if (kPass == kCount && kLanes > 1) {
 #pragma unroll
       for (int o = kLanes / 2; o > 0; o >>= 1) count += __shfl_xor_sync(group, count, o);
     }
     if (gl == 0) {
       rowcount[a] = count;
-      if (kPass == kSlot && count > slots) atomicMax(longest, count);
+      if (kPass == kSlot && count > slots) atomicMax(&state->longest, count);
     }
   }
 }
@@ -630,10 +654,10 @@ int launch_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, const
   const Band band = band_of(grid);
   if (n <= kLaneRows || (band.exact && grid.dense))
     scan_rows<T, D, kKind, kPass, 8><<<static_cast<unsigned>((n * 8 + 127) / 128), 128, 0, s>>>(
-        p, n, row_limit, to_dev(grid), cs, band, c2, w.rowcount, rowptr, out, slots, w.longest);
+        p, n, row_limit, to_dev(grid), cs, band, c2, w.rowcount, rowptr, out, slots, w.state);
   else
     scan_rows<T, D, kKind, kPass, 1><<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(
-        p, n, row_limit, to_dev(grid), cs, band, c2, w.rowcount, rowptr, out, slots, w.longest);
+        p, n, row_limit, to_dev(grid), cs, band, c2, w.rowcount, rowptr, out, slots, w.state);
   TSPH_LAUNCH_CHECK();
   return TSPH_OK;
 }
@@ -653,8 +677,7 @@ template <RowKind kKind>
 int count_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, const BuildWs& w, int64_t* rowptr,
                cudaStream_t s) {
   const bool slots = use_slots<kKind>(grid);
-  // without slots every row has outgrown them
-  TSPH_CUDA_CHECK(cudaMemsetAsync(w.longest, slots ? 0 : 0x7f, sizeof(int), s));
+  TSPH_CUDA_CHECK(cudaMemsetAsync(w.state, 0, sizeof(RowState), s));
   int rc = dispatch(grid.dtype, grid.dim, [&](auto t, auto d) {
     using T = decltype(t);
     constexpr int D = decltype(d)::value;
@@ -665,14 +688,15 @@ int count_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, const 
   return exclusive_scan_i32_to_i64(w.rowcount, rowptr, grid.n, rowptr + grid.n, w.scan_scratch, s);
 }
 
-// The rows in their slots, or in `full` when some row has outgrown them.
+// The rows in their slots, or in `full` when the slots do not hold them.
 struct FoundRows {
   uint32_t *slot, *full;
   const int64_t* ptr;
-  const int* longest;
+  const RowState* state;
   int slots;
+  long long limit;
   __device__ __forceinline__ uint32_t* src(int64_t r) const {
-    return *longest > slots ? full + ptr[r] : slot + r * slots;
+    return in_slots(state, slots, limit) ? slot + r * slots : full + ptr[r];
   }
   __device__ __forceinline__ int64_t dst(int64_t r) const { return ptr[r]; }
   __device__ __forceinline__ int64_t len(int64_t r) const { return ptr[r + 1] - ptr[r]; }
@@ -686,8 +710,9 @@ int emit_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, int64_t
     return launch_rows<decltype(t), decltype(d)::value, kKind, kFill>(pos, grid, row_limit, w, rowptr, full, s);
   });
   if (rc) return rc;
-  return sort_rows(FoundRows{w.slots, full, rowptr, w.longest, static_cast<int>(row_slots(grid))}, rows, count, out,
-                   w.sort_scratch, s);
+  const long long limit = kKind == kForward ? kAllForward : static_cast<long long>(row_limit);
+  return sort_rows(FoundRows{w.slots, full, rowptr, w.state, static_cast<int>(row_slots(grid)), limit}, rows, count,
+                   out, w.sort_scratch, s);
 }
 
 // --------------------------------------------------------- brute force ---
@@ -851,7 +876,9 @@ int tsph_grid_build(const void* pos, const tsph_grid* grid, void* ws, int64_t ws
     }
   }
   int32_t* slots = w.order_tmp;
-  if (grid->dense) TSPH_CUDA_CHECK(cudaMemsetAsync(w.counts, 0, grid->total_cells * sizeof(int32_t), s));
+  // the counts and, behind them, what the slots held of earlier positions
+  const size_t counts = reinterpret_cast<char*>(w.state + 1) - reinterpret_cast<char*>(w.counts);
+  TSPH_CUDA_CHECK(cudaMemsetAsync(w.counts, 0, counts, s));
   return dispatch(grid->dtype, grid->dim, [&](auto t, auto d) -> int {
     using T = decltype(t);
     constexpr int D = decltype(d)::value;

@@ -180,3 +180,57 @@ def test_exact_grids_of_many_rows(gpu, dtype, n, dim):
     pos[-64:, 0] += 1.0e6
     pos = pos.astype(dtype)[rng.permutation(n)]
     assert np.array_equal(search(pos, 1.6, gpu), on.cell_linked_pairs_batched(pos, 1.6))
+
+
+@pytest.mark.parametrize("counts,cutoff", [((200,), 2.6), ((40, 41), 2.6), ((40, 41), 6.0), ((12, 13, 11), 2.6),
+                                           ((31, 30, 29), 2.6), ((12, 13, 11), 5.5)])
+def test_emit_after_other_counts(gpu, counts, cutoff):
+    """An emit gives the rows of its own count whatever was counted on the grid in between:
+    the list and the rows share the slots (6.0 and 5.5: rows that outgrow them)."""
+    import ctypes
+    from tensorsph_b200 import _lib
+    from tensorsph_b200.neighbor_search import _plan
+    pos = lattice(counts, 1.0, np.float64, 0.2)
+    pos = torch.from_numpy(pos[np.random.default_rng(6).permutation(pos.shape[0])]).to(gpu)
+    n, L, s = pos.shape[0], _lib.lib(), _lib.stream(gpu)
+    grid, ws = _plan(pos, cutoff)
+    head = (pos.data_ptr(), ctypes.byref(grid))
+    work = (ws.data_ptr(), ws.numel())
+
+    def count_rows(limit):
+        ptr, c = torch.empty(n + 1, dtype=torch.long, device=gpu), ctypes.c_int64(0)
+        _lib.check(L.tsph_rows_count(*head, limit, *work, ptr.data_ptr(), ctypes.byref(c), s), "rows_count")
+        return limit, ptr, c.value
+
+    def emit_rows(limit, ptr, c):
+        out = torch.empty(c, dtype=torch.int32, device=gpu)
+        _lib.check(L.tsph_rows_emit(*head, limit, *work, ptr.data_ptr(), out.data_ptr(), c, s), "rows_emit")
+        return out
+
+    def count_pairs(limit):
+        c, total = ctypes.c_int64(0), ctypes.c_int64(0)
+        _lib.check(L.tsph_pairs_count(*head, limit, *work, ctypes.byref(c), ctypes.byref(total), s), "pairs_count")
+        return limit, c.value
+
+    def emit_pairs(limit, c):
+        out = torch.empty((c, 2), dtype=torch.long, device=gpu)
+        ews = _lib.workspace(L.tsph_pairs_emit_workspace_bytes(c, n), gpu)
+        _lib.check(L.tsph_pairs_emit(*head, limit, *work, ews.data_ptr(), ews.numel(), out.data_ptr(), c, s),
+                   "pairs_emit")
+        return out
+
+    _lib.check(L.tsph_grid_build(*head, *work, None, s), "tsph_grid_build")
+    list_, half = count_pairs(n), n // 2
+    want = emit_pairs(*list_)
+    assert np.array_equal(want.cpu().numpy(), on.cell_linked_pairs(pos.cpu().numpy(), cutoff))
+    whole = count_rows(n)
+    rows = emit_rows(*whole)
+    part = count_rows(half)
+    part_rows = emit_rows(*part)
+    assert torch.equal(emit_pairs(*list_), want)              # after the rows of another limit
+    assert torch.equal(emit_rows(*whole), rows)
+    assert torch.equal(emit_rows(*part), part_rows)
+    short = count_pairs(half)                                 # the list's count between rows' count and emit
+    assert torch.equal(emit_pairs(*short), want[want[:, 0] < half])
+    assert torch.equal(emit_rows(*whole), rows)
+    assert torch.equal(emit_rows(*part), part_rows)
