@@ -80,6 +80,11 @@ int64_t tsph_grid_plan_scratch_bytes(void);
 int tsph_grid_plan(const void* pos, int64_t n, int64_t dim, int64_t dtype, double cutoff,
                    const double* box, void* scratch, tsph_grid* grid, tsph_stream stream);
 
+/* A workspace larger than grid->workspace_bytes by tsph_grid_slot_bytes saves
+ * the counts below (symmetric 0: the list's, 1: the rows') a second scan at the
+ * emit; pass the same size to both.  0 where it would not pay. */
+int64_t tsph_grid_slot_bytes(const tsph_grid* grid, int64_t symmetric);
+
 /* Particles by cell (counting sort, or a radix sort of the keys of a grid that
  * is not dense).  order_out (nullable, n int64) receives the stable cell order -- the
  * permutation the reference obtains as argsort(inverse, stable=True). */

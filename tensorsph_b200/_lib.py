@@ -185,6 +185,7 @@ _SIGNATURES = {
     "tsph_grid_plan_scratch_bytes": (c_int64, []),
     "tsph_grid_plan": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_double, c_void_p, c_void_p,
                                POINTER(Grid), c_void_p]),
+    "tsph_grid_slot_bytes": (c_int64, [POINTER(Grid), c_int64]),
     "tsph_grid_build": (c_int, [c_void_p, POINTER(Grid), c_void_p, c_int64, c_void_p, c_void_p]),
     "tsph_pairs_count": (c_int, [c_void_p, POINTER(Grid), c_int64, c_void_p, c_int64,
                                  POINTER(c_int64), POINTER(c_int64), c_void_p]),

@@ -74,10 +74,10 @@ struct BuildWs {
   int64_t* start;      // total_cells + 1 (dense) or 1: first sorted position of a cell
   int64_t* rowptr;     // n + 1 (pair rows)
   int32_t* rowcount;   // n
-  uint32_t* slots;     // n * row_slots
   char* radix_scratch;
   char* scan_scratch;
   char* sort_scratch;
+  uint32_t* slots;     // last: n * row_slots, where the workspace has room for them
 };
 
 // Slots per row: a 3-D row of 2h + 0.25 h holds 104 neighbours, half of them
@@ -85,9 +85,25 @@ struct BuildWs {
 constexpr int kSlots[4] = {0, 16, 48, 128};
 constexpr int64_t kSlotBytes = int64_t(4) << 30;  // a grid that would take more keeps none
 
-int64_t row_slots(const tsph_grid& g) {
+// What a row holds: kForward b > a (the list's pairs (a, b)); kBoth every
+// neighbour whose pair's first index is below the limit, as gather-row entries
+// (b, with the top bit when a is the pair's second element).
+enum RowKind { kForward, kBoth };
+
+// Slots worth having: none where the mean row of a full grid already comes near
+// them (most rows would be scanned twice and written twice).
+int64_t wanted_slots(const tsph_grid& g, RowKind kind) {
   const int64_t k = kSlots[g.dim];
-  return g.n * k * static_cast<int64_t>(sizeof(uint32_t)) <= kSlotBytes ? k : 0;
+  const double ball[4] = {0.0, 2.0, 3.1416, 4.1888};
+  const double mean = ball[g.dim] * static_cast<double>(g.n) / static_cast<double>(g.total_cells) *
+                      (kind == kForward ? 0.5 : 1.0);
+  return g.n * k * static_cast<int64_t>(sizeof(uint32_t)) <= kSlotBytes && static_cast<double>(k) > 1.2 * mean ? k : 0;
+}
+
+// Slots that a workspace of ws_bytes has room for.
+int row_slots(const tsph_grid& g, RowKind kind, int64_t ws_bytes) {
+  const int64_t k = wanted_slots(g, kind);
+  return ws_bytes - g.workspace_bytes >= g.n * k * static_cast<int64_t>(sizeof(uint32_t)) ? static_cast<int>(k) : 0;
 }
 
 size_t build_layout(const tsph_grid& g, BuildWs* w, void* base) {
@@ -112,10 +128,10 @@ size_t build_layout(const tsph_grid& g, BuildWs* w, void* base) {
   t.start = reinterpret_cast<int64_t*>(take((cells + 1) * sizeof(int64_t)));
   t.rowptr = reinterpret_cast<int64_t*>(take((n + 1) * sizeof(int64_t)));
   t.rowcount = reinterpret_cast<int32_t*>(take(n * sizeof(int32_t)));
-  t.slots = reinterpret_cast<uint32_t*>(take(n * row_slots(g) * sizeof(uint32_t)));
   t.radix_scratch = take(radix_scratch_bytes(n));
   t.scan_scratch = take(scan_scratch_bytes(std::max<int64_t>(n, cells) + 1));
   t.sort_scratch = take(segsort_scratch_bytes(n));
+  t.slots = reinterpret_cast<uint32_t*>(cur + used);
   if (w) *w = t;
   return used;
 }
@@ -402,10 +418,6 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
   return r;
 }
 
-// What a row holds: kForward b > a (the list's pairs (a, b)); kBoth every
-// neighbour whose pair's first index is below the limit, as gather-row entries
-// (b, with the top bit when a is the pair's second element).
-enum RowKind { kForward, kBoth };
 enum RowPass { kCount, kSlot, kFill };
 
 // The rows of all particles, thread per row (kLanes = 1) or kLanes lanes per
@@ -645,12 +657,11 @@ constexpr int64_t kLaneRows = 24576;
 
 template <class T, int D, RowKind kKind, RowPass kPass>
 int launch_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, const BuildWs& w, const int64_t* rowptr,
-                uint32_t* out, cudaStream_t s) {
+                uint32_t* out, int slots, cudaStream_t s) {
   const int64_t n = grid.n;
   const Cells cs{w.rec, w.order, w.cell, w.start, w.keys};
   const T c2 = static_cast<T>(grid.cutoff * grid.cutoff);
   const T* p = static_cast<const T*>(pos);
-  const int slots = static_cast<int>(row_slots(grid));
   const Band band = band_of(grid);
   if (n <= kLaneRows || (band.exact && grid.dense))
     scan_rows<T, D, kKind, kPass, 8><<<static_cast<unsigned>((n * 8 + 127) / 128), 128, 0, s>>>(
@@ -662,27 +673,16 @@ int launch_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, const
   return TSPH_OK;
 }
 
-// Whether the rows are worth slots: not where the mean row of a full grid
-// already comes near them (most rows would be scanned twice and written twice).
-template <RowKind kKind>
-bool use_slots(const tsph_grid& g) {
-  const double ball[4] = {0.0, 2.0, 3.1416, 4.1888};
-  const double mean = ball[g.dim] * static_cast<double>(g.n) / static_cast<double>(g.total_cells) *
-                      (kKind == kForward ? 0.5 : 1.0);
-  return static_cast<double>(row_slots(g)) > 1.2 * mean;
-}
-
 // Row lengths (and the rows in their slots), scanned into rowptr.
 template <RowKind kKind>
-int count_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, const BuildWs& w, int64_t* rowptr,
-               cudaStream_t s) {
-  const bool slots = use_slots<kKind>(grid);
+int count_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, const BuildWs& w, int slots,
+               int64_t* rowptr, cudaStream_t s) {
   TSPH_CUDA_CHECK(cudaMemsetAsync(w.state, 0, sizeof(RowState), s));
   int rc = dispatch(grid.dtype, grid.dim, [&](auto t, auto d) {
     using T = decltype(t);
     constexpr int D = decltype(d)::value;
-    return slots ? launch_rows<T, D, kKind, kSlot>(pos, grid, row_limit, w, nullptr, w.slots, s)
-                 : launch_rows<T, D, kKind, kCount>(pos, grid, row_limit, w, nullptr, nullptr, s);
+    return slots ? launch_rows<T, D, kKind, kSlot>(pos, grid, row_limit, w, nullptr, w.slots, slots, s)
+                 : launch_rows<T, D, kKind, kCount>(pos, grid, row_limit, w, nullptr, nullptr, 0, s);
   });
   if (rc) return rc;
   return exclusive_scan_i32_to_i64(w.rowcount, rowptr, grid.n, rowptr + grid.n, w.scan_scratch, s);
@@ -704,14 +704,15 @@ struct FoundRows {
 
 // The first `rows` rows sorted into out; `full`: room for their `count` entries.
 template <RowKind kKind, class Out>
-int emit_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, int64_t rows, const BuildWs& w,
+int emit_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, int64_t rows, const BuildWs& w, int slots,
               const int64_t* rowptr, uint32_t* full, int64_t count, Out out, cudaStream_t s) {
   int rc = dispatch(grid.dtype, grid.dim, [&](auto t, auto d) {
-    return launch_rows<decltype(t), decltype(d)::value, kKind, kFill>(pos, grid, row_limit, w, rowptr, full, s);
+    return launch_rows<decltype(t), decltype(d)::value, kKind, kFill>(pos, grid, row_limit, w, rowptr, full, slots,
+                                                                                  s);
   });
   if (rc) return rc;
   const long long limit = kKind == kForward ? kAllForward : static_cast<long long>(row_limit);
-  return sort_rows(FoundRows{w.slots, full, rowptr, w.state, static_cast<int>(row_slots(grid)), limit}, rows, count,
+  return sort_rows(FoundRows{w.slots, full, rowptr, w.state, slots, limit}, rows, count,
                    out, w.sort_scratch, s);
 }
 
@@ -846,6 +847,11 @@ int tsph_grid_plan(const void* pos, int64_t n, int64_t dim, int64_t dtype, doubl
   return TSPH_OK;
 }
 
+int64_t tsph_grid_slot_bytes(const tsph_grid* grid, int64_t symmetric) {
+  if (!grid || grid->dim < 1 || grid->dim > 3) return 0;
+  return grid->n * wanted_slots(*grid, symmetric ? kBoth : kForward) * static_cast<int64_t>(sizeof(uint32_t));
+}
+
 int tsph_grid_build(const void* pos, const tsph_grid* grid, void* ws, int64_t ws_bytes,
                     int64_t* order_out, tsph_stream stream) {
   if (!grid) return TSPH_ERR_ARG;
@@ -913,7 +919,7 @@ int tsph_pairs_count(const void* pos, const tsph_grid* grid, int64_t row_limit, 
   if (row_limit > n) row_limit = n;
   BuildWs w;
   build_layout(*grid, &w, ws);
-  int rc = count_rows<kForward>(pos, *grid, n, w, w.rowptr, s);
+  int rc = count_rows<kForward>(pos, *grid, n, w, row_slots(*grid, kForward, ws_bytes), w.rowptr, s);
   if (rc) return rc;
   int64_t host[2] = {0, 0};
   TSPH_CUDA_CHECK(cudaMemcpyAsync(&host[1], w.rowptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
@@ -945,10 +951,11 @@ int tsph_pairs_emit(const void* pos, const tsph_grid* grid, int64_t row_limit, v
   BuildWs w;
   build_layout(*grid, &w, ws);
   uint32_t* cols = static_cast<uint32_t*>(emit_ws);
+  const int slots = row_slots(*grid, kForward, ws_bytes);
   if (reinterpret_cast<uintptr_t>(pairs) % 16 == 0)
-    return emit_rows<kForward>(pos, *grid, row_limit, row_limit, w, w.rowptr, cols, pair_count,
+    return emit_rows<kForward>(pos, *grid, row_limit, row_limit, w, slots, w.rowptr, cols, pair_count,
                                AsPairs<true>{pairs}, s);
-  return emit_rows<kForward>(pos, *grid, row_limit, row_limit, w, w.rowptr, cols, pair_count,
+  return emit_rows<kForward>(pos, *grid, row_limit, row_limit, w, slots, w.rowptr, cols, pair_count,
                              AsPairs<false>{pairs}, s);
 }
 
@@ -965,7 +972,8 @@ int tsph_rows_count(const void* pos, const tsph_grid* grid, int64_t row_limit, v
   }
   BuildWs w;
   build_layout(*grid, &w, ws);
-  int rc = count_rows<kBoth>(pos, *grid, std::min(std::max<int64_t>(row_limit, 0), n), w, rowptr, s);
+  int rc = count_rows<kBoth>(pos, *grid, std::min(std::max<int64_t>(row_limit, 0), n), w,
+                             row_slots(*grid, kBoth, ws_bytes), rowptr, s);
   if (rc) return rc;
   TSPH_CUDA_CHECK(cudaMemcpyAsync(entry_count, rowptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   TSPH_CUDA_CHECK(cudaStreamSynchronize(s));
@@ -981,8 +989,8 @@ int tsph_rows_emit(const void* pos, const tsph_grid* grid, int64_t row_limit, vo
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   BuildWs w;
   build_layout(*grid, &w, ws);
-  return emit_rows<kBoth>(pos, *grid, std::min(std::max<int64_t>(row_limit, 0), n), n, w, rowptr, entries,
-                          entry_count, AsEntries{entries}, s);
+  return emit_rows<kBoth>(pos, *grid, std::min(std::max<int64_t>(row_limit, 0), n), n, w,
+                          row_slots(*grid, kBoth, ws_bytes), rowptr, entries, entry_count, AsEntries{entries}, s);
 }
 
 int64_t tsph_brute_workspace_bytes(int64_t n) {

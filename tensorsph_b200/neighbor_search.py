@@ -5,11 +5,12 @@ Same names, arguments, return contract and exceptions as the reference module
 lexicographically, as a ``(P, 2)`` int64 tensor on the input's device.
 
 What runs underneath is the CUDA path of ``csrc/cells.cu``: integer cell keys,
-a stable radix (counting) sort by key, a cell-run table and one candidate scan
-per particle that counts, then emits, its row of partners, rows sorted in
-registers/shared memory.  Results are bit-identical to the reference (same
-cell arithmetic, same distance filter), which the GPU tests check against the
-committed reference fixtures.
+a counting sort of FP32 records by cell (a radix sort of the keys where the grid
+is not dense), one candidate scan per particle that counts its row of partners
+and keeps it in slots, the candidates near the cutoff decided in the positions'
+dtype, rows sorted in registers/shared memory.  Results are bit-identical to the
+reference (same cell arithmetic, same distance filter), which the GPU tests
+check against the committed reference fixtures.
 """
 from __future__ import annotations
 
@@ -44,7 +45,19 @@ def _empty(device):
     return torch.empty((0, 2), dtype=torch.long, device=device)
 
 
-def _plan(pos, cutoff, box=None):
+def _without_slots_when_tight(search, *args):
+    """``search(*args, slots=True)``; the row slots (up to 4 GiB) only save a second scan, so
+    where they leave no memory for themselves or the result, the search runs again without."""
+    try:
+        return search(*args, slots=True)
+    except torch.OutOfMemoryError:
+        pass
+    return search(*args, slots=False)
+
+
+def _plan(pos, cutoff, box=None, slots="rows"):
+    """The cloud's grid and its workspace, with row slots for a list (``slots`` "list"), for gather
+    rows ("rows") or without (None)."""
     L = _lib.lib()
     dev = pos.device
     scratch = _lib.workspace(L.tsph_grid_plan_scratch_bytes(), dev)
@@ -58,7 +71,8 @@ def _plan(pos, cutoff, box=None):
     if rc == _lib.ERR_NONFINITE:
         raise ValueError("positions must contain only finite values")
     _lib.check(rc, "tsph_grid_plan")
-    ws = _lib.workspace(grid.workspace_bytes, dev)
+    extra = L.tsph_grid_slot_bytes(ctypes.byref(grid), int(slots == "rows")) if slots else 0
+    ws = _lib.workspace(grid.workspace_bytes + extra, dev)
     return grid, ws
 
 
@@ -69,10 +83,14 @@ def grid_pairs(pos: torch.Tensor, cutoff: float, box=None, row_limit: int | None
     ``row_limit`` keeps only pairs whose first index is below it (the
     ``fluid_count`` pruning); ``total`` is the unpruned count.
     """
+    return _without_slots_when_tight(_grid_pairs, pos, cutoff, box, row_limit, with_order)
+
+
+def _grid_pairs(pos, cutoff, box, row_limit, with_order, slots):
     L = _lib.lib()
     dev = pos.device
     n = pos.shape[0]
-    grid, ws = _plan(pos, cutoff, box)
+    grid, ws = _plan(pos, cutoff, box, "list" if slots else None)
     order = torch.empty(n, dtype=torch.long, device=dev) if with_order else None
     s = _lib.stream(dev)
     _lib.check(L.tsph_grid_build(pos.data_ptr(), ctypes.byref(grid), ws.data_ptr(), ws.numel(),
@@ -95,10 +113,14 @@ def grid_rows(pos: torch.Tensor, cutoff: float, row_limit: int | None = None):
     """Symmetric gather rows ``(rowptr, entries, entry_count)`` of a CUDA-resident cloud (two
     particles at least): the rows that ``symmetric_rows`` makes of the pairs whose first
     index is below ``row_limit``, built from the cells without the pair list."""
+    return _without_slots_when_tight(_grid_rows, pos, cutoff, row_limit)
+
+
+def _grid_rows(pos, cutoff, row_limit, slots):
     L = _lib.lib()
     dev = pos.device
     n = pos.shape[0]
-    grid, ws = _plan(pos, cutoff)
+    grid, ws = _plan(pos, cutoff, slots="rows" if slots else None)
     s = _lib.stream(dev)
     _lib.check(L.tsph_grid_build(pos.data_ptr(), ctypes.byref(grid), ws.data_ptr(), ws.numel(),
                                  None, s), "tsph_grid_build")
@@ -135,7 +157,7 @@ def cell_order(positions: torch.Tensor, cutoff: float) -> torch.Tensor:
     dev = _lib.cuda_device(positions)
     pos = _lib.to_dev(positions.detach(), dev)
     L = _lib.lib()
-    grid, ws = _plan(pos, cutoff)
+    grid, ws = _plan(pos, cutoff, slots=None)
     order = torch.empty(pos.shape[0], dtype=torch.long, device=dev)
     _lib.check(L.tsph_grid_build(pos.data_ptr(), ctypes.byref(grid), ws.data_ptr(), ws.numel(),
                                  order.data_ptr(), _lib.stream(dev)), "tsph_grid_build")

@@ -234,3 +234,45 @@ def test_emit_after_other_counts(gpu, counts, cutoff):
     assert torch.equal(emit_pairs(*short), want[want[:, 0] < half])
     assert torch.equal(emit_rows(*whole), rows)
     assert torch.equal(emit_rows(*part), part_rows)
+
+
+@pytest.mark.parametrize("at", ["slots", "result"])
+@pytest.mark.parametrize("counts,cutoff", [((40, 41), 2.6), ((12, 13, 11), 2.6), ((31, 30, 29), 2.6)])
+def test_search_without_memory_for_slots(gpu, monkeypatch, at, counts, cutoff):
+    """Where torch has no memory for the row slots, or for the result beside them, the
+    search runs without them."""
+    from tensorsph_b200 import _lib
+    from tensorsph_b200 import neighbor_search as ns
+    pos = lattice(counts, 1.0, np.float64, 0.2)
+    n = pos.shape[0]
+    t = torch.from_numpy(pos).to(gpu)
+    want = on.cell_linked_pairs(pos, cutoff)
+    rows = ns.grid_rows(t, cutoff, row_limit=n // 2)
+    plain, empty, refused, sizes = _lib.workspace, torch.empty, [], []
+    fewest = 4 * n * 48                                        # the slots of 48 (2-D) or 128 a row
+
+    def tight(nbytes, device):
+        sizes.append(nbytes)
+        if at == "slots" and nbytes > fewest and not refused:
+            refused.append(nbytes)
+            raise torch.OutOfMemoryError("no room")
+        return plain(nbytes, device)
+
+    def no_result(*a, **k):
+        result = k.get("dtype") in (torch.long, torch.int32) and (a[0] == (want.shape[0], 2) or a[0] == rows[2])
+        if at == "result" and result and not refused:
+            refused.append(a[0])
+            raise torch.OutOfMemoryError("no room")
+        return empty(*a, **k)
+
+    monkeypatch.setattr(_lib, "workspace", tight)
+    monkeypatch.setattr(torch, "empty", no_result)
+    assert np.array_equal(ns.cell_linked_pairs(t, cutoff).cpu().numpy(), want)
+    assert len(refused) == 1
+    refused.clear()
+    sizes.clear()
+    got = ns.grid_rows(t, cutoff, row_limit=n // 2)
+    assert len(refused) == 1 and got[2] == rows[2]
+    assert torch.equal(got[0], rows[0]) and torch.equal(got[1], rows[1])
+    big = [b for b in sizes if b > 1024]
+    assert big[-1] <= big[0] - fewest                          # the second one has no slots
