@@ -2924,6 +2924,11 @@ __global__ void k_read(Dev e, int begin, int n, int dim, double* __restrict__ x,
   }
 }
 
+struct StepGraph {
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+};
+
 struct CaseHost {
   CaseDev dev;
   tsph_case_params prm;
@@ -2945,8 +2950,8 @@ struct tsph_engine {
   int64_t total_cells = 0;
   int block = tsph::kBlock;
   int batch = tsph::kBatch;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  tsph::StepGraph step, spare; // the step graph of the batch's median route (digit_median), of the other one
+  bool digits = false;         // step's route
   cudaStream_t captured_on = nullptr;
   cudaStream_t aux = nullptr;  // captures the bodies of the step graph's conditional nodes
   cudaStream_t side = nullptr; // the shifting percentile's branch beside the gradient pass
@@ -3062,12 +3067,27 @@ void release_streams(tsph_engine* E) {
   E->fork_ev = E->join_ev = nullptr;
 }
 
+void drop(StepGraph& g) {
+  if (g.exec) cudaGraphExecDestroy(g.exec);
+  if (g.graph) cudaGraphDestroy(g.graph);
+  g = StepGraph{};
+}
+
 void invalidate_graph(tsph_engine* E) {
-  if (E->exec) cudaGraphExecDestroy(E->exec);
-  if (E->graph) cudaGraphDestroy(E->graph);
-  E->exec = nullptr;
-  E->graph = nullptr;
+  drop(E->step);
+  drop(E->spare);
   E->captured_on = nullptr;
+}
+
+// Whether the median of |det M| takes a launch per digit: some surface-tension
+// case has more rows than a block's shared memory.  The two routes differ in the
+// step graph's nodes, so each keeps a graph: a batch that goes from one to the
+// other and back updates them in place (a large drop admitted beside small ones:
+// 380 us to the end of its first step, 660 with an instantiation).
+bool digit_median(const tsph_engine* E) {
+  for (const CaseHost& c : E->order)
+    if (c.dev.csf && c.dev.n_fluid > E->select_rows) return true;
+  return false;
 }
 
 bool shifting(const tsph_engine* E) { return E->order.size() == 1 && E->order[0].prm.shift_every > 0; }
@@ -3254,15 +3274,15 @@ int enqueue_step(tsph_engine* E, cudaStream_t s, cudaEvent_t* marks = nullptr, b
     k_csf_colour<<<g, B, 0, s>>>(d);
     const unsigned gh = static_cast<unsigned>((d.nf + 255) / 256);
     const unsigned gp = static_cast<unsigned>((d.n_slots + 3) / 4);
-    int most = 0;
-    for (const CaseHost& c : E->order) most = std::max(most, c.dev.n_fluid);
-    if (most <= E->select_rows) {
-      k_csf_select<<<d.n_slots, 1024, static_cast<size_t>(most) * sizeof(unsigned long long), s>>>(d);
-    } else {
+    if (digit_median(E)) {
       for (int shift = 56; shift >= 0; shift -= 8) {
         k_csf_hist<<<gh, 256, 0, s>>>(d, shift);
         k_csf_pick<<<gp, 128, 0, s>>>(d, shift);
       }
+    } else {
+      int most = 0;
+      for (const CaseHost& c : E->order) most = c.dev.csf ? std::max(most, c.dev.n_fluid) : most;
+      k_csf_select<<<d.n_slots, 1024, static_cast<size_t>(most) * sizeof(unsigned long long), s>>>(d);
     }
     k_csf_grad<<<gf, B, 0, s>>>(d);
     if (d.csf_kinds & 4) k_csf_range<<<gf, B, 0, s>>>(d);
@@ -3796,7 +3816,11 @@ int tsph_engine_step(tsph_engine* E, int64_t steps, tsph_stream stream) {
   if (!E || steps < 0) return TSPH_ERR_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (E->order.empty()) return TSPH_OK;
-  if (E->exec && E->stale && E->captured_on == s) {
+  if (E->stale && E->digits != digit_median(E)) {
+    std::swap(E->step, E->spare);
+    E->digits = !E->digits;
+  }
+  if (E->step.exec && E->stale && E->captured_on == s) {
     // a batch change: capture the new step and update the instantiated graph
     // in place (same kernels and topology, new parameters and grids); a
     // change of topology falls through to a new instantiation
@@ -3807,24 +3831,25 @@ int tsph_engine_step(tsph_engine* E, int64_t steps, tsph_stream stream) {
     cudaError_t ce = cudaStreamEndCapture(s, &g);
     if (rc == TSPH_OK && ce == cudaSuccess) {
       cudaGraphExecUpdateResultInfo info{};
-      if (cudaGraphExecUpdate(E->exec, g, &info) == cudaSuccess) {
-        if (E->graph) cudaGraphDestroy(E->graph);
-        E->graph = g;
+      if (cudaGraphExecUpdate(E->step.exec, g, &info) == cudaSuccess) {
+        if (E->step.graph) cudaGraphDestroy(E->step.graph);
+        E->step.graph = g;
         ++E->updates;
       } else {
         cudaGetLastError();
         cudaGraphDestroy(g);
-        invalidate_graph(E);
+        drop(E->step);
       }
     } else {
       if (g) cudaGraphDestroy(g);
       cudaGetLastError();
-      invalidate_graph(E);
+      drop(E->step);
       if (rc) return rc;
     }
   }
-  if (!E->exec || E->captured_on != s || E->stale) {
-    invalidate_graph(E);
+  if (!E->step.exec || E->captured_on != s || E->stale) {
+    if (E->captured_on != s) invalidate_graph(E);
+    drop(E->step);
     E->stale = false;
     // with conditional rebuild nodes first; without them if the capture or
     // the instantiation fails
@@ -3835,13 +3860,13 @@ int tsph_engine_step(tsph_engine* E, int64_t steps, tsph_stream stream) {
       cudaGraph_t g = nullptr;
       cudaError_t ce = cudaStreamEndCapture(s, &g);
       if (rc == TSPH_OK && ce == cudaSuccess) {
-        ce = cudaGraphInstantiate(&E->exec, g, 0);
+        ce = cudaGraphInstantiate(&E->step.exec, g, 0);
         if (ce == cudaSuccess) {
-          E->graph = g;
+          E->step.graph = g;
           ++E->instantiations;
           break;
         }
-        E->exec = nullptr;
+        E->step.exec = nullptr;
       }
       if (g) cudaGraphDestroy(g);
       if (!cond || attempt > 0) return rc ? rc : TSPH_ERR_CUDA;
@@ -3851,7 +3876,7 @@ int tsph_engine_step(tsph_engine* E, int64_t steps, tsph_stream stream) {
     }
     E->captured_on = s;
   }
-  for (int64_t i = 0; i < steps; ++i) TSPH_CUDA_CHECK(cudaGraphLaunch(E->exec, s));
+  for (int64_t i = 0; i < steps; ++i) TSPH_CUDA_CHECK(cudaGraphLaunch(E->step.exec, s));
   return TSPH_OK;
 }
 
@@ -3888,11 +3913,11 @@ int tsph_engine_graph_kernels(tsph_engine* E, int64_t* kernels) {
   if (!E || !kernels) return TSPH_ERR_ARG;
   kernels[0] = 0;
   kernels[1] = E->conditional ? E->rebuild_kernels : 0;
-  if (!E->graph) return TSPH_ERR_ARG;
+  if (!E->step.graph) return TSPH_ERR_ARG;
   size_t count = 0;
-  TSPH_CUDA_CHECK(cudaGraphGetNodes(E->graph, nullptr, &count));
+  TSPH_CUDA_CHECK(cudaGraphGetNodes(E->step.graph, nullptr, &count));
   std::vector<cudaGraphNode_t> nodes(count);
-  TSPH_CUDA_CHECK(cudaGraphGetNodes(E->graph, nodes.data(), &count));
+  TSPH_CUDA_CHECK(cudaGraphGetNodes(E->step.graph, nodes.data(), &count));
   int64_t k = 0;
   for (size_t i = 0; i < count; ++i) {
     cudaGraphNodeType t;

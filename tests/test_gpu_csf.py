@@ -161,3 +161,32 @@ def test_csf_median_select_routes_agree(neighbour_dx, gpu):
     for other in got[1:]:
         for a, b in zip(got[0], other):
             assert torch.equal(a, b)
+
+
+def test_csf_median_routes_keep_their_graphs(gpu):
+    """A drop of 30.5 k rows admitted beside small ones and retired, again and again: each of the
+    two median routes is instantiated once and updated in place after that, and the small drop's
+    state is the one it has alone."""
+    from dataclasses import replace
+
+    from tensorsph_b200.engine import BatchEngine, capacity_for, droplet_impact_case
+    spec = droplet_impact_case(drop_config(0.0728))
+    big = droplet_impact_case(replace(drop_config(0.0728), dx=0.00025, dt=0.25 * 1.3 * 0.00025 / 20.0))
+    eng = BatchEngine(**capacity_for([spec, spec, big], max_neighbors=64, diag_ring=32))
+    first, _ = eng.add(spec), eng.add(spec)
+    eng.step(1)
+    for _ in range(3):
+        cid = eng.add(big)
+        eng.step(2)
+        eng.remove(cid)
+        eng.step(1)
+    stats = eng.graph_stats()
+    assert stats == {"instantiations": 2, "updates": 5}, stats
+    got = [t.cpu() for t in eng.read(first)]
+    eng.close()
+    eng = BatchEngine(**capacity_for([spec], max_neighbors=64, diag_ring=32))
+    cid = eng.add(spec)
+    eng.step(10)
+    for a, b in zip(got, eng.read(cid)):
+        assert torch.equal(a, b.cpu())
+    eng.close()
