@@ -2381,10 +2381,6 @@ __global__ void __launch_bounds__(kMaxBlock) k_integrate(const __grid_constant__
   if (c >= 0) add_meters(e.ctl[c], s);
 }
 
-// Per-case meter row: max rho, max |v|, front x, obstacle force xyz, kinetic
-// and potential energy, escapes, clamps, rebuilds, longest row, step, status,
-// obstacle impulse x, c_ref, the correction's log (16-19, written after the
-// update), obstacle impulse y and z, and the clamp impulse xyz.
 // What k_finalize reads of a case.
 struct FinalDev {
   int adaptive, shift_every, tvc_every, tvc_bulk, comp;
@@ -2400,6 +2396,10 @@ __device__ __forceinline__ unsigned int remainder_of(unsigned long long step, in
                     : static_cast<unsigned int>(step) % static_cast<unsigned int>(m);
 }
 
+// Per-case meter row: max rho, max |v|, front x, obstacle force xyz, kinetic
+// and potential energy, escapes, clamps, rebuilds, longest row, step, status,
+// obstacle impulse x, c_ref, the correction's log (16-19, written after the
+// update), obstacle impulse y and z, and the clamp impulse xyz.
 // The case's state is read whole before anything is written (one wait on memory
 // instead of one per field behind each store), with 32-bit remainders: 8.1 -> 3.3
 // us for one case, 13.4 -> 6.6 for 64.

@@ -106,19 +106,31 @@ inline unsigned row_grid(int64_t n, int lanes, int block = kGatherBlock) {
   return static_cast<unsigned>(g < 1 ? 1 : g);
 }
 
-// Calls f(lanes per row) for rows of a D-dimensional cloud.  The lines lie where
-// whole rhs passes (density, diffusion, force; FP32, then FP64; us) cross:
+// Calls f(lanes per row) for rows of a D-dimensional cloud.  Device time of the
+// three passes of an rhs (density, diffusion, force; FP32, then FP64; us):
 //   2-D, ~20 entries    L = 1        2        4
-//       5 k rows       51  59    44  44    37  41
-//      60 k            58  66    49  54    57  64
-//     250 k            99 124    91 119   130 160
-//     1.0 M           275 409   297 414   447 613
+//       5 k rows        30  35   21  24   16  18
+//      24 k             33  38   23  26   18  21
+//      36 k             34  40   25  28   21  28
+//      49 k             35  41   26  31   27  36
+//     250 k             79  98   73  98   92 124
+//     400 k            108 150  108 148
+//     550 k            140 200  144 204
+//     1.0 M            243 344  252 359
 //   3-D, ~80 entries    L = 2        4        8
-//       5 k rows      110 122    74  81    58  62
-//      24 k           114 129    78  89    76  96
-//      82 k           140 201   132 178   153 203
-//     241 k           313 486   324 491   408 604
-// (L = 4 in 2-D and 8 in 3-D measured with divisions in the terms.)
+//       4 k rows        65  73   37  42   24  26
+//      23 k             67  79   42  50   37  54
+//      33 k             69  82   49  70   50  66
+//      48 k             77  90   68  95   63  90
+//      81 k             96 150   94 135   95 140
+//     161 k            177 250  168 255
+//     201 k            216 318  210 323
+//     420 k            424 642  441 680
+// (threed's passes alike, FP64: 24 k rows 101 / 102 with four / eight lanes, 36 k
+// 160 / 135, 64 k 210 / 209.)  One line serves both dtypes and every pass: four lanes
+// in 2-D pay up to 36 k rows in FP64 and 45 k in FP32, and cost at most 5 us of a
+// ~110 us call between there and the line; eight in 3-D are the fastest or within
+// 4 us up to theirs.
 template <int D, class F>
 int with_lanes(int64_t rows, F&& f) {
   if (D == 3) {

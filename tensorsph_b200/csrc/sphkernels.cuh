@@ -84,20 +84,12 @@ struct Cubic {
     W = sigma * (s > T(0) ? s : T(0));
     g = g2(R);
   }
-  // lap3 from q and 1 / r: f'' + 2 f' / q with the quotient written out (-6 + 4.5 q
-  // below q = 1, its limit at 0 included).
+  // 3-D Laplacian of W (threed/kernel3.py:108-124): sigma / h^2 (f'' + 2 f' / q) with the
+  // quotient written out (f' / q = -3 + 2.25 q below q = 1, its limit at 0 included).
   __device__ __forceinline__ T lap2(const Radial& R) const {
     const T t = T(2) - R.q;
     const T near = T(-9) + T(9) * R.q, far = t * (T(1.5) - T(1.5) * t * (h * R.ir));
     return sigma_hh * (R.q < T(1) ? near : (R.q < T(2) ? far : T(0)));
-  }
-  // 3-D Laplacian of W (threed/kernel3.py:108-124).
-  __device__ __forceinline__ T lap3(T r) const {
-    T q = r / h;
-    if (!(q < T(2))) return T(0);
-    T second = q < T(1) ? T(-3) + T(4.5) * q : T(1.5) * (T(2) - q);
-    T twice = q > T(1e-10) ? T(2) * dshape(q) / (q > eps ? q : eps) : T(-6);
-    return sigma * (second + twice) / (h * h);
   }
 };
 
