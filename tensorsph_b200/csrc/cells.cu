@@ -18,8 +18,8 @@
 //                candidates of its 3^D cells, into a fixed number of slots
 //   scan -> [host: list length]
 //   rows_sort    each row in index order, written out as pairs or gather rows
-// Where a row outgrows its slots, a second scan_rows writes the rows to their
-// places in the list before the sort.
+// Where a row outgrows its slots, or the workspace has none, a second scan_rows
+// writes the rows to their places in the list before the sort.
 // A grid with far more cells than particles sorts its keys instead (radix) and
 // finds the cells by bisection.  The order inside a cell is arbitrary (slots
 // come from atomics) and does not show: rows are sorted by index.
@@ -58,8 +58,8 @@ constexpr long long kAllForward = -1;
 
 __device__ __forceinline__ bool in_slots(const RowState* state, int slots, long long limit) {
   const int4 v = *reinterpret_cast<const int4*>(state);
-  const long long counted = static_cast<long long>(static_cast<uint64_t>(static_cast<uint32_t>(v.w)) << 32 | static_cast<uint32_t>(v.z));
-  return slots > 0 && v.y == slots && v.x <= slots && counted == limit;
+  const uint64_t counted = static_cast<uint64_t>(static_cast<uint32_t>(v.w)) << 32 | static_cast<uint32_t>(v.z);
+  return slots > 0 && v.y == slots && v.x <= slots && static_cast<long long>(counted) == limit;
 }
 
 struct BuildWs {
@@ -275,13 +275,13 @@ int plan_bounds(const void* pos, int64_t n, double cutoff, unsigned long long* d
 
 // ----------------------------------------------------------------- build ---
 
-// Cell of one coordinate (relative to the grid's origin, or wrapped into the
-// box) and its record: the coordinate from the grid's corner, moved by whole
-// boxes into the same cell when periodic, in cutoffs.
 __device__ __forceinline__ float record(double length, double scale) {
   return scale == 0.0 ? 0.f : static_cast<float>(length * scale);
 }
 
+// Cell of one coordinate (relative to the grid's origin, or wrapped into the
+// box) and its record: the coordinate from the grid's corner, moved by whole
+// boxes into the same cell when periodic, in cutoffs.
 template <class T>
 __device__ __forceinline__ long long cell_of(T x, const GridDev& g, int k, float* local) {
   if (g.periodic) {
@@ -707,8 +707,7 @@ template <RowKind kKind, class Out>
 int emit_rows(const void* pos, const tsph_grid& grid, int64_t row_limit, int64_t rows, const BuildWs& w, int slots,
               const int64_t* rowptr, uint32_t* full, int64_t count, Out out, cudaStream_t s) {
   int rc = dispatch(grid.dtype, grid.dim, [&](auto t, auto d) {
-    return launch_rows<decltype(t), decltype(d)::value, kKind, kFill>(pos, grid, row_limit, w, rowptr, full, slots,
-                                                                                  s);
+    return launch_rows<decltype(t), decltype(d)::value, kKind, kFill>(pos, grid, row_limit, w, rowptr, full, slots, s);
   });
   if (rc) return rc;
   const long long limit = kKind == kForward ? kAllForward : static_cast<long long>(row_limit);
